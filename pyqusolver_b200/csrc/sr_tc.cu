@@ -225,7 +225,8 @@ __global__ void tc_build_vp_kernel(TcDims d, bool cplx, const V* __restrict__ v,
 __device__ __forceinline__ uint32_t spin_window(const uint32_t* wrd, int nw, int i0) {
   if (i0 < 0) return wrd[0] << (-i0);
   const int w = i0 >> 5, sh = i0 & 31;
-  const uint32_t lo = wrd[128 * w], hi = (w + 1 < nw) ? wrd[128 * (w + 1)] : 0u;
+  // a window past the last word (the v_b row and the padding when ns is a multiple of 32) reads as 0
+  const uint32_t lo = (w < nw) ? wrd[128 * w] : 0u, hi = (w + 1 < nw) ? wrd[128 * (w + 1)] : 0u;
   return __funnelshift_r(lo, hi, sh);
 }
 __device__ __forceinline__ uint32_t low_mask(int c) {

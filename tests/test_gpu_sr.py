@@ -428,3 +428,31 @@ def test_cg_single_reduction_matches_two_reduction_form(impl, rtol):
         assert np.max(np.abs(x1 - x0)) / np.max(np.abs(x0)) < 1e-6
     else:
         assert abs(i1["iterations"] - i0["iterations"]) <= max(2, 0.25 * i0["iterations"])
+
+
+@pytest.mark.parametrize("cplx,ns,nh,n", [(True, 32, 57, 600), (False, 64, 30, 300), (True, 96, 40, 257),
+                                          (False, 96, 470, 200)])
+def test_o_v_on_exactly_full_spin_words(cplx, ns, nh, n):
+    """O v over the hidden axis (tc_ov_kernel, whose epilogue reads 16-bit windows of the spin words) at site
+    counts that fill their last 32-bit word: the v_b row and the padding start past the last word.  The last
+    shape runs it by default (its direction operand does not fit the z form)."""
+    net = RBM((ns,), n_hidden=nh, dtype="complex64" if cplx else "float32", seed=5, init_scale=0.1)
+    rng = np.random.default_rng(6)
+    st = np.where(rng.random((n, ns)) < 0.5, 0.5, -0.5)
+    bits = dv.pack_states(st)
+    _, tn, _ = dv.rbm_forward(net.flat, ns, nh, bits, tanh=True, logpsi=False)
+    P = dv.n_params(ns, nh)
+    v = rng.normal(size=P) + (1j * rng.normal(size=P) if cplx else 0)
+    try:
+        _lib.call("qes_sr_set_ovz", 0)
+        y = dv.sr_matvec(net.flat, ns, nh, bits, tn, torch.as_tensor(v).cuda(), shift=1e-2).cpu().numpy()
+    finally:
+        _lib.call("qes_sr_set_ovz", 1)
+    t = tn.cpu().numpy().astype(np.complex128 if cplx else np.float64)
+    sg = np.where(st > 0, 1.0, -1.0)
+    a, b, W = v[:ns], v[ns:ns + nh], v[ns + nh:].reshape(ns, nh)
+    w = sg @ a + np.sum(t * (sg @ W + b), axis=1)
+    u = (w - w.mean()) / n
+    q = t.conj() * u[:, None]
+    ref = np.concatenate([sg.T @ u, q.sum(axis=0), (sg.T @ q).reshape(-1)]) + 1e-2 * v
+    assert np.max(np.abs(y - ref)) / np.max(np.abs(ref)) < 1e-4          # the SR matvec's bar
