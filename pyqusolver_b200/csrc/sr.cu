@@ -14,6 +14,7 @@
 // result does not depend on how often the host checks.
 #include "common.cuh"
 #include "sr_tc.h"
+#include "sr_pcg.h"
 
 #include <algorithm>
 #include <atomic>
@@ -1506,6 +1507,10 @@ struct SRWork {
   bool tc;            // tensor-core matvec in use
   TcDims td;
   TcWork tw;
+  bool pcg;           // the shapes admit the persistent CG kernel
+  PcgDims pd;
+  double* slots;      // its exchange slots
+  void* pvz;          // its direction operand
   int nsplit;         // partial P-vectors written by the O^H u stage
   int mv_nsplit;      // partial P-vectors written by the matvec (tc_matvec_nsplit on the tensor-core path)
   size_t total;
@@ -1533,7 +1538,9 @@ static SRWork sr_layout(int dtype, int ns, int nh, int64_t n_samples, char* base
   L.wpart = (float2*)take((size_t)((nh + PT_U - 1) / PT_U) * n_samples * (L.fp64 ? sizeof(double2) : sizeof(float2)));
   L.w64 = L.fp64 ? (double2*)take((size_t)n_samples * sizeof(double2)) : nullptr;
   L.wmean = (double*)take(4 * sizeof(double));
-  L.partial = take((size_t)std::max<int64_t>(nsplit_max, 1) * P * (L.fp64 ? vs : ts));
+  L.pcg = tc_ok && pcg_plan(dtype, ns, nh, n_samples, &L.pd);
+  L.partial = take(std::max((size_t)std::max<int64_t>(nsplit_max, 1) * P * (L.fp64 ? vs : ts),
+                            L.pcg ? pcg_partial_bytes(L.pd) : 0));
   L.x = take(P * vs); L.r = take(P * vs); L.p = take(P * vs); L.Ap = take(P * vs); L.b = take(P * vs);
   L.parts = (double*)take(5 * std::max(RED_BLOCKS, RS_MAX_BLOCKS) * sizeof(double));
   L.scal = (double*)take(16 * sizeof(double));
@@ -1544,6 +1551,8 @@ static SRWork sr_layout(int dtype, int ns, int nh, int64_t n_samples, char* base
   L.counter = (unsigned int*)take(128 * sizeof(unsigned int));     // tickets, barrier words (own lines)
   char* tcb = tc_ok ? take(tc_workspace_bytes(L.td)) : nullptr;
   L.tw = (tc_ok && base) ? tc_layout(L.td, tcb) : TcWork{};
+  L.slots = L.pcg ? (double*)take(pcg_slot_bytes(L.pd)) : nullptr;
+  L.pvz = L.pcg ? take(pcg_operand_bytes(L.pd)) : nullptr;
   L.wts = nullptr;
   L.total = off;
   return L;
@@ -1999,6 +2008,46 @@ static int sr_jacobi_t(int ns, int nh, int64_t n_samples, const uint32_t* bits, 
   return QES_OK;
 }
 
+// CG of the unweighted start x = 0 without a preconditioner as one launch (sr_pcg.cu)
+template <class T>
+static int sr_cg_persistent_t(int ns, int nh, int64_t n_samples, const uint32_t* bits, const T* tt, const float2* eloc,
+                              const qes_sr_options* opt, typename VecT<T>::type* x_out, qes_sr_result* res,
+                              const SRWork& L, cudaStream_t st) {
+  using V = typename VecT<T>::type;
+  const int64_t P = (int64_t)ns + nh + (int64_t)ns * nh;
+  const int dtype = ScalarTraits<T>::is_complex ? QES_DTYPE_C64 : QES_DTYPE_F32;
+  QES_CUDA_CHECK(cudaMemsetAsync(L.counter, 0, 128 * sizeof(unsigned int), st));
+  const PcgArgs a{bits, tt, eloc, L.wts, opt->shift, opt->rtol, opt->atol, opt->rhs_prefactor, opt->maxiter,
+                  L.x, L.b, x_out, L.scal, L.partial, L.pvz, L.slots, L.tw.status, (int*)(L.counter + 4)};
+  int rc = pcg_solve(dtype, L.pd, n_samples, a, st);
+  if (rc) return rc;
+  double hs[16] = {0}, true_rr = -1.0;
+  QES_CUDA_CHECK(cudaMemcpyAsync(hs, L.scal, 16 * sizeof(double), cudaMemcpyDeviceToHost, st));
+  if ((rc = sr_check_status(L, st, true))) return rc;      // synchronises the stream
+  if (opt->maxiter > 0 && !opt->skip_true_residual) {
+    if ((rc = sr_prepare(dtype, n_samples, bits, tt, L, st))) return rc;
+    if ((rc = sr_matvec_t<T>(ns, nh, n_samples, bits, tt, opt->shift, (const V*)L.x, (V*)L.Ap, nullptr, L, st, false)))
+      return rc;
+    diff_norm2_kernel<V><<<RED_BLOCKS, RED_THREADS, 0, st>>>(P, (const V*)L.b, (const V*)L.Ap, L.parts);
+    sum_parts_kernel<<<1, SC_THREADS, 0, st>>>(RED_BLOCKS, L.parts, L.scal + 10);
+    QES_LAUNCH_CHECK_N(2);
+    QES_CUDA_CHECK(cudaMemcpyAsync(&true_rr, L.scal + 10, sizeof(double), cudaMemcpyDeviceToHost, st));
+    if ((rc = sr_check_status(L, st))) return rc;
+  }
+  const bool done = hs[4] != 0.0;
+  if (res) {
+    res->iterations = (int)hs[5];
+    res->converged = done ? 1 : 0;
+    res->residual = sqrt(hs[2]);
+    res->rhs_norm = sqrt(hs[6]);
+    res->e_mean_re = hs[12];
+    res->e_mean_im = hs[13];
+    res->true_residual = true_rr < 0.0 ? -1.0 : (hs[6] > 0.0 ? sqrt(true_rr / hs[6]) : 0.0);
+    res->acond = -1.0;
+  }
+  return done ? QES_OK : QES_ERR_NOT_CONVERGED;
+}
+
 // x0: start of the iteration for the unscaled system (nullptr: zero)
 template <class T>
 static int sr_cg_t(int ns, int nh, int64_t n_samples, const uint32_t* bits, const T* tt, const float2* eloc,
@@ -2008,7 +2057,13 @@ static int sr_cg_t(int ns, int nh, int64_t n_samples, const uint32_t* bits, cons
   const int64_t P = (int64_t)ns + nh + (int64_t)ns * nh;
   V* x = (V*)L.x; V* r = (V*)L.r; V* p = (V*)L.p; V* Ap = (V*)L.Ap; V* b = (V*)L.b;
   const int dtype = ScalarTraits<T>::is_complex ? QES_DTYPE_C64 : QES_DTYPE_F32;
-  int rc = sr_prepare(dtype, n_samples, bits, tt, L, st);
+  int rc;
+  // one persistent kernel for the force and all iterations, where the shapes admit it and no other form of
+  // the solve is asked for
+  if (L.pcg && L.tc && tc_default_form() && !x0 && opt->precond == QES_PRECOND_NONE && g_cg_fused.load() == 1 &&
+      g_cg_single.load() == 0 && g_bar_extra.load() == 0 && g_l2_persist.load() == 0 && !qes_prof_on())
+    return sr_cg_persistent_t<T>(ns, nh, n_samples, bits, tt, eloc, opt, x_out, res, L, st);
+  rc = sr_prepare(dtype, n_samples, bits, tt, L, st);
   if (rc) return rc;
   // b = F
   rc = sr_force_t<T>(ns, nh, n_samples, bits, tt, eloc, b, L, st);

@@ -1964,6 +1964,11 @@ extern "C" int qes_sr_set_tiling(int mode, int nc, int ctas) {
   return QES_OK;
 }
 
+bool tc_default_form() {
+  return g_tile_mode.load() == 0 && g_tile_nc.load() == 0 && g_tile_ctas.load() == 0 && g_ov_split.load() == 0 &&
+         g_ovz.load() == 1 && g_ohu_pairs.load() == 0 && g_sv.load() == 0;
+}
+
 bool tc_plan(int dtype, int ns, int nh, int64_t n_samples, TcDims* dout) {
   const bool cplx = dtype == QES_DTYPE_C64;
   const int H = cplx ? 2 : 1;

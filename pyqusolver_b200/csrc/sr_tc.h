@@ -64,6 +64,7 @@ struct TcWork {
 
 constexpr size_t kTcSmemLimit = 220 * 1024;
 
+bool tc_default_form();          // no tiling or product override is set (qes_sr_set_*)
 bool tc_plan(int dtype, int ns, int nh, int64_t n_samples, TcDims* d);
 size_t tc_workspace_bytes(const TcDims& d);
 TcWork tc_layout(const TcDims& d, char* base);

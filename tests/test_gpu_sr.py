@@ -456,3 +456,74 @@ def test_o_v_on_exactly_full_spin_words(cplx, ns, nh, n):
     q = t.conj() * u[:, None]
     ref = np.concatenate([sg.T @ u, q.sum(axis=0), (sg.T @ q).reshape(-1)]) + 1e-2 * v
     assert np.max(np.abs(y - ref)) / np.max(np.abs(ref)) < 1e-4          # the SR matvec's bar
+
+
+# ------------------------------------------------------------------------- the persistent CG kernel
+def _oracle_system(bits, tn, eloc, ns, probs, shift):
+    """S + shift and F in float64 from the float32 T, formed (small shapes only)."""
+    st = np.where(dv.unpack_states(bits, ns).cpu().numpy() > 0, 1.0, -1.0)
+    t = tn.cpu().numpy()
+    t = t.astype(np.complex128 if np.iscomplexobj(t) else np.float64)
+    n = st.shape[0]
+    O = np.concatenate([st.astype(t.dtype), t, (st[:, :, None] * t[:, None, :]).reshape(n, -1)], axis=1)
+    p = np.ones(n) if probs is None else probs / probs.sum() * n
+    e = eloc.cpu().numpy().astype(np.complex128)
+    e = e if np.iscomplexobj(t) else e.real
+    Oc = O - (p[:, None] * O).sum(axis=0) / n
+    F = Oc.conj().T @ (p * (e - (p * e).sum() / n)) / n
+    return Oc.conj().T @ (p[:, None] * Oc) / n + shift * np.eye(O.shape[1]), F
+
+
+# samples per CTA: 16 (one k-step) to 128; one CTA, up to 32 (direct exchanges) and more (collectors); fewer
+# samples than CTAs that the parameter vector needs; ragged last CTA; hidden units at and off the operand
+# padding; ones column that opens a new k-step (ns = 16, 32, 48)
+@pytest.mark.parametrize("cplx,ns,nh,n,weighted", [
+    (True, 3, 2, 1, False), (False, 5, 7, 15, False), (True, 16, 8, 17, True), (False, 32, 16, 129, False),
+    (True, 31, 33, 40, False), (True, 9, 18, 700, True), (False, 48, 15, 2049, True), (True, 20, 41, 4097, False)])
+def test_persistent_cg_matches_float64_solution(cplx, ns, nh, n, weighted):
+    """The default solve (one persistent kernel) against the float64 dense solution of the same system (the SR
+    tests' bar on the backward error, 1e-4); two solves are bit-identical."""
+    net, bits, tn, eloc = _persistent_problem(cplx, ns, nh, n)
+    probs = np.exp(0.4 * np.random.default_rng(9).normal(size=n)).astype(np.float32) if weighted else None
+    pt = None if probs is None else torch.as_tensor(probs).cuda()
+    kw = dict(shift=1e-2, rtol=1e-8, maxiter=2000, probs=pt)
+    x, info = dv.sr_solve_cg(net.flat, ns, nh, bits, tn, eloc, **kw)
+    x2, info2 = dv.sr_solve_cg(net.flat, ns, nh, bits, tn, eloc, check_every=1, **kw)
+    assert torch.equal(x, x2) and info == info2
+    assert info["converged"]
+    A, F = _oracle_system(bits, tn, eloc, ns, probs, 1e-2)
+    got = -x.cpu().numpy()                                   # rhs_prefactor -1
+    nF = np.linalg.norm(F)
+    assert abs(info["rhs_norm"] - nF) <= 1e-4 * nF + 1e-12
+    if nF > 0:
+        assert np.linalg.norm(F - A @ got) <= 1e-4 * nF
+        assert info["true_residual"] < 1e-4
+
+
+def _persistent_problem(cplx, ns, nh, n, seed=21):
+    net = RBM((ns,), n_hidden=nh, dtype="complex64" if cplx else "float32", seed=seed, init_scale=0.2)
+    rng = np.random.default_rng(seed)
+    bits = dv.pack_states(np.where(rng.random((n, ns)) < 0.5, 0.5, -0.5))
+    _, tn, _ = dv.rbm_forward(net.flat, ns, nh, bits, tanh=True, logpsi=False)
+    e = -20 + rng.normal(size=n) + (1j * rng.normal(size=n) if cplx else 0)
+    return net, bits, tn, torch.as_tensor(np.asarray(e, dtype=np.complex64)).cuda()
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+def test_persistent_cg_stops_as_the_rule_says(cplx):
+    """No iteration for a zero force or maxiter = 0; a system that converges at once (a shift far above S:
+    |r|^2 drops below 1e-6 in one step, where it is summed from the vector); maxiter reached."""
+    ns, nh, n = 12, 20, 500
+    net, bits, tn, eloc = _persistent_problem(cplx, ns, nh, n)
+    flat_e = torch.full_like(eloc, -3.0)
+    x, info = dv.sr_solve_cg(net.flat, ns, nh, bits, tn, flat_e, shift=1e-2)
+    assert info["converged"] and info["iterations"] == 0 and float(x.abs().max()) == 0.0
+    x, info = dv.sr_solve_cg(net.flat, ns, nh, bits, tn, eloc, shift=1e-2, maxiter=0)
+    assert not info["converged"] and info["iterations"] == 0 and float(x.abs().max()) == 0.0
+    F = dv.sr_force(net.flat, ns, nh, bits, tn, eloc)
+    x, info = dv.sr_solve_cg(net.flat, ns, nh, bits, tn, eloc, shift=1e9, rtol=1e-6)
+    assert info["converged"] and info["iterations"] == 1
+    # x = -F / shift up to |S| / shift, and F up to the two forms' operator rounding (bar 1e-4)
+    assert float((x * -1e9 - F).abs().max()) <= 1e-4 * float(F.abs().max())
+    _, info = dv.sr_solve_cg(net.flat, ns, nh, bits, tn, eloc, shift=1e-6, rtol=1e-12, maxiter=3)
+    assert not info["converged"] and info["iterations"] == 3
