@@ -250,3 +250,16 @@ QES_D double warp_sum(double v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
+
+// ----------------------------------------------------------------------------
+// asynchronous copies to shared memory (4, 8 or 16 bytes, both sides aligned to the size)
+// ----------------------------------------------------------------------------
+template <int BYTES>
+QES_D void cp_async(void* smem, const void* g, bool valid) {         // zero-filled when not valid
+  const unsigned d = (unsigned)__cvta_generic_to_shared(smem);
+  const int n = valid ? BYTES : 0;
+  if constexpr (BYTES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(g), "r"(n) : "memory");
+  else asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(d), "l"(g), "n"(BYTES), "r"(n) : "memory");
+}
+QES_D void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+QES_D void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }

@@ -115,14 +115,299 @@ QES_D void eloc_moves_block(int kb, int64_t sb, int ns, int nh, int64_t n_sample
   }
 }
 
+// ----------------------------------------------------------------------------
+// Register-tiled form for one problem.  A block takes 32 moves x 32 RS samples with 8 x 32 threads; a thread
+// owns 4 consecutive moves x RS samples (row, row + 32, ...).  Per chunk of ELOC_RENORM units the block holds C
+// and S (unit-major, real and imaginary parts apart) and T (sample-major) in shared memory, double-buffered:
+// T by asynchronous copies, C and S through registers, both requested a chunk ahead.  A factor is C + t (g S)
+// with g = -sigma_i: the sign goes into t by one xor.  The sign bit of (move, sample) shares a register with the
+// product's exponent (biased, so that it cannot carry into the sign).
+// Factors, roundings and the order of the sum over the 32 moves are those of the form above, so the energies
+// are bit-identical to it: in a stochastic-reconfiguration step even the last bits of E_loc reach the
+// weights through the near-null directions of S.
+// Bound by the FP32 and integer pipes: 2 multiply-adds and 1 xor per real factor, 8 and 2 per complex one.
+// Measured (B200, 16,384 samples unless stated), the form above / this one: 20x20 TFIM x 1,600 real 3.81 / 1.51 ms
+// (0.57 ms at the FP32 rate), TFIM-100 x 200 real 173 / 88 us, 10x10 x 200 complex 452 / 401 us, 6x6 J1-J2 x 144
+// complex, 8,192 samples, 139 / 122 us.  Packed f32x2 multiply-adds ran the same (1.53 ms, 425 us); four complex
+// samples per thread at 128 registers 413 us.
+// ----------------------------------------------------------------------------
+constexpr int ELT_K = 4;                 // moves per thread
+constexpr int ELT_COLS = 8;              // thread columns: 32 moves
+constexpr int ELT_ROWS = 32;             // thread rows
+constexpr int ELT_THREADS = ELT_COLS * ELT_ROWS;
+constexpr uint32_t ELT_EX0 = 1u << 30;   // bias of the exponent field
+
+QES_D float xor_sign(float t, uint32_t v) { return __uint_as_float(__float_as_uint(t) ^ (v & 0x80000000u)); }
+// VEC: rows of C, S and T start on 16-byte boundaries every 4 (real) / 2 (complex) elements
+template <class T, int RS, bool VEC>
+__global__ void __launch_bounds__(ELT_THREADS, ScalarTraits<T>::is_complex ? 3 : 2) eloc_tile_kernel(
+    int ns, int nh, int64_t n_samples, const uint32_t* __restrict__ bits, const T* __restrict__ tanh_theta, int K,
+    const int32_t* __restrict__ mi, const int32_t* __restrict__ mj,
+    const int32_t* __restrict__ mkind, const float4* __restrict__ mcoef, const T* __restrict__ Ct,
+    const T* __restrict__ St, const T* __restrict__ A, float2* __restrict__ partial /* [gridDim.x][n_samples] */) {
+  constexpr bool CPLX = ScalarTraits<T>::is_complex;
+  constexpr int H = CPLX ? 2 : 1;
+  constexpr int UM = ELOC_RENORM;
+  constexpr int TK = ELT_K * ELT_COLS, TS = RS * ELT_ROWS;
+  constexpr int TW = H * UM + 4;                                     // floats per staged T row
+  constexpr int NT = 2 * H;                                          // C, S | C.re, C.im, S.re, S.im
+  extern __shared__ __align__(16) float elt_sm[];
+  float* s_cs = elt_sm;                                              // [2][NT][UM][TK]
+  float* s_t = elt_sm + 2 * NT * UM * TK;                            // [2][TS][TW]
+  float2* s_red = reinterpret_cast<float2*>(elt_sm);                 // [ELT_COLS][TS], after the products
+  const int tid = threadIdx.x;
+  const int col = tid % ELT_COLS, row = tid / ELT_COLS;
+  const int k0 = blockIdx.x * TK;
+  const int64_t s0 = (int64_t)blockIdx.y * TS;
+  const int nw = n_words(ns);
+
+  // staging: this thread's C or S entries (table, unit, 4 moves) and its share of T
+  const int st_tab = tid >> 7, st_u = (tid >> 3) & (UM - 1), st_k = k0 + ELT_K * (tid & 7);
+  float cs[H][ELT_K];
+  auto load_cs = [&](int m0) {
+    const int m = m0 + st_u;
+    const T* src = (st_tab ? St : Ct) + (int64_t)m * K + st_k;
+    const T fill = st_tab ? ScalarTraits<T>::zero() : ScalarTraits<T>::one();
+    if (VEC && m < nh && st_k + ELT_K <= K) {
+      if constexpr (CPLX) {
+        const float4 x = __ldg(reinterpret_cast<const float4*>(src)), y = __ldg(reinterpret_cast<const float4*>(src) + 1);
+        cs[0][0] = x.x; cs[1][0] = x.y; cs[0][1] = x.z; cs[1][1] = x.w;
+        cs[0][2] = y.x; cs[1][2] = y.y; cs[0][3] = y.z; cs[1][3] = y.w;
+      } else {
+        const float4 x = __ldg(reinterpret_cast<const float4*>(src));
+        cs[0][0] = x.x; cs[0][1] = x.y; cs[0][2] = x.z; cs[0][3] = x.w;
+      }
+    } else {
+#pragma unroll
+      for (int a = 0; a < ELT_K; ++a) {
+        const T x = (m < nh && st_k + a < K) ? src[a] : fill;        // a factor of one past the units and moves
+        if constexpr (CPLX) {
+          cs[0][a] = x.x;
+          cs[1][a] = x.y;
+        } else {
+          cs[0][a] = x;
+        }
+      }
+    }
+  };
+  auto store_cs = [&](int buf) {
+    float* o = s_cs + ((buf * NT + H * st_tab) * UM + st_u) * TK + ELT_K * (tid & 7);
+#pragma unroll
+    for (int h = 0; h < H; ++h)
+      *reinterpret_cast<float4*>(o + h * UM * TK) = make_float4(cs[h][0], cs[h][1], cs[h][2], cs[h][3]);
+  };
+  auto copy_t = [&](int m0, int buf) {
+    constexpr int PER = VEC ? 16 / (int)sizeof(T) : 1;               // elements per copy
+    constexpr int CPR = UM / PER;                                    // copies per row
+#pragma unroll
+    for (int e = tid; e < TS * CPR; e += ELT_THREADS) {
+      const int ss = e / CPR, u = (e % CPR) * PER;
+      const bool ok = s0 + ss < n_samples && m0 + u < nh;            // VEC: nh is a multiple of PER
+      cp_async<PER * (int)sizeof(T)>(s_t + (size_t)(buf * TS + ss) * TW + H * u,
+                                     ok ? tanh_theta + (s0 + ss) * nh + m0 + u : tanh_theta, ok);
+    }
+    cp_async_commit();
+  };
+  copy_t(0, 0);
+  load_cs(0);
+
+  // sign bit and activity of every (move, sample) of the thread
+  uint32_t v[ELT_K][RS];
+  uint32_t act = 0;
+#pragma unroll
+  for (int a = 0; a < ELT_K; ++a) {
+    const int k = k0 + ELT_K * col + a;
+    const bool kval = k < K;
+    const int kind = kval ? mkind[k] : 0, i = kval ? mi[k] : 0;
+    const int j = (kval && kind != QES_MOVE_FLIP1) ? mj[k] : i;
+#pragma unroll
+    for (int q = 0; q < RS; ++q) {
+      const int64_t s = s0 + ELT_ROWS * q + row;
+      const bool ok = kval && s < n_samples;
+      const uint32_t* w = bits + (ok ? s : 0) * nw;
+      const uint32_t bi = bit_of(w, i), bj = bit_of(w, j);
+      v[a][q] = (bi << 31) | ELT_EX0;                                // g = -sigma_i: negative for spin up
+      const bool on = ok && (kind == QES_MOVE_FLIP1 || ((kind == QES_MOVE_PAIR_ANTI) == (bi != bj)));
+      act |= (on ? 1u : 0u) << (a * RS + q);
+    }
+  }
+  float accr[ELT_K][RS], acci[ELT_K][RS];
+#pragma unroll
+  for (int a = 0; a < ELT_K; ++a)
+#pragma unroll
+    for (int q = 0; q < RS; ++q) {
+      accr[a][q] = 1.f;
+      acci[a][q] = 0.f;
+    }
+  store_cs(0);
+  cp_async_wait_all();
+  __syncthreads();
+
+  const int nchunk = (nh + UM - 1) / UM;
+  for (int ch = 0; ch < nchunk; ++ch) {
+    const int buf = ch & 1;
+    if (ch + 1 < nchunk) {
+      copy_t((ch + 1) * UM, buf ^ 1);
+      load_cs((ch + 1) * UM);
+    }
+    const float* cb = s_cs + buf * NT * UM * TK + ELT_K * col;
+    const float* tb = s_t + (size_t)buf * TS * TW + (size_t)row * TW;
+    constexpr int UV = 4 / H;                                        // units per 16-byte load of T
+    // units past nh (only in the last chunk): C = 1, S = 0, t = 0, an exact factor of one
+#pragma unroll
+    for (int u0 = 0; u0 < UM; u0 += UV) {
+      float4 t4[RS];
+#pragma unroll
+      for (int q = 0; q < RS; ++q) t4[q] = *reinterpret_cast<const float4*>(tb + (size_t)q * ELT_ROWS * TW + H * u0);
+#pragma unroll
+      for (int uu = 0; uu < UV; ++uu) {
+        float c[2 * H][ELT_K];
+#pragma unroll
+        for (int h = 0; h < 2 * H; ++h) {
+          const float4 x = *reinterpret_cast<const float4*>(cb + (h * UM + u0 + uu) * TK);
+          c[h][0] = x.x; c[h][1] = x.y; c[h][2] = x.z; c[h][3] = x.w;
+        }
+#pragma unroll
+        for (int q = 0; q < RS; ++q) {
+          const float tv[4] = {t4[q].x, t4[q].y, t4[q].z, t4[q].w};
+#pragma unroll
+          for (int a = 0; a < ELT_K; ++a) {
+            if constexpr (CPLX) {
+              const float tr = xor_sign(tv[2 * uu], v[a][q]), ti = xor_sign(tv[2 * uu + 1], v[a][q]);
+              const float fr = __fmaf_rn(tr, c[2][a], __fmaf_rn(-ti, c[3][a], c[0][a]));
+              const float fi = __fmaf_rn(tr, c[3][a], __fmaf_rn(ti, c[2][a], c[1][a]));
+              // contractions written out: the same roundings in every instantiation
+              const float r = __fmaf_rn(accr[a][q], fr, -__fmul_rn(acci[a][q], fi));
+              acci[a][q] = __fmaf_rn(accr[a][q], fi, __fmul_rn(acci[a][q], fr));
+              accr[a][q] = r;
+            } else {
+              accr[a][q] *= __fmaf_rn(xor_sign(tv[uu], v[a][q]), c[1][a], c[0][a]);
+            }
+          }
+        }
+      }
+    }
+    // power-of-two renormalisation (exact) of a thread whose products have left 2^-7 .. 2^9: most never do.
+    // An exponent e in [120, 135] has e + 8 = 1000xxxx in binary.
+    uint32_t far = 0;
+#pragma unroll
+    for (int a = 0; a < ELT_K; ++a)
+#pragma unroll
+      for (int q = 0; q < RS; ++q) {
+        const float m = CPLX ? fmaxf(fabsf(accr[a][q]), fabsf(acci[a][q])) : accr[a][q];
+        far |= (__float_as_uint(m) + (8u << 23)) ^ 0x40000000u;
+      }
+    if (far & 0x78000000u) {
+#pragma unroll
+      for (int a = 0; a < ELT_K; ++a)
+#pragma unroll
+        for (int q = 0; q < RS; ++q) {
+          int ex = 0;
+          if constexpr (CPLX) {
+            float2 z = make_float2(accr[a][q], acci[a][q]);
+            renorm(z, ex);
+            accr[a][q] = z.x;
+            acci[a][q] = z.y;
+          } else {
+            renorm(accr[a][q], ex);
+          }
+          v[a][q] += (uint32_t)ex;                                   // |sum| < 2^30: no carry into the sign bit
+        }
+    }
+    if (ch + 1 < nchunk) {
+      store_cs(buf ^ 1);                                             // its last readers passed the previous barrier
+      cp_async_wait_all();
+    }
+    __syncthreads();
+  }
+
+  // contribution = coef * exp(g*2*A + ex*ln2) * acc   (g = -sigma_i), summed over the 32 moves as a warp
+  // would by xor shuffles: move distances 16, 8, 4 (thread columns), then 2 and 1 (a thread's own moves)
+  float2 sum[ELT_K];
+#pragma unroll
+  for (int a = 0; a < ELT_K; ++a) {
+    const int k = k0 + ELT_K * col + a;
+    float4 cf = make_float4(0.f, 0.f, 0.f, 0.f);
+    T Ak = ScalarTraits<T>::zero();
+    if (k < K) {
+      cf = mcoef[k];
+      Ak = A[k];
+    }
+    __syncthreads();                                                 // the staged operands, the previous move's sums
+#pragma unroll
+    for (int q = 0; q < RS; ++q) {
+      float2 e = make_float2(0.f, 0.f);
+      if ((act >> (a * RS + q)) & 1u) {
+        const float g = (v[a][q] >> 31) ? -1.f : 1.f;
+        int ex = (int)(v[a][q] & 0x7fffffffu) - (int)ELT_EX0;
+        const float sig = -g;
+        const float2 coef = make_float2(cf.x + sig * cf.z, cf.y + sig * cf.w);
+        const float2 z = to_c(scal(2.f * g, Ak));
+        if constexpr (CPLX) {
+          float2 acc = make_float2(accr[a][q], acci[a][q]);
+          renorm(acc, ex);
+          const float lx = __fmul_rn(0.69314718055994531f, (float)ex);
+          const float2 x = expx(make_float2(__fadd_rn(z.x, lx), z.y));
+          e = coef * (x * acc);
+        } else {
+          float acc = accr[a][q];
+          renorm(acc, ex);
+          const float lx = __fmul_rn(0.69314718055994531f, (float)ex);
+          const float m = expf(__fadd_rn(z.x, lx)) * acc;
+          e = make_float2(coef.x * m, coef.y * m);
+        }
+      }
+      s_red[col * TS + ELT_ROWS * q + row] = e;
+    }
+    __syncthreads();
+    if (tid < TS)
+      sum[a] = ((s_red[tid] + s_red[4 * TS + tid]) + (s_red[2 * TS + tid] + s_red[6 * TS + tid])) +
+               ((s_red[TS + tid] + s_red[5 * TS + tid]) + (s_red[3 * TS + tid] + s_red[7 * TS + tid]));
+  }
+  if (tid < TS && s0 + tid < n_samples)
+    partial[(int64_t)blockIdx.x * n_samples + s0 + tid] = (sum[0] + sum[2]) + (sum[1] + sum[3]);
+}
+
+QES_HD int eloc_kblocks(int K) { return (K + 31) / 32; }
+
+template <class T, int RS>
+constexpr size_t eloc_tile_smem() {
+  constexpr int H = ScalarTraits<T>::is_complex ? 2 : 1, NT = 2 * H;
+  return std::max((size_t)(2 * NT * ELOC_RENORM * ELT_K * ELT_COLS + 2 * RS * ELT_ROWS * (H * ELOC_RENORM + 4)) * sizeof(float),
+                  (size_t)ELT_COLS * RS * ELT_ROWS * sizeof(float2));
+}
+
+template <class T, int RS>
+static int launch_eloc_tiles(int ns, int nh, int64_t n, const uint32_t* bits, const T* tt, const qes_hamiltonian* ham,
+                             const T* Ct, const T* St, const T* A, float2* partial, cudaStream_t st) {
+  const int K = ham->n_moves;
+  const int64_t nsb = (n + RS * ELT_ROWS - 1) / (RS * ELT_ROWS);
+  QES_ARG_CHECK(nsb <= 65535, "qes_local_energy: too many samples for one launch");
+  constexpr int E = 16 / (int)sizeof(T);
+  const uintptr_t al = reinterpret_cast<uintptr_t>(tt) | reinterpret_cast<uintptr_t>(Ct) | reinterpret_cast<uintptr_t>(St);
+  const bool vec = nh % E == 0 && K % E == 0 && (al & 15) == 0;
+  constexpr size_t smem = eloc_tile_smem<T, RS>();
+  auto kern = vec ? eloc_tile_kernel<T, RS, true> : eloc_tile_kernel<T, RS, false>;
+  QES_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  kern<<<dim3(eloc_kblocks(K), (unsigned)nsb), ELT_THREADS, smem, st>>>(ns, nh, n, bits, tt, K, ham->move_i, ham->move_j,
+                                                                       ham->move_kind, (const float4*)ham->move_coef, Ct,
+                                                                       St, A, partial);
+  QES_LAUNCH_CHECK();
+  return QES_OK;
+}
+
+// samples per thread: as many as leave two blocks per SM (complex: at most two, three blocks of 80 registers
+// per SM), down to one
 template <class T>
-__global__ void __launch_bounds__(32 * ELOC_ROWS) eloc_moves_kernel(
-    int ns, int nh, int64_t n_samples, const uint32_t* __restrict__ bits, const T* __restrict__ tanh_theta,
-    int K, const int32_t* __restrict__ mi, const int32_t* __restrict__ mj, const int32_t* __restrict__ mkind,
-    const float4* __restrict__ mcoef, const T* __restrict__ Ct, const T* __restrict__ St,
-    const T* __restrict__ A, float2* __restrict__ partial /* [gridDim.x][n_samples] */) {
-  eloc_moves_block<T>(blockIdx.x, blockIdx.y, ns, nh, n_samples, bits, tanh_theta, K, mi, mj, mkind, mcoef, Ct, St, A,
-                      partial);
+static int launch_eloc_moves(int ns, int nh, int64_t n, const uint32_t* bits, const T* tt, const qes_hamiltonian* ham,
+                             const T* Ct, const T* St, const T* A, float2* partial, cudaStream_t st) {
+  auto blocks = [&](int rs) {
+    return (int64_t)eloc_kblocks(ham->n_moves) * ((n + rs * ELT_ROWS - 1) / (rs * ELT_ROWS));
+  };
+  if constexpr (!ScalarTraits<T>::is_complex)
+    if (blocks(4) >= 2 * 148) return launch_eloc_tiles<T, 4>(ns, nh, n, bits, tt, ham, Ct, St, A, partial, st);
+  if (blocks(2) >= 2 * 148) return launch_eloc_tiles<T, 2>(ns, nh, n, bits, tt, ham, Ct, St, A, partial, st);
+  return launch_eloc_tiles<T, 1>(ns, nh, n, bits, tt, ham, Ct, St, A, partial, st);
 }
 
 // diagonal part + move partials of sample s
@@ -141,17 +426,51 @@ QES_D void eloc_reduce_sample(int64_t s, int ns, int64_t n_samples, const uint32
   eloc[s] = e;
 }
 
-__global__ void eloc_reduce_kernel(int ns, int64_t n_samples, const uint32_t* __restrict__ bits, int nkb,
-                                   const float2* __restrict__ partial, int n_zf, const int32_t* __restrict__ zf_site,
-                                   const float* __restrict__ zf_h, int n_zz, const int32_t* __restrict__ zz_i,
-                                   const int32_t* __restrict__ zz_j, const float* __restrict__ zz_J,
-                                   float2* __restrict__ eloc) {
-  const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+// A thread per sample, the terms in order.  Spin words and the terms are staged in shared memory (word-major and
+// 128 terms at a time): reading both through L1 for each of the 800 bonds of a 20x20 lattice left the
+// threads waiting on loads.
+constexpr int ELR_THREADS = 64, ELR_TERMS = 128, ELR_WORDS = 64;     // more words than this are read from global memory
+__global__ void __launch_bounds__(ELR_THREADS) eloc_reduce_kernel(int ns, int64_t n_samples, const uint32_t* __restrict__ bits,
+                                                                 int nkb, const float2* __restrict__ partial, int n_zf,
+                                                                 const int32_t* __restrict__ zf_site,
+                                                                 const float* __restrict__ zf_h, int n_zz,
+                                                                 const int32_t* __restrict__ zz_i,
+                                                                 const int32_t* __restrict__ zz_j,
+                                                                 const float* __restrict__ zz_J,
+                                                                 float2* __restrict__ eloc) {
+  __shared__ uint32_t s_w[ELR_WORDS][ELR_THREADS];
+  __shared__ int2 s_ij[ELR_TERMS];
+  __shared__ float s_J[ELR_TERMS];
+  const int tid = threadIdx.x, nw = n_words(ns);
+  const int64_t s0 = (int64_t)blockIdx.x * ELR_THREADS, s = s0 + tid;
+  const int rows = (int)min((int64_t)ELR_THREADS, n_samples - s0);
+  const bool staged = nw <= ELR_WORDS;
+  if (staged)
+    for (int e = tid; e < rows * nw; e += ELR_THREADS) s_w[e % nw][e / nw] = bits[s0 * nw + e];
+  const uint32_t* gw = bits + (s < n_samples ? s : s0) * nw;
+  auto bit = [&](int i) { return ((staged ? s_w[i >> 5][tid] : gw[i >> 5]) >> (i & 31)) & 1u; };
+  float d = 0.f;
+  for (int t0 = 0; t0 < n_zf + n_zz; t0 += ELR_TERMS) {
+    __syncthreads();                                                 // words staged; previous terms consumed
+    for (int q = tid; q < ELR_TERMS && t0 + q < n_zf + n_zz; q += ELR_THREADS) {
+      const int t = t0 + q;
+      s_ij[q] = t < n_zf ? make_int2(zf_site[t], -1) : make_int2(zz_i[t - n_zf], zz_j[t - n_zf]);
+      s_J[q] = t < n_zf ? zf_h[t] : zz_J[t - n_zf];
+    }
+    __syncthreads();
+    const int nt = min(ELR_TERMS, n_zf + n_zz - t0);
+#pragma unroll 4
+    for (int q = 0; q < nt; ++q) {
+      const int2 ij = s_ij[q];
+      const uint32_t bi = bit(ij.x), bj = ij.y < 0 ? 1u : bit(ij.y);
+      d += s_J[q] * (bi == bj ? 1.f : -1.f);                         // a field term: sigma_i
+    }
+  }
   if (s >= n_samples) return;
-  eloc_reduce_sample(s, ns, n_samples, bits, nkb, partial, n_zf, zf_site, zf_h, n_zz, zz_i, zz_j, zz_J, eloc);
+  float2 e = make_float2(d, 0.f);
+  for (int b = 0; b < nkb; ++b) e = e + partial[(int64_t)b * n_samples + s];
+  eloc[s] = e;
 }
-
-QES_HD int eloc_kblocks(int K) { return (K + 31) / 32; }
 
 extern "C" int qes_local_energy_workspace_bytes(int dtype, int ns, int nh, int64_t n_samples, int n_moves,
                                                 size_t* bytes) {
@@ -177,29 +496,19 @@ extern "C" int qes_local_energy(int dtype, int ns, int nh, int64_t n_samples, co
     return QES_ERR_WORKSPACE;
   }
   cudaStream_t st = (cudaStream_t)stream;
-  const int nkb = eloc_kblocks(K);
   float2* partial = (float2*)workspace;
   if (K > 0) {
     QES_ARG_CHECK(tanh_theta && Ct && St && A && ham->move_i && ham->move_j && ham->move_kind && ham->move_coef,
                   "qes_local_energy: null move pointer");
-    const int64_t nsb = (n_samples + ELOC_SB - 1) / ELOC_SB;
-    QES_ARG_CHECK(nsb <= 65535, "qes_local_energy: too many samples for one launch");
-    dim3 grid(nkb, (unsigned)nsb), block(32, ELOC_ROWS);
-    if (dtype == QES_DTYPE_F32)
-      eloc_moves_kernel<float><<<grid, block, 0, st>>>(ns, nh, n_samples, bits, (const float*)tanh_theta, K,
-                                                       ham->move_i, ham->move_j, ham->move_kind,
-                                                       (const float4*)ham->move_coef, (const float*)Ct,
-                                                       (const float*)St, (const float*)A, partial);
-    else
-      eloc_moves_kernel<float2><<<grid, block, 0, st>>>(ns, nh, n_samples, bits, (const float2*)tanh_theta, K,
-                                                        ham->move_i, ham->move_j, ham->move_kind,
-                                                        (const float4*)ham->move_coef, (const float2*)Ct,
-                                                        (const float2*)St, (const float2*)A, partial);
-    QES_LAUNCH_CHECK();
+    const int rc = dtype == QES_DTYPE_F32
+                       ? launch_eloc_moves<float>(ns, nh, n_samples, bits, (const float*)tanh_theta, ham, (const float*)Ct,
+                                                  (const float*)St, (const float*)A, partial, st)
+                       : launch_eloc_moves<float2>(ns, nh, n_samples, bits, (const float2*)tanh_theta, ham,
+                                                   (const float2*)Ct, (const float2*)St, (const float2*)A, partial, st);
+    if (rc) return rc;
   }
-  const int bs = 256;
-  eloc_reduce_kernel<<<(unsigned)((n_samples + bs - 1) / bs), bs, 0, st>>>(
-      ns, n_samples, bits, K > 0 ? nkb : 0, partial, ham->n_zfield, ham->zf_site, ham->zf_h, ham->n_zz, ham->zz_i,
+  eloc_reduce_kernel<<<(unsigned)((n_samples + ELR_THREADS - 1) / ELR_THREADS), ELR_THREADS, 0, st>>>(
+      ns, n_samples, bits, K > 0 ? eloc_kblocks(K) : 0, partial, ham->n_zfield, ham->zf_site, ham->zf_h, ham->n_zz, ham->zz_i,
       ham->zz_j, ham->zz_J, (float2*)eloc_out);
   QES_LAUNCH_CHECK();
   return QES_OK;

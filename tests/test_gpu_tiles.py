@@ -1,0 +1,83 @@
+"""Register-tiled kernels at the edges of their tiles, against float64 (the float32 bar: 1e-5)."""
+
+import numpy as np
+import pytest
+import torch
+
+from oracle import lattice as olat, hamiltonian as oH, rbm as orbm, estimator as oest
+import pyqusolver_b200 as qb
+from pyqusolver_b200 import device as dv
+from pyqusolver_b200.rbm import RBM
+
+pytestmark = pytest.mark.gpu
+
+
+def _problem(cplx, ns, nh, n, scale, seed=3):
+    net = RBM((ns,), n_hidden=nh, dtype="complex64" if cplx else "float32", seed=seed, init_scale=scale)
+    rng = np.random.default_rng(seed)
+    st = np.where(rng.random((n, ns)) < 0.5, 0.5, -0.5)
+    p = orbm.RBMParams.from_flat(net.flat.cpu().numpy().astype(np.complex128 if cplx else np.float64), ns, nh)
+    return net, st, dv.pack_states(st), p
+
+
+# sites per staged slice (32), hidden units per pass (128) and per thread (4), samples per thread (1, 2, 4, 8) and
+# per block; 1,184 and 9,500 rows reach the two- and eight-sample tiles of the real form
+@pytest.mark.parametrize("cplx,ns,nh,n", [(False, 5, 3, 1), (True, 33, 129, 9), (False, 32, 128, 1185), (True, 31, 130, 2400),
+                                           (False, 64, 5, 9500), (True, 3, 4, 4800), (False, 70, 260, 4750)])
+def test_forward_tiles(cplx, ns, nh, n):
+    net, st, bits, p = _problem(cplx, ns, nh, n, 0.05)
+    th, tn, lp = dv.rbm_forward(net.flat, ns, nh, bits, theta=True)
+    sg = np.where(st > 0, 1.0, -1.0)
+    ref = orbm.theta(p, sg)
+    tol = lambda x: 1e-5 * max(1.0, np.max(np.abs(x)))
+    assert np.max(np.abs(th.cpu().numpy() - ref)) <= tol(ref)
+    # tanh of a complex theta near a pole amplifies theta's rounding: checked at the path's own theta
+    own = np.tanh(th.cpu().numpy().astype(ref.dtype))
+    assert np.max(np.abs(tn.cpu().numpy() - own)) <= tol(own)
+    d = lp.cpu().numpy() - orbm.log_psi(p, sg)
+    assert np.max(np.abs(d.real)) <= tol(ref) * 10
+    if cplx:
+        assert np.max(np.abs(np.angle(np.exp(1j * d.imag)))) <= tol(ref) * 10
+    _, t2, none = dv.rbm_forward(net.flat, ns, nh, bits, logpsi=False)
+    assert none is None and torch.equal(t2, tn)
+
+
+# moves per thread (4) and per block (32), units per renormalisation (16), samples per thread and block;
+# scale 1.5: products that leave 2^+-8 and are renormalised
+@pytest.mark.parametrize("lx,ly,model,cplx,nh,n,scale", [
+    (3, 1, "tfim", False, 1, 1, 0.1), (17, 1, "tfim", False, 33, 70, 0.1), (65, 1, "tfim", False, 16, 4300, 0.1),
+    (5, 3, "xxz", True, 17, 130, 0.1), (9, 9, "xxz", True, 31, 1300, 0.1), (7, 3, "j1j2", True, 48, 2500, 0.1),
+    (33, 1, "tfim", False, 40, 257, 1.5), (4, 3, "j1j2", True, 40, 65, 1.0), (40, 1, "tfim", True, 20, 12000, 0.1)])
+def test_local_energy_tiles(lx, ly, model, cplx, nh, n, scale):
+    dim, ns = (2 if ly > 1 else 1), lx * ly
+    L, OL = qb.SquareLattice(dim, lx, ly), olat.SquareLattice(dim, lx, ly)
+    if model == "tfim":
+        m, terms = qb.TransverseFieldIsing(L, j=1.0, hx=0.7, hz=0.3), oH.tfim_terms(OL, 1.0, 0.7, 0.3)
+    elif model == "xxz":
+        m, terms = qb.XXZ(L, jxy=-1.0, jz=-1.0), oH.xxz_terms(OL, -1.0, -1.0)
+    else:
+        m, terms = qb.J1J2Model(L, J1=-1.0, J2=-0.5), oH.j1j2_terms(OL, -1.0, -0.5)
+    net, st, bits, p = _problem(cplx, ns, nh, n, scale / np.sqrt(ns))
+    _, tn, _ = dv.rbm_forward(net.flat, ns, nh, bits, logpsi=False)
+    h = dv.DeviceHamiltonian(m.lower())
+    tables = dv.move_tables(net.flat, ns, nh, h.move_i, h.move_j, h.move_kind, move_major=False)
+    e = dv.local_energy(net.flat, ns, nh, bits, tn, h, tables).cpu().numpy()
+    rows = np.unique(np.linspace(0, n - 1, 40).astype(int))       # the full re-evaluation is the slow side
+    ref = oest.local_energy_full(p, terms, st[rows])
+    assert np.max(np.abs(e[rows] - ref)) <= 1e-5 * max(1.0, np.max(np.abs(ref)))
+    assert np.all(np.isfinite(e))
+
+
+# rows whose W blocks start on and off 16-byte boundaries (odd P, odd nh), fewer elements than one vector
+@pytest.mark.parametrize("cplx,ns,nh,n", [(False, 1, 1, 3), (False, 5, 3, 7), (True, 4, 3, 5), (True, 7, 8, 2),
+                                           (False, 33, 130, 4), (True, 20, 41, 9)])
+def test_log_derivative_rows(cplx, ns, nh, n):
+    net, st, bits, p = _problem(cplx, ns, nh, n, 0.2)
+    _, tn, _ = dv.rbm_forward(net.flat, ns, nh, bits, logpsi=False)
+    O = dv.log_derivatives(net.flat, ns, nh, bits, tn)
+    sg = torch.as_tensor(np.where(st > 0, 1.0, -1.0)).cuda().to(tn.dtype)
+    ref = torch.cat([sg, tn, (sg[:, :, None] * tn[:, None, :]).reshape(n, -1)], dim=1)
+    assert torch.equal(O, ref)
+    wide = torch.full((n, dv.n_params(ns, nh) + 3), 7.0, dtype=tn.dtype, device="cuda")       # rows of a wider array
+    dv.log_derivatives(net.flat, ns, nh, bits, tn, out=wide)
+    assert torch.equal(wide[:, :-3], ref) and bool((wide[:, -3:] == 7.0).all())
