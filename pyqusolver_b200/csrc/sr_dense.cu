@@ -13,7 +13,8 @@
 //      accumulator (the lo*lo term is below 2^-16 relative).
 //   4. S from G in float64 (S_re = G_rr + G_ii, S_im = G_ri - G_ir, / Ns), full Hermitian.
 //   5. A = S + shift, L L^H = A by 64-column blocks (diagonal block in one CTA, panel triangular
-//      solve, register-tiled trailing update of the lower triangle), L y = F, L^H x = y.
+//      solve, register-tiled trailing update of the lower triangle); F^H rides along as one more row,
+//      which becomes y^H of L y = F; L^H x = y block by block.
 //
 // Every mbarrier wait is bounded; a time-out sets QES_ERR_TIMEOUT in the status word, the kernel
 // still waits (bounded) for its own MMAs, frees its TMEM and returns.
@@ -56,11 +57,6 @@ __device__ __forceinline__ double zsub(double a, double b) { return a - b; }
 __device__ __forceinline__ double2 zsub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
 __device__ __forceinline__ double zscale(double s, double a) { return s * a; }
 __device__ __forceinline__ double2 zscale(double s, double2 a) { return make_double2(s * a.x, s * a.y); }
-// a - b * conj(c)
-__device__ __forceinline__ double zmsc(double a, double b, double c) { return fma(-b, c, a); }
-__device__ __forceinline__ double2 zmsc(double2 a, double2 b, double2 c) {
-  return make_double2(a.x - (b.x * c.x + b.y * c.y), a.y - (b.y * c.x - b.x * c.y));
-}
 __device__ __forceinline__ double zfrom(double x, double) { return x; }
 __device__ __forceinline__ double2 zfrom(double x, double2) { return make_double2(x, 0.0); }
 __device__ __forceinline__ double zzero(double) { return 0.0; }
@@ -89,28 +85,60 @@ __device__ __forceinline__ V o_elem(int ns, int nh, int64_t p, const uint32_t* w
 
 }  // namespace
 
-// out_p = sum_s conj(O_sp) g_s  (float64; one thread per parameter, samples in a fixed order).
-// With g_s = p_s / Ns it is conj(O-bar); with g_s = p_s (E_s - <E>) / Ns it is the force F.
+// out_p = sum_s conj(O_sp) g_s  (float64).  With g_s = p_s / Ns it is conj(O-bar); with g_s = p_s (E_s - <E>) / Ns
+// it is the force F.  The parameters form a (ns + 1) x (nh + 1) array: entry (i, m) of W, b in row ns
+// (spin +1), a in column nh (t = 1).  A block of 4 rows x 32 columns stages q = conj(t) g for 32 samples, the
+// next 32 samples' T already requested; each thread adds its +-q in sample order, one chain of additions.
+// Bound by the latency of a stage's loads (the flat form of one thread per parameter, which read spins, t and g
+// from global memory and divided its index by nh for every sample, took 4.6 ms for 5,364 complex parameters and
+// 8,192 samples; this one 0.28 ms, the same sums in the same order).
+constexpr int OHG_S = 32, OHG_R = 4;
 template <class V>
-__global__ void __launch_bounds__(256) dense_ohg_kernel(int ns, int nh, int64_t n_samples,
+__global__ void __launch_bounds__(32 * OHG_R) dense_ohg_kernel(int ns, int nh, int64_t n_samples,
                                                          const uint32_t* __restrict__ bits,
                                                          const typename DenseT<V>::T* __restrict__ tt,
                                                          const double2* __restrict__ g, V* __restrict__ out) {
-  const int64_t P = (int64_t)ns + nh + (int64_t)ns * nh;
-  const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= P) return;
-  const int nw = n_words(ns);
-  V acc = zzero(V());
-  for (int64_t s = 0; s < n_samples; ++s) {
-    const V o = o_elem<V>(ns, nh, p, bits + s * nw, tt + s * nh);
-    const double2 gs = g[s];
-    if constexpr (DenseT<V>::cplx) {
-      acc = zadd(acc, zmul(zconj(o), make_double2(gs.x, gs.y)));
-    } else {
-      acc = acc + o * gs.x;
+  using T = typename DenseT<V>::T;
+  __shared__ V q[2][OHG_S][33];
+  __shared__ uint32_t sb[2][OHG_R];                             // per row of the block: its spins over the samples
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int m = blockIdx.x * 32 + tx, i = blockIdx.y * OHG_R + ty, nw = n_words(ns);
+  // staging: thread (tx, ty) takes unit m of the samples ty, ty + OHG_R, ...; lane tx the spin of row ty, sample tx
+  T tv[OHG_S / OHG_R];
+  double2 gv[OHG_S / OHG_R];
+  uint32_t bit = 0;
+  auto load = [&](int64_t c0) {
+#pragma unroll
+    for (int e = 0; e < OHG_S / OHG_R; ++e) {
+      const int64_t s = c0 + ty + OHG_R * e;
+      gv[e] = s < n_samples ? g[s] : make_double2(0.0, 0.0);
+      if (s < n_samples && m < nh) tv[e] = tt[s * nh + m];
+      else tv[e] = ScalarTraits<T>::one();                  // column nh: t = 1
     }
+    const int64_t s = c0 + tx;
+    bit = (s < n_samples && i < ns) ? ((bits[s * nw + (i >> 5)] >> (i & 31)) & 1u) : 1u;
+  };
+  load(0);
+  V acc = zzero(V());
+  int buf = 0;
+  for (int64_t c0 = 0; c0 < n_samples; c0 += OHG_S, buf ^= 1) {
+#pragma unroll
+    for (int e = 0; e < OHG_S / OHG_R; ++e) {
+      if constexpr (DenseT<V>::cplx) q[buf][ty + OHG_R * e][tx] = zmul(zconj(t_to_d(tv[e], V())), gv[e]);
+      else q[buf][ty + OHG_R * e][tx] = t_to_d(tv[e], V()) * gv[e].x;
+    }
+    const uint32_t word = __ballot_sync(0xffffffffu, bit != 0);
+    if (tx == 0) sb[buf][ty] = word;
+    __syncthreads();                                        // staged; the other buffer's readers are past it
+    if (c0 + OHG_S < n_samples) load(c0 + OHG_S);
+    const uint32_t w = sb[buf][ty];
+    const int nc = (int)min((int64_t)OHG_S, n_samples - c0);
+#pragma unroll 8
+    for (int k = 0; k < nc; ++k) acc = zadd(acc, zscale(((w >> k) & 1u) ? 1.0 : -1.0, q[buf][k][tx]));
   }
-  out[p] = acc;
+  if (i < ns && m < nh) out[ns + nh + (int64_t)i * nh + m] = acc;
+  else if (i == ns && m < nh) out[ns + m] = acc;
+  else if (i < ns && m == nh) out[i] = acc;
 }
 
 // X^T as BF16 hi/lo core-matrix tiles: row r of the real embedding (r < P: Re O_c[:, r]; complex:
@@ -317,79 +345,182 @@ __global__ void dense_combine_kernel(int64_t P, int64_t ldg, const float* __rest
 }
 
 // ---------------------------------------------------------------- Cholesky (lower, row-major, lda = P)
-// diagonal block [k0, k0 + nb): unblocked right-looking factorisation in shared memory.  A pivot that
-// is not positive (S + shift not positive definite in float64) sets *info = column + 1 and is
-// replaced by 1 so that the factorisation finishes without NaN; the host reports the failure.
+// The matrix has an extra row P that starts as F^H: the panel and trailing steps turn it into y^H of L y = F, so
+// the forward substitution costs nothing of its own.
+//
+// a - b * c for the trailing updates, in multiply-adds only
+__device__ __forceinline__ double zfms(double a, double b, double c) { return fma(-b, c, a); }
+__device__ __forceinline__ double2 zfms(double2 a, double2 b, double2 c) {
+  return make_double2(fma(b.y, c.y, fma(-b.x, c.x, a.x)), fma(-b.y, c.x, fma(-b.x, c.y, a.y)));
+}
+// a + b * conj(c)
+__device__ __forceinline__ double zfmac(double a, double b, double c) { return fma(b, c, a); }
+__device__ __forceinline__ double2 zfmac(double2 a, double2 b, double2 c) {
+  return make_double2(fma(b.y, c.y, fma(b.x, c.x, a.x)), fma(-b.x, c.y, fma(b.y, c.x, a.y)));
+}
+__device__ __forceinline__ double qshfl(double v, int src) { return __shfl_sync(0xffffffffu, v, src, 4); }
+__device__ __forceinline__ double2 qshfl(double2 v, int src) {
+  return make_double2(__shfl_sync(0xffffffffu, v.x, src, 4), __shfl_sync(0xffffffffu, v.y, src, 4));
+}
+
+// diagonal block [k0, k0 + nb): right-looking factorisation with the block in registers.  Thread (row, t) of
+// 64 x 4 holds the columns 4 s + t of its row; a step publishes one column in shared memory (one barrier) and
+// every thread subtracts a_ij conj(a_lj) / d_j; the scaling by 1 / sqrt(d_j) waits until the end.  Entries above
+// the diagonal are carried along unread (rows above the pivot publish zero), so the step has no branch.  A pivot
+// that is not positive (S + shift not positive definite in float64) sets *info = column + 1 and is replaced by 1
+// so that the factorisation finishes without NaN; the host reports the failure.  Latency-bound: 64 x (barrier,
+// division, multiply-add chain):
+// 31 us, 78 with the block in shared memory and three barriers a step.
+template <class V>
+__device__ void factor_diag(V* A, int64_t lda, int64_t k0, int nb, int* info, V (*colb)[CB], double* piv) {
+  const int row = threadIdx.x >> 2, t = threadIdx.x & 3;
+  V a[CB / 4];
+#pragma unroll
+  for (int q = 0; q < CB / 4; ++q) {
+    const int c = 4 * q + t;
+    a[q] = (row < nb && c <= row) ? A[(k0 + row) * lda + k0 + c] : zzero(V());
+  }
+#pragma unroll
+  for (int qb = 0; qb < CB / 4; ++qb) {
+#pragma unroll 1
+    for (int jt = 0; jt < 4; ++jt) {
+      const int j = 4 * qb + jt;
+      if (j >= nb) break;
+      V* cb = colb[j & 1];
+      if (t == jt) cb[row] = row >= j ? a[qb] : zzero(V());
+      __syncthreads();
+      double d = d_re(cb[j]);
+      if (!(d > 0.0)) {
+        if (threadIdx.x == 0) atomicCAS(info, 0, (int)(k0 + j + 1));
+        d = 1.0;
+      }
+      if (threadIdx.x == 0) piv[j] = d;
+      const V x = zscale(1.0 / d, cb[row]);
+      const V xq = t > jt ? x : zzero(V());                 // columns up to j are finished
+      a[qb] = zfms(a[qb], xq, zconj(cb[4 * qb + t]));
+#pragma unroll
+      for (int q = qb + 1; q < CB / 4; ++q) a[q] = zfms(a[q], x, zconj(cb[4 * q + t]));
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < CB / 4; ++q) {
+    const int c = 4 * q + t;
+    if (row < nb && c <= row) {
+      const double r = sqrt(piv[c]);
+      A[(k0 + row) * lda + k0 + c] = c == row ? zfrom(r, V()) : zscale(1.0 / r, a[q]);
+    }
+  }
+}
 template <class V>
 __global__ void __launch_bounds__(256) chol_diag_kernel(V* __restrict__ A, int64_t lda, int64_t k0, int nb,
                                                         int* __restrict__ info) {
-  extern __shared__ __align__(16) uint8_t csm[];
-  V* L = reinterpret_cast<V*>(csm);                         // [nb][nb + 1]
-  const int ld = nb + 1;
-  for (int e = threadIdx.x; e < nb * nb; e += blockDim.x) {
-    const int i = e / nb, j = e % nb;
-    L[i * ld + j] = (j <= i) ? A[(k0 + i) * lda + k0 + j] : zzero(V());
+  __shared__ V colb[2][CB];
+  __shared__ double piv[CB];
+  factor_diag(A, lda, k0, nb, info, colb, piv);
+}
+
+// L_kk in shared memory (rows of CB + 1, zero past nb) and 1 / its diagonal
+constexpr int LP = CB + 1;
+template <class V>
+__device__ __forceinline__ void stage_diag(const V* A, int64_t lda, int64_t k0, int nb, V* Ls, double* rinv) {
+#pragma unroll 8
+  for (int e = threadIdx.x; e < CB * CB; e += blockDim.x) {
+    const int c = e / CB, j = e % CB;
+    Ls[c * LP + j] = (c < nb && j <= c) ? A[(k0 + c) * lda + k0 + j] : zzero(V());
   }
-  __syncthreads();
-  for (int j = 0; j < nb; ++j) {
-    if (threadIdx.x == 0) {
-      double d = d_re(L[j * ld + j]);
-      if (!(d > 0.0)) {
-        atomicCAS(info, 0, (int)(k0 + j + 1));
-        d = 1.0;
-      }
-      L[j * ld + j] = zfrom(sqrt(d), V());
+  if (threadIdx.x < CB) rinv[threadIdx.x] = threadIdx.x < nb ? 1.0 / d_re(A[(k0 + threadIdx.x) * lda + k0 + threadIdx.x]) : 1.0;
+}
+// one row of x L_kk^{-H}: its four threads hold the columns 4 s + t in registers; a step hands the finished entry
+// to the other three by a shuffle.  All rows of the block read the same entries of L_kk.
+template <class V>
+__device__ __forceinline__ void solve_row(V (&a)[CB / 4], const V* Ls, const double* rinv, int t) {
+#pragma unroll
+  for (int qb = 0; qb < CB / 4; ++qb) {
+#pragma unroll 1
+    for (int jt = 0; jt < 4; ++jt) {
+      const int j = 4 * qb + jt;
+      const V xj = qshfl(zscale(rinv[j], a[qb]), jt);
+      const V* Lj = Ls + t * LP + j;
+      if (t == jt) a[qb] = xj;
+      a[qb] = zfms(a[qb], t > jt ? xj : zzero(V()), zconj(Lj[4 * qb * LP]));
+#pragma unroll
+      for (int q = qb + 1; q < CB / 4; ++q) a[q] = zfms(a[q], xj, zconj(Lj[4 * q * LP]));
     }
-    __syncthreads();
-    const double inv = 1.0 / d_re(L[j * ld + j]);
-    for (int i = j + 1 + threadIdx.x; i < nb; i += blockDim.x) L[i * ld + j] = zscale(inv, L[i * ld + j]);
-    __syncthreads();
-    // trailing update of the lower triangle: L[i][k] -= L[i][j] conj(L[k][j]), j < k <= i
-    const int m = nb - j - 1;
-    for (int e = threadIdx.x; e < m * m; e += blockDim.x) {
-      const int i = j + 1 + e / m, k = j + 1 + e % m;
-      if (k <= i) L[i * ld + k] = zmsc(L[i * ld + k], L[i * ld + j], L[k * ld + j]);
-    }
-    __syncthreads();
-  }
-  for (int e = threadIdx.x; e < nb * nb; e += blockDim.x) {
-    const int i = e / nb, j = e % nb;
-    if (j <= i) A[(k0 + i) * lda + k0 + j] = L[i * ld + j];
   }
 }
 
-// panel below the diagonal block: row x of A[k0 + nb .. P)[k0 .. k0 + nb) becomes x L_kk^{-H}
-// (forward substitution over the block's columns, one thread per row, L_kk in shared memory)
+// panel below the diagonal block: row x of A[k0 + nb .. n_rows)[k0 .. k0 + nb) becomes x L_kk^{-H}, 32 rows per
+// block (the panel is short of rows to fill the chip).  Latency-bound (64 dependent steps): 21 us on average over
+// the 84 panels of 5,364 complex columns, 23 with 64 rows per block, 312 with one thread per row that walked its
+// row in global memory.  As a product with the inverse of L_kk it takes 18, but the inverses then lengthen the
+// diagonal steps by 15 and the whole by 2 %.
+constexpr int PR = 32;
 template <class V>
-__global__ void __launch_bounds__(128) chol_panel_kernel(V* __restrict__ A, int64_t lda, int64_t k0, int nb, int64_t P) {
+__global__ void __launch_bounds__(4 * PR) chol_panel_kernel(V* __restrict__ A, int64_t lda, int64_t k0, int nb,
+                                                            int64_t n_rows) {
   extern __shared__ __align__(16) uint8_t csm[];
-  V* L = reinterpret_cast<V*>(csm);                         // [nb][nb]
-  for (int e = threadIdx.x; e < nb * nb; e += blockDim.x) {
-    const int i = e / nb, j = e % nb;
-    L[e] = (j <= i) ? A[(k0 + i) * lda + k0 + j] : zzero(V());
-  }
+  V* Ls = reinterpret_cast<V*>(csm);
+  __shared__ double rinv[CB];
+  const int t = threadIdx.x & 3;
+  const int64_t row = k0 + nb + (int64_t)blockIdx.x * PR + (threadIdx.x >> 2);
+  const bool valid = row < n_rows;                          // whole quads stay for the shuffles
+  V* x = A + (valid ? row : k0) * lda + k0;
+  V a[CB / 4];
+#pragma unroll
+  for (int q = 0; q < CB / 4; ++q) a[q] = (valid && 4 * q + t < nb) ? x[4 * q + t] : zzero(V());
+  stage_diag(A, lda, k0, nb, Ls, rinv);
   __syncthreads();
-  const int64_t row = k0 + nb + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (row >= P) return;
-  V* x = A + row * lda + k0;
-  for (int j = 0; j < nb; ++j) {
-    V a = x[j];
-    for (int l = 0; l < j; ++l) a = zmsc(a, x[l], L[j * nb + l]);
-    x[j] = zscale(1.0 / d_re(L[j * nb + j]), a);
+  solve_row(a, Ls, rinv, t);
+#pragma unroll
+  for (int q = 0; q < CB / 4; ++q)
+    if (valid && 4 * q + t < nb) x[4 * q + t] = a[q];
+}
+
+// L_kk^{-H} of every diagonal block (one block of threads each: the rows of the identity through solve_row), for
+// the backward substitution.  Upper triangular: its entries above the diagonal go to that place of A, which
+// the factorisation does not use; its diagonal is 1 / L_jj.
+template <class V>
+__global__ void __launch_bounds__(256) chol_inv_kernel(V* __restrict__ A, int64_t lda, int64_t P) {
+  extern __shared__ __align__(16) uint8_t csm[];
+  V* Ls = reinterpret_cast<V*>(csm);
+  __shared__ double rinv[CB];
+  const int64_t k0 = (int64_t)blockIdx.x * CB;
+  const int nb = (int)min((int64_t)CB, P - k0);
+  stage_diag(A, lda, k0, nb, Ls, rinv);
+  __syncthreads();
+  const int t = threadIdx.x & 3, row = threadIdx.x >> 2;
+  V a[CB / 4];
+#pragma unroll
+  for (int q = 0; q < CB / 4; ++q) a[q] = 4 * q + t == row ? zfrom(1.0, V()) : zzero(V());
+  solve_row(a, Ls, rinv, t);
+#pragma unroll
+  for (int q = 0; q < CB / 4; ++q) {
+    const int j = 4 * q + t;
+    if (j < nb && row < j) A[(k0 + row) * lda + k0 + j] = a[q];
   }
 }
 
-// trailing update of the lower triangle: A[I][J] -= L[I][K] L[J][K]^H for the 64 x 64 tiles I >= J
-// of rows / columns [k1, P), K = [k0, k0 + nb); 16 x 16 threads with 4 x 4 register tiles
+// trailing update of the lower triangle: A[I][J] -= L[I][K] L[J][K]^H for the 64 x 64 tiles I >= J of rows
+// [k1, n_rows) and columns [k1, P), K = [k0, k0 + nb); 16 x 16 threads with 4 x 4 register tiles.  The blocks of
+// the grid are the tiles of the triangle; the first one goes on to factor the next diagonal block while the
+// others run.  Bound by the float64 multiply-adds, four per complex product (as a product and a sum it took six):
+// 13.3 ms for 5,364 complex columns where the instructions alone take 11.8; 18.9 before, and the diagonal blocks'
+// 6.6 on their own.
 template <class V>
-__global__ void __launch_bounds__(256) chol_update_kernel(V* __restrict__ A, int64_t lda, int64_t k0, int nb,
-                                                          int64_t k1, int64_t P) {
+__global__ void __launch_bounds__(256, 2) chol_update_kernel(V* __restrict__ A, int64_t lda, int64_t k0, int nb,
+                                                          int64_t k1, int64_t P, int64_t n_rows,
+                                                          int* __restrict__ info) {
   constexpr int TK = 16;
   __shared__ V Li[CB][TK + 1];
   __shared__ V Lj[CB][TK + 1];
-  const int bi = blockIdx.y, bj = blockIdx.x;
-  if (bj > bi) return;
+  // tile index -> (bi, bj), bj <= bi
+  int bi = (int)((sqrt(8.0 * (double)blockIdx.x + 1.0) - 1.0) * 0.5);
+  while ((int64_t)(bi + 1) * (bi + 2) / 2 <= (int64_t)blockIdx.x) ++bi;
+  while ((int64_t)bi * (bi + 1) / 2 > (int64_t)blockIdx.x) --bi;
+  const int bj = (int)((int64_t)blockIdx.x - (int64_t)bi * (bi + 1) / 2);
   const int64_t i0 = k1 + (int64_t)bi * CB, j0 = k1 + (int64_t)bj * CB;
+  if (j0 >= P) return;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
   V acc[4][4];
 #pragma unroll
@@ -402,7 +533,7 @@ __global__ void __launch_bounds__(256) chol_update_kernel(V* __restrict__ A, int
       const int r = e / TK, k = e % TK;
       const int64_t gi = i0 + r, gj = j0 + r;
       const bool kin = kk + k < nb;
-      Li[r][k] = (gi < P && kin) ? A[gi * lda + k0 + kk + k] : zzero(V());
+      Li[r][k] = (gi < n_rows && kin) ? A[gi * lda + k0 + kk + k] : zzero(V());
       Lj[r][k] = (gj < P && kin) ? A[gj * lda + k0 + kk + k] : zzero(V());
     }
     __syncthreads();
@@ -412,11 +543,11 @@ __global__ void __launch_bounds__(256) chol_update_kernel(V* __restrict__ A, int
 #pragma unroll
       for (int r = 0; r < 4; ++r) a[r] = Li[ty + 16 * r][k];
 #pragma unroll
-      for (int c = 0; c < 4; ++c) b[c] = zconj(Lj[tx + 16 * c][k]);
+      for (int c = 0; c < 4; ++c) b[c] = Lj[tx + 16 * c][k];
 #pragma unroll
       for (int r = 0; r < 4; ++r)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) acc[r][c] = zadd(acc[r][c], zmul(a[r], b[c]));
+        for (int c = 0; c < 4; ++c) acc[r][c] = zfmac(acc[r][c], a[r], b[c]);
     }
   }
 #pragma unroll
@@ -425,8 +556,13 @@ __global__ void __launch_bounds__(256) chol_update_kernel(V* __restrict__ A, int
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
       const int64_t gj = j0 + tx + 16 * c;
-      if (gi < P && gj <= gi) A[gi * lda + gj] = zsub(A[gi * lda + gj], acc[r][c]);
+      if (gi < n_rows && gj <= gi && gj < P) A[gi * lda + gj] = zsub(A[gi * lda + gj], acc[r][c]);
     }
+  }
+  if (blockIdx.x == 0) {
+    __shared__ double piv[CB];
+    __syncthreads();                                        // the tile is written, Li is free
+    factor_diag(A, lda, k1, (int)min((int64_t)CB, P - k1), info, reinterpret_cast<V(*)[CB]>(&Li[0][0]), piv);
   }
 }
 
@@ -446,52 +582,53 @@ __device__ __forceinline__ double2 dwarp_sum(double2 v) {
 }
 }  // namespace
 
-// ---------------------------------------------------------------- triangular solves with L (row-major)
-// L y = b on the diagonal block [k0, k0 + nb) (one warp; lanes split the dot products)
+// ---------------------------------------------------------------- backward substitution L^H x = y
+// row P of the matrix: F^H at the start; y = (that row)^H, in place, at the end
 template <class V>
-__global__ void trsv_fwd_diag_kernel(const V* __restrict__ A, int64_t lda, int64_t k0, int nb, V* __restrict__ y) {
-  const int lane = threadIdx.x;
-  for (int j = 0; j < nb; ++j) {
-    V part = zzero(V());
-    for (int l = lane; l < j; l += 32) part = zadd(part, zmul(A[(k0 + j) * lda + k0 + l], y[k0 + l]));
-    part = dwarp_sum(part);
-    if (lane == 0) y[k0 + j] = zscale(1.0 / d_re(A[(k0 + j) * lda + k0 + j]), zsub(y[k0 + j], part));
-    __syncwarp();
+__global__ void conj_copy_kernel(int64_t n, const V* src, V* dst) {
+  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x)
+    dst[k] = zconj(src[k]);
+}
+// Block [k0, k0 + nb), going up: x = L_kk^{-H} y (chol_inv_kernel's rows), then y_i -= sum_l conj(L_li) x_l for the rows
+// above.  64 rows i per block, the 64 terms shared by four threads each with all their loads in flight; every
+// block of the grid computes x for itself, the first writes it.  Bound by the two trips to memory and the launch:
+// 12 us per 64 columns, 113 when one warp solved the diagonal block entry by entry and a second launch updated.
+template <class V>
+__global__ void __launch_bounds__(256) trsv_bwd_kernel(const V* __restrict__ A, int64_t lda, int64_t k0, int nb,
+                                                       V* __restrict__ y, V* __restrict__ x) {
+  __shared__ V part[4][CB];
+  __shared__ V xs[CB];
+  const int i = threadIdx.x & 63, g = threadIdx.x >> 6;
+  const int64_t gi = (int64_t)blockIdx.x * CB + i;
+  V l[CB / 4];
+#pragma unroll
+  for (int q = 0; q < CB / 4; ++q) {
+    const int r = g * (CB / 4) + q;
+    l[q] = (gi < k0 && r < nb) ? A[(k0 + r) * lda + gi] : zzero(V());
   }
-}
-// y_i -= sum_{l in block} L_il y_l for the rows below the block (one warp per row)
-template <class V>
-__global__ void trsv_fwd_update_kernel(const V* __restrict__ A, int64_t lda, int64_t k0, int nb, int64_t P,
-                                       V* __restrict__ y) {
-  const int lane = threadIdx.x & 31;
-  const int64_t i = k0 + nb + (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (i >= P) return;
-  V part = zzero(V());
-  for (int l = lane; l < nb; l += 32) part = zadd(part, zmul(A[i * lda + k0 + l], y[k0 + l]));
-  part = dwarp_sum(part);
-  if (lane == 0) y[i] = zsub(y[i], part);
-}
-// L^H x = y on the diagonal block, j descending: x_j = (y_j - sum_{l > j} conj(L_lj) x_l) / L_jj
-template <class V>
-__global__ void trsv_bwd_diag_kernel(const V* __restrict__ A, int64_t lda, int64_t k0, int nb, V* __restrict__ y) {
-  const int lane = threadIdx.x;
-  for (int j = nb - 1; j >= 0; --j) {
-    V part = zzero(V());
-    for (int l = j + 1 + lane; l < nb; l += 32) part = zadd(part, zmul(zconj(A[(k0 + l) * lda + k0 + j]), y[k0 + l]));
-    part = dwarp_sum(part);
-    if (lane == 0) y[k0 + j] = zscale(1.0 / d_re(A[(k0 + j) * lda + k0 + j]), zsub(y[k0 + j], part));
-    __syncwarp();
+  {
+    const int row = threadIdx.x >> 2, t = threadIdx.x & 3;
+    V sum = zzero(V());
+#pragma unroll
+    for (int q = 0; q < CB / 4; ++q) {
+      const int j = 4 * q + t;
+      if (j < nb && row < j) sum = zfms(sum, A[(k0 + row) * lda + k0 + j], zscale(-1.0, y[k0 + j]));
+    }
+    if (t == 0 && row < nb) sum = zadd(sum, zscale(1.0 / d_re(A[(k0 + row) * lda + k0 + row]), y[k0 + row]));
+    sum = zadd(sum, qshfl(sum, t ^ 1));
+    sum = zadd(sum, qshfl(sum, t ^ 2));
+    if (t == 0) {
+      xs[row] = sum;
+      if (blockIdx.x == 0 && row < nb) x[k0 + row] = sum;
+    }
   }
-}
-// y_i -= sum_{l in block} conj(L_li) x_l for the rows above the block (one thread per row: the reads
-// L[l][i] are consecutive across the threads)
-template <class V>
-__global__ void trsv_bwd_update_kernel(const V* __restrict__ A, int64_t lda, int64_t k0, int nb, V* __restrict__ y) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= k0) return;
-  V part = zzero(V());
-  for (int l = 0; l < nb; ++l) part = zadd(part, zmul(zconj(A[(k0 + l) * lda + i]), y[k0 + l]));
-  y[i] = zsub(y[i], part);
+  __syncthreads();
+  V acc = zzero(V());
+#pragma unroll
+  for (int q = 0; q < CB / 4; ++q) acc = zfms(acc, zconj(l[q]), xs[g * (CB / 4) + q]);
+  part[g][i] = acc;
+  __syncthreads();
+  if (g == 0 && gi < k0) y[gi] = zadd(y[gi], zadd(zadd(part[0][i], part[1][i]), zadd(part[2][i], part[3][i])));
 }
 
 // per-row |b - M x|^2 and |b|^2 of the dense system (one warp per row), then one block sums them
@@ -570,10 +707,10 @@ DenseWork dense_layout(int dtype, int ns, int nh, int64_t n, bool with_A, char* 
   W.emean = (double*)take(4 * sizeof(double));
   W.obar = take((size_t)W.P * vs);
   W.F = take((size_t)W.P * vs);
-  W.y = take((size_t)W.P * vs);
   W.xt = (uint16_t*)take((size_t)W.n_rb * W.nK * 2 * GR * GK * 2);
   W.G = (float*)take(std::max((size_t)Rp * Rp * sizeof(float), with_A ? (size_t)W.P * W.P * vs : 0));
-  W.A = with_A ? take((size_t)W.P * W.P * vs) : nullptr;
+  W.A = take(with_A ? (size_t)(W.P + 1) * W.P * vs : (size_t)W.P * vs);   // row P: F^H, then y^H, then y
+  W.y = base && with_A ? (uint8_t*)W.A + (size_t)W.P * W.P * vs : W.A;
   W.rr = (double*)take((size_t)W.P * sizeof(double));
   W.bb = (double*)take((size_t)W.P * sizeof(double));
   W.scal = (double*)take(8 * sizeof(double));
@@ -589,8 +726,8 @@ int dense_gram_t(int ns, int nh, int64_t n, const uint32_t* bits, const typename
                  const float2* eloc, const float* probs, double shift, V* A, const DenseWork& W, cudaStream_t st) {
   QES_CUDA_CHECK(cudaMemsetAsync(W.flags, 0, 8 * sizeof(int), st));
   dense_g_kernel<<<1, 1024, 0, st>>>(n, eloc, probs, W.gw, eloc ? W.ge : nullptr, W.emean);
-  const int pb = (int)((W.P + 255) / 256);
-  dense_ohg_kernel<V><<<pb, 256, 0, st>>>(ns, nh, n, bits, tt, W.gw, (V*)W.obar);
+  const dim3 og((unsigned)((nh + 1 + 31) / 32), (unsigned)((ns + 1 + OHG_R - 1) / OHG_R));
+  dense_ohg_kernel<V><<<og, 32 * OHG_R, 0, st>>>(ns, nh, n, bits, tt, W.gw, (V*)W.obar);
   const int64_t items = (int64_t)W.n_rb * W.nK * GR * (GK / 8);
   dense_x_tiles_kernel<V><<<(unsigned)std::min<int64_t>((items + 255) / 256, 4 * 1184), 256, 0, st>>>(
       ns, nh, n, (int)W.rows, W.n_rb, W.nK, bits, tt, probs, (const V*)W.obar, W.xt);
@@ -634,48 +771,49 @@ int dense_solve_t(int ns, int nh, int64_t n, const uint32_t* bits, const typenam
   if (rc) return rc;
   // keep S + shift for the residual check (the Gram tiles are no longer needed)
   QES_CUDA_CHECK(cudaMemcpyAsync(W.G, A, (size_t)P * P * sizeof(V), cudaMemcpyDeviceToDevice, st));
-  const int pb = (int)((P + 255) / 256);
-  dense_ohg_kernel<V><<<pb, 256, 0, st>>>(ns, nh, n, bits, tt, W.ge, (V*)W.F);
-  QES_LAUNCH_CHECK();
-  // blocked Cholesky
-  const size_t sm_diag = (size_t)CB * (CB + 1) * sizeof(V), sm_panel = (size_t)CB * CB * sizeof(V);
-  QES_CUDA_CHECK(cudaFuncSetAttribute(chol_diag_kernel<V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_diag));
+  const dim3 og((unsigned)((nh + 1 + 31) / 32), (unsigned)((ns + 1 + OHG_R - 1) / OHG_R));
+  dense_ohg_kernel<V><<<og, 32 * OHG_R, 0, st>>>(ns, nh, n, bits, tt, W.ge, (V*)W.F);
+  const unsigned vg = (unsigned)std::min<int64_t>((P + 255) / 256, 1184);
+  conj_copy_kernel<V><<<vg, 256, 0, st>>>(P, (const V*)W.F, y);
+  QES_LAUNCH_CHECK_N(2);
+  // blocked Cholesky with the row F^H below the matrix
+  const size_t sm_block = (size_t)CB * LP * sizeof(V);
   QES_CUDA_CHECK(cudaFuncSetAttribute(chol_panel_kernel<V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)sm_panel));
+                                      (int)sm_block));
+  QES_CUDA_CHECK(cudaFuncSetAttribute(chol_inv_kernel<V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_block));
+  const int64_t n_rows = P + 1;
   const int pfc = qes_prof_begin(QES_PROF_CHOL, st);
+  chol_diag_kernel<V><<<1, 256, 0, st>>>(A, P, 0, (int)std::min<int64_t>(CB, P), W.flags);
+  QES_LAUNCH_CHECK();
   for (int64_t k0 = 0; k0 < P; k0 += CB) {
     const int nb = (int)std::min<int64_t>(CB, P - k0);
-    chol_diag_kernel<V><<<1, 256, sm_diag, st>>>(A, P, k0, nb, W.flags);
-    const int64_t k1 = k0 + nb, rest = P - k1;
-    if (rest > 0) {
-      chol_panel_kernel<V><<<(unsigned)((rest + 127) / 128), 128, sm_panel, st>>>(A, P, k0, nb, P);
-      const unsigned nt = (unsigned)((rest + CB - 1) / CB);
-      chol_update_kernel<V><<<dim3(nt, nt), 256, 0, st>>>(A, P, k0, nb, k1, P);
-      QES_LAUNCH_CHECK_N(3);
-    } else {
+    const int64_t k1 = k0 + nb, rest = n_rows - k1;         // at least the row F^H
+    chol_panel_kernel<V><<<(unsigned)((rest + PR - 1) / PR), 4 * PR, sm_block, st>>>(A, P, k0, nb, n_rows);
+    QES_LAUNCH_CHECK();
+    if (k1 < P) {                                           // and the factorisation of the next diagonal block
+      const int64_t nt = (rest + CB - 1) / CB;
+      QES_ARG_CHECK(nt * (nt + 1) / 2 < (1ll << 31), "dense SR: too many Cholesky tiles");
+      chol_update_kernel<V><<<(unsigned)(nt * (nt + 1) / 2), 256, 0, st>>>(A, P, k0, nb, k1, P, n_rows, W.flags);
       QES_LAUNCH_CHECK();
     }
   }
+  chol_inv_kernel<V><<<(unsigned)((P + CB - 1) / CB), 256, sm_block, st>>>(A, P, P);
+  QES_LAUNCH_CHECK();
   qes_prof_end(pfc, st);
-  // L y = F, L^H x = y
-  QES_CUDA_CHECK(cudaMemcpyAsync(y, W.F, (size_t)P * sizeof(V), cudaMemcpyDeviceToDevice, st));
-  for (int64_t k0 = 0; k0 < P; k0 += CB) {
-    const int nb = (int)std::min<int64_t>(CB, P - k0);
-    trsv_fwd_diag_kernel<V><<<1, 32, 0, st>>>(A, P, k0, nb, y);
-    const int64_t rest = P - k0 - nb;
-    if (rest > 0) trsv_fwd_update_kernel<V><<<(unsigned)((rest + 7) / 8), 256, 0, st>>>(A, P, k0, nb, P, y);
-  }
+  // L^H x = y: x in the O-bar buffer, which the Gram tiles no longer need
+  V* x = (V*)W.obar;
+  conj_copy_kernel<V><<<vg, 256, 0, st>>>(P, y, y);
+  QES_LAUNCH_CHECK();
   for (int64_t k0 = ((P - 1) / CB) * CB; k0 >= 0; k0 -= CB) {
     const int nb = (int)std::min<int64_t>(CB, P - k0);
-    trsv_bwd_diag_kernel<V><<<1, 32, 0, st>>>(A, P, k0, nb, y);
-    if (k0 > 0) trsv_bwd_update_kernel<V><<<(unsigned)((k0 + 255) / 256), 256, 0, st>>>(A, P, k0, nb, y);
+    trsv_bwd_kernel<V><<<(unsigned)std::max<int64_t>(1, k0 / CB), 256, 0, st>>>(A, P, k0, nb, y, x);
+    QES_LAUNCH_CHECK();
   }
-  QES_LAUNCH_CHECK();
   // residual in S + shift (kept in W.G), then x_out = rhs_prefactor * x
-  dense_resid_kernel<V><<<(unsigned)((P + 7) / 8), 256, 0, st>>>((const V*)W.G, P, y, (const V*)W.F, W.rr, W.bb);
+  dense_resid_kernel<V><<<(unsigned)((P + 7) / 8), 256, 0, st>>>((const V*)W.G, P, x, (const V*)W.F, W.rr, W.bb);
   dense_sum2_kernel<<<1, 1024, 0, st>>>(P, W.rr, W.bb, W.scal);
   dense_scale_copy_kernel<V><<<(unsigned)std::min<int64_t>((P + 255) / 256, 1184), 256, 0, st>>>(
-      P, opt->rhs_prefactor, y, x_out);
+      P, opt->rhs_prefactor, x, x_out);
   QES_LAUNCH_CHECK_N(3);
   double sc[2] = {0, 0}, em[2] = {0, 0};
   QES_CUDA_CHECK(cudaMemcpyAsync(sc, W.scal, 2 * sizeof(double), cudaMemcpyDeviceToHost, st));

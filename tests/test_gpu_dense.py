@@ -88,6 +88,31 @@ def test_dense_solve_matches_oracle(name, n, shift):
     assert rc < 1e-4
 
 
+# number of parameters (ns + 1)(nh + 1) - 1 just below, at and above whole 64-column blocks; sample counts around
+# the 32 that a staging step of the force takes
+@pytest.mark.parametrize("dtype", ["float32", "complex64"])
+@pytest.mark.parametrize("ns,nh,n", [(2, 1, 5), (7, 7, 33), (12, 4, 64), (10, 5, 31), (42, 2, 257), (12, 9, 96),
+                                     (33, 17, 200)])
+def test_block_edges_of_the_factorisation(ns, nh, n, dtype):
+    rng = np.random.default_rng(ns * 100 + nh)
+    net = RBM((ns,), n_hidden=nh, dtype=dtype, seed=ns, init_scale=0.2)
+    st = np.where(rng.random((n, ns)) < 0.5, 0.5, -0.5)
+    bits = dv.pack_states(st)
+    _, tn, _ = dv.rbm_forward(net.flat, ns, nh, bits, tanh=True, logpsi=True)
+    e = rng.standard_normal(n) + (1j * rng.standard_normal(n) if net.is_complex else 0.0)
+    eloc = torch.tensor(e.astype(np.complex64), device=net.flat.device)
+    shift = 1e-2
+    x, info, _ = dv.sr_solve_dense(net.flat, ns, nh, bits, tn, eloc, shift=shift, rhs_prefactor=1.0)
+    assert info["converged"]
+    S = dv.sr_gram(net.flat, ns, nh, bits, tn).cpu().numpy()
+    _, F = _oracle(st, tn, eloc, net.is_complex)
+    A = S + shift * np.eye(S.shape[0])
+    ev = np.linalg.eigvalsh(A)
+    # a backward-stable factorisation leaves |A x - F| <= c P u |A| |x|, |A| |x| <= kappa |F|; F itself is a sum of n
+    tol = 16 * (S.shape[0] * ev[-1] / ev[0] + n) * 2.0 ** -53
+    assert np.linalg.norm(A @ x.cpu().numpy() - F) <= tol * np.linalg.norm(F)
+
+
 def test_tdvp_form_matrix_uses_the_dense_path_and_nqs_trains():
     model = qb.TransverseFieldIsing(qb.SquareLattice(1, 8), j=1.0, hx=1.0, hz=0.0)
     nqs = qb.NQS("rbm", model, alpha=1.0, dtype="float32", seed=1, s_numchains=256, s_numsamples=8,
