@@ -36,7 +36,7 @@ from ._lib import call, ptr, stream_ptr
 from .hamiltonian import SpinHamiltonian
 
 OHU_SPLIT = 256                             # samples per split of the O^H u partials (sr.cu)
-OV_ROWS, FWD_SB, ELOC_SB, RED_SB = 64, 16, 32, 256
+OV_ROWS, FWD_SB, ELOC_SB, RED_SB = 256, 16, 32, 256
 
 
 def _ceil(a, b):

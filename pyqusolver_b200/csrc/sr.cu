@@ -16,6 +16,7 @@
 #include "sr_tc.h"
 #include "sr_pcg.h"
 
+#include <cooperative_groups.h>
 #include <algorithm>
 #include <atomic>
 #include <vector>
@@ -2909,309 +2910,440 @@ __global__ void __launch_bounds__(BCG_THREADS) batch_mean_kernel(const qes_batch
 }
 
 // ---- matvec halves of the batched solve (small problems) -------------------------------------
-// ov  item (b, first row, rows <= BOV_ROWS, 0): the block stages V = v_W (float32), v_b, v_a and
-//     the spins of its rows (as +-1 floats, site-major) in shared memory and computes
-//       z_m = v_b,m + sum_i sigma_i V_im ,  (O v)_s = sum_m t_sm z_m + sigma . v_a
-//     in 4 x 4 register tiles (batch_ov_tile_kernel below).
-// ohu item (b, split z, 0, 0): the block owns every (site, hidden unit) entry of the split's
-//     partial, in 4 x 4 register tiles (batch_ohu_tile_kernel below).
-constexpr int BOV_ROWS = 64;
-// block size limit of the tile kernels (complex tiles hold twice the registers: half the block)
+// ov  item (b, first row, rows, 0):  z_m = p_b,m + sum_i sigma_i p_W,im ,  (O p)_s = sum_m t_sm z_m + sigma . p_a
+// ohu item (b, split z, 0, 0):  g_W,im = sum_s sigma_si q_sm ,  g_b,m = sum_s q_sm ,  g_a,i = sum_s sigma_si u_s  with
+//     q_s = conj(t_s) u_s over the split's 256 samples.
+// Both products have spins, +-1, for one operand, so that they run on the tensor cores in float32 precision: the other
+// operand (p_W, q) is the exact sum of three BF16 numbers, three MMAs with FP32 accumulation.  The operands are made
+// where they are used: the spins' fragments from the packed words (a shift, a byte permute and a mask per pair),
+// q's fragments in the registers of the one warp that needs them.  That is why these are warp-level MMAs (m16n8k16):
+// tcgen05 would want the spins and three copies of q written to shared memory first, and the MMAs themselves are
+// a few percent of the time.  As float32 multiply-adds both kernels were bound by the 128 bytes a clock that
+// shared memory delivers to the registers: 91 and 76 us with 4 x 4 register tiles, 62 and 56 with 4 x 8, 38 and 32
+// now (O^H u, O p; 64 chains of 12-64 sites, two hidden units per site, 2,048 samples each), of which the prologues'
+// latency is the larger part.  Error against a float64 solve over 12-130 sites: that of the float32 multiply-adds.
 template <class T>
-constexpr int bohu_max_threads() { return ScalarTraits<T>::is_complex ? 512 : 1024; }
+constexpr int bparts() { return ScalarTraits<T>::is_complex ? 2 : 1; }   // real numbers per T
+constexpr int BMM_THREADS = 256, BMM_WARPS = BMM_THREADS / 32;
+constexpr int64_t BMEAN_ROWS = 16384;            // up to here every ohu block sums its problem's w itself
 
 QES_HD int64_t bsmall_align16(int64_t bytes) { return (bytes + 15) & ~(int64_t)15; }
-
-// ov tiles: thread t owns 4 rows x 4 hidden units (tm = t % n_mt fastest) of
-// z_sm = v_b,m + sum_i sigma_si V_im; per site it reads one float4 of signs (4 rows, site-major
-// staging) and four V values for 16 multiply-adds, then folds its units into sum_m t_sm z_sm.
-// The per-unit-group partial sums meet in shared memory and are added in a fixed order.
-QES_HD int bov_round4(int x) { return (x + 3) & ~3; }
-template <class T>
-QES_HD size_t batch_ov_smem(int ns, int nh) {
-  const int nmt = bov_round4(nh) / 4;
-  return (size_t)bsmall_align16((int64_t)((int64_t)ns * bov_round4(nh) + bov_round4(nh) + ns) * sizeof(T)) +
-         (size_t)bsmall_align16((int64_t)ns * BOV_ROWS * sizeof(float)) + (size_t)BOV_ROWS * nmt * sizeof(T);
+QES_HD int bround(int x, int q) { return (x + q - 1) / q * q; }
+QES_D float shfl_xor_t(float v, int o) { return __shfl_xor_sync(0xffffffffu, v, o); }
+QES_D float2 shfl_xor_t(float2 v, int o) {
+  return make_float2(__shfl_xor_sync(0xffffffffu, v.x, o), __shfl_xor_sync(0xffffffffu, v.y, o));
+}
+QES_D float shfl_t(float v, int l) { return __shfl_sync(0xffffffffu, v, l); }
+QES_D float2 shfl_t(float2 v, int l) {
+  return make_float2(__shfl_sync(0xffffffffu, v.x, l), __shfl_sync(0xffffffffu, v.y, l));
+}
+QES_D float part_of(float v, int) { return v; }
+QES_D float part_of(float2 v, int c) { return c ? v.y : v.x; }
+// D += A B, 16 x 8 x 16, BF16 in, FP32 out.  Lane (g, t) = (lane / 4, lane % 4) holds of A rows g, g + 8 and columns
+// 2t, 2t + 1, 2t + 8, 2t + 9, of B the same four rows of column g, of D rows g, g + 8 and columns 2t, 2t + 1
+QES_D void mma16816(float (&d)[4], const uint32_t (&a)[4], uint2 b) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b.x), "r"(b.y));
+}
+// two floats as three pairs of BF16 (hi + mid + lo is exact: 3 x 8 bits)
+QES_D void split3(float x, float y, uint32_t (&o)[3]) {
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(o[k]) : "f"(y), "f"(x));
+    x -= __uint_as_float(o[k] << 16);
+    y -= __uint_as_float(o[k] & 0xffff0000u);
+  }
+}
+// bits 8 i + 7 and 8 j + 7 of y as a pair of +-1 in BF16 (set = +1)
+template <int I, int J>
+QES_D uint32_t sign_pair(uint32_t yi, uint32_t yj) {
+  return (__byte_perm(yi, yj, (I << 4) | ((4 + J) << 12)) & 0x80008000u) ^ 0xbf80bf80u;
 }
 
-template <class T, class V>
-__global__ void __launch_bounds__(bohu_max_threads<T>()) batch_ov_tile_kernel(const qes_batch_instance* __restrict__ inst,
-                                                                             const int4* __restrict__ items,
-                                                                             const uint32_t* __restrict__ bits,
-                                                                             const T* __restrict__ tt,
-                                                                             const V* __restrict__ v,
-                                                                             float2* __restrict__ w,
-                                                                             const double* __restrict__ bscal) {
+// O p: a warp takes 32 rows, eight warps a block.  p_W lies in shared memory as B fragments, split once per block:
+// [step of 16 sites][tile of 8 units (complex: Re and Im)][hi, mid, lo][lane].  Step ks holds of the sites' word
+// ks / 2 the bits 8 e + 2 t + ks % 2 (t = lane % 4, e = 0..3), which the spins' fragments read off byte by byte.
+// Four B tiles at a time; T is loaded ahead of their MMAs, and the product sum_m t_sm z_m is a sum over the lanes of a quad.
+template <class T>
+QES_HD size_t batch_ov_smem(int ns, int nh) {
+  return (size_t)bround(ns, 32) * bround(nh, 8) * bparts<T>() * 6 + (size_t)(ns + bround(nh, 8)) * sizeof(T);
+}
+
+template <class T>
+__global__ void __launch_bounds__(BMM_THREADS, 2) batch_ov_mma_kernel(const qes_batch_instance* __restrict__ inst,
+                                                                      const int4* __restrict__ items,
+                                                                      const uint32_t* __restrict__ bits,
+                                                                      const T* __restrict__ tt,
+                                                                      const T* __restrict__ pf,
+                                                                      float2* __restrict__ w,
+                                                                      const double* __restrict__ bscal) {
   extern __shared__ __align__(16) uint8_t bov_sm[];
+  constexpr bool CPLX = ScalarTraits<T>::is_complex;
+  constexpr int NP = bparts<T>(), NT = 4 / NP;                // NT unit tiles = 4 B tiles at a time
   const int4 it = items[blockIdx.x];
   if (bscal[(int64_t)it.x * BSC + 4] != 0.0) return;
   const qes_batch_instance I = inst[it.x];
   const int ns = I.ns, nh = I.nh, nw = n_words(ns);
-  const int nhp = bov_round4(nh), nmt = nhp / 4, n_tiles = (BOV_ROWS / 4) * nmt;
-  const int64_t r0 = it.y;
-  const int nr = it.z;
-  T* Vs = reinterpret_cast<T*>(bov_sm);                      // [ns][nhp]
-  T* vbs = Vs + (int64_t)ns * nhp;                            // [nhp]
-  T* vas = vbs + nhp;                                         // [ns]
-  float* sigT = reinterpret_cast<float*>(bov_sm + bsmall_align16((int64_t)((int64_t)ns * nhp + nhp + ns) * sizeof(T)));
-  T* red = reinterpret_cast<T*>(reinterpret_cast<uint8_t*>(sigT) + bsmall_align16((int64_t)ns * BOV_ROWS * sizeof(float)));
-  const int tid = threadIdx.x, nthr = blockDim.x;
-  const V* pv = v + I.param_off;
-  {
-    const int cm = tid % nhp, ci0 = tid / nhp, cid = nthr / nhp;   // V entry (i, m), divided once
-    if (ci0 < cid)
-      for (int i = ci0; i < ns; i += cid) Vs[i * nhp + cm] = (cm < nh) ? to_f(pv[ns + nh + (int64_t)i * nh + cm]) : ScalarTraits<T>::zero();
-  }
-  for (int m = tid; m < nhp; m += nthr) vbs[m] = (m < nh) ? to_f(pv[ns + m]) : ScalarTraits<T>::zero();
-  for (int i = tid; i < ns; i += nthr) vas[i] = to_f(pv[i]);
-  const uint32_t* bw = bits + I.sample_word_off;
-  {
-    const int q = tid % BOV_ROWS, i0 = tid / BOV_ROWS, di = nthr / BOV_ROWS;
-    for (int i = i0; i < ns; i += di) {
-      float sg = 0.f;
-      if (q < nr) sg = ((bw[(r0 + q) * nw + (i >> 5)] >> (i & 31)) & 1u) ? 1.f : -1.f;
-      sigT[i * BOV_ROWS + q] = sg;
+  const int nks = bround(ns, 32) / 16, nt = bround(nh, 8) / 8;
+  uint2* Bf = reinterpret_cast<uint2*>(bov_sm);               // [nks][nt][NP][3][32]
+  T* vbs = reinterpret_cast<T*>(Bf + (int64_t)nks * nt * NP * 96);   // [8 nt]
+  T* vas = vbs + 8 * nt;                                      // [ns]
+  const int tid = threadIdx.x, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const T* pv = pf + I.param_off;
+  const T* pw = pv + ns + nh;
+  // quads of sites x units: consecutive threads take consecutive units
+  for (int e = tid; e < nks * 4 * 8 * nt; e += BMM_THREADS) {
+    const int kq = e / (8 * nt), m = e - kq * 8 * nt, ks = kq >> 2, tq = kq & 3;
+    T v[4];
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      const int i = 32 * (ks >> 1) + 8 * x + 2 * tq + (ks & 1);
+      v[x] = (i < ns && m < nh) ? pw[(int64_t)i * nh + m] : ScalarTraits<T>::zero();
+    }
+#pragma unroll
+    for (int c = 0; c < NP; ++c) {
+      uint32_t lo[3], hi[3];
+      split3(part_of(v[0], c), part_of(v[1], c), lo);
+      split3(part_of(v[2], c), part_of(v[3], c), hi);
+      uint2* o = Bf + (((int64_t)ks * nt + (m >> 3)) * NP + c) * 96 + (m & 7) * 4 + tq;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) o[32 * k] = make_uint2(lo[k], hi[k]);
     }
   }
+  for (int m = tid; m < 8 * nt; m += BMM_THREADS) vbs[m] = (m < nh) ? pv[ns + m] : ScalarTraits<T>::zero();
+  for (int i = tid; i < ns; i += BMM_THREADS) vas[i] = pv[i];
   __syncthreads();
+  const uint32_t* bw = bits + I.sample_word_off;
   const T* tb = tt + I.tanh_off;
-  for (int t0 = 0; t0 < n_tiles; t0 += nthr) {
-    const int t = t0 + tid;
-    if (t < n_tiles) {
-      const int tm = t % nmt, sg = t / nmt;
-      T z[4][4];
+  const bool pairs = !CPLX && nh % 2 == 0 && reinterpret_cast<uintptr_t>(tb) % 8 == 0;   // two units in one load
+  for (int c0 = 32 * (tid >> 5); c0 < it.z; c0 += 32 * BMM_WARPS) {
+    const int64_t r0 = (int64_t)it.y + c0;
+    const int nr = min(32, it.z - c0);
+    // lane = row: sigma . p_a
+    T sva = ScalarTraits<T>::zero();
+    for (int wd = 0; wd < nw; ++wd) {
+      const uint32_t b = lane < nr ? bw[(r0 + lane) * nw + wd] : 0u;
+      const int i1 = min(32, ns - 32 * wd);
+#pragma unroll 8
+      for (int i = 0; i < i1; ++i) sva = fma_s(((b >> i) & 1u) ? 1.f : -1.f, vas[32 * wd + i], sva);
+    }
+    T acc[4];                                                 // rows g, g + 8, g + 16, g + 24
 #pragma unroll
-      for (int b = 0; b < 4; ++b) {
-        const T vb = vbs[4 * tm + b];
+    for (int a = 0; a < 4; ++a) acc[a] = ScalarTraits<T>::zero();
+    for (int n0 = 0; n0 < nt; n0 += NT) {
+      T tv[NT][4][2];
 #pragma unroll
-        for (int a = 0; a < 4; ++a) z[a][b] = vb;
-      }
-      for (int i = 0; i < ns; ++i) {
-        const float4 s4 = *reinterpret_cast<const float4*>(sigT + i * BOV_ROWS + 4 * sg);
-        const T* vr = Vs + (int64_t)i * nhp + 4 * tm;
-        T vv[4];
-        if constexpr (ScalarTraits<T>::is_complex) {
-          const float4 a01 = reinterpret_cast<const float4*>(vr)[0], a23 = reinterpret_cast<const float4*>(vr)[1];
-          vv[0] = make_float2(a01.x, a01.y); vv[1] = make_float2(a01.z, a01.w);
-          vv[2] = make_float2(a23.x, a23.y); vv[3] = make_float2(a23.z, a23.w);
-        } else {
-          const float4 a4 = *reinterpret_cast<const float4*>(vr);
-          vv[0] = a4.x; vv[1] = a4.y; vv[2] = a4.z; vv[3] = a4.w;
+      for (int j = 0; j < NT; ++j) {
+        const int m = 8 * (n0 + j) + 2 * t;
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+          const T* src = tb + (r0 + g + 8 * a) * nh + m;
+          const bool ok = g + 8 * a < nr;
+          if constexpr (!CPLX) {
+            if (pairs) {
+              const float2 f = (ok && m < nh) ? *reinterpret_cast<const float2*>(src) : make_float2(0.f, 0.f);
+              tv[j][a][0] = f.x;
+              tv[j][a][1] = f.y;
+              continue;
+            }
+          }
+          tv[j][a][0] = (ok && m < nh) ? src[0] : ScalarTraits<T>::zero();
+          tv[j][a][1] = (ok && m + 1 < nh) ? src[1] : ScalarTraits<T>::zero();
         }
-        const float sv[4] = {s4.x, s4.y, s4.z, s4.w};
+      }
+      float d[2][4][4];                                       // [16 rows][B tile][..], starting at p_b
+#pragma unroll
+      for (int j = 0; j < NT; ++j)
+#pragma unroll
+        for (int c = 0; c < NP; ++c) {
+          const int m = min(8 * (n0 + j), 8 * nt - 8) + 2 * t;
+          const float b0 = part_of(vbs[m], c), b1 = part_of(vbs[m + 1], c);
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            d[h][j * NP + c][0] = d[h][j * NP + c][2] = b0;
+            d[h][j * NP + c][1] = d[h][j * NP + c][3] = b1;
+          }
+        }
+      const int nb = min(NT, nt - n0) * NP;
+      for (int wd = 0; wd < nks / 2; ++wd) {
+        uint32_t sw[4];
+#pragma unroll
+        for (int a = 0; a < 4; ++a) sw[a] = g + 8 * a < nr ? bw[(r0 + g + 8 * a) * nw + wd] : 0u;
+#pragma unroll
+        for (int kk = 0; kk < 2; ++kk) {
+          uint32_t A[2][4];
+#pragma unroll
+          for (int a = 0; a < 4; ++a) {
+            const uint32_t y = sw[a] << (7 - 2 * t - kk);
+            A[a >> 1][a & 1] = sign_pair<0, 1>(y, y);
+            A[a >> 1][2 + (a & 1)] = sign_pair<2, 3>(y, y);
+          }
+          const uint2* bp = Bf + ((int64_t)(2 * wd + kk) * nt + n0) * NP * 96 + lane;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            if (j < nb) {
+#pragma unroll
+              for (int k = 2; k >= 0; --k) {                  // small parts first
+                const uint2 b = bp[j * 96 + 32 * k];
+                mma16816(d[0][j], A[0], b);
+                mma16816(d[1][j], A[1], b);
+              }
+            }
+          }
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < NT; ++j)
 #pragma unroll
         for (int a = 0; a < 4; ++a)
 #pragma unroll
-          for (int b = 0; b < 4; ++b) z[a][b] = addx(z[a][b], scal(sv[a], vv[b]));
-      }
-#pragma unroll
-      for (int a = 0; a < 4; ++a) {
-        const int q = 4 * sg + a;
-        T acc = ScalarTraits<T>::zero();
-        if (q < nr) {
-          const T* trow = tb + (r0 + q) * nh;
-#pragma unroll
-          for (int b = 0; b < 4; ++b) {
-            const int m = 4 * tm + b;
-            if (m < nh) acc = addx(acc, mulx(trow[m], z[a][b]));
+          for (int x = 0; x < 2; ++x) {
+            T z;
+            if constexpr (CPLX) z = make_float2(d[a >> 1][2 * j][2 * (a & 1) + x], d[a >> 1][2 * j + 1][2 * (a & 1) + x]);
+            else z = d[a >> 1][j][2 * (a & 1) + x];
+            acc[a] = addx(acc[a], mulx(tv[j][a][x], z));
           }
-        }
-        red[q * nmt + tm] = acc;
-      }
+    }
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+      acc[a] = addx(acc[a], shfl_xor_t(acc[a], 1));
+      acc[a] = addx(acc[a], shfl_xor_t(acc[a], 2));
+      const T sv = shfl_t(sva, g + 8 * a);
+      if (t == 0 && g + 8 * a < nr) w[I.sample_off + r0 + g + 8 * a] = to_c(addx(acc[a], sv));
     }
   }
-  __syncthreads();
-  float2* wo = w + I.sample_off;
-  for (int q = tid; q < nr; q += nthr) {
-    T acc = ScalarTraits<T>::zero();
-    for (int g = 0; g < nmt; ++g) acc = addx(acc, red[q * nmt + g]);
-    for (int i = 0; i < ns; ++i) acc = addx(acc, scal(sigT[i * BOV_ROWS + q], vas[i]));
-    wo[r0 + q] = to_c(acc);
-  }
 }
 
-// ohu tiles: the split's partial is the (ns + 1) x (nh + 1) matrix  sum_s sigma'_si q'_sm  with a
-// virtual site ns (sigma' = 1: row ns is g_b = sum_s q_s) and a virtual hidden unit nh
-// (q' = u: column nh is g_a = sum_s sigma_s u_s); entry (ns, nh) is unused.  Thread t owns a
-// 4 x 4 tile (sites 4 ti.., units 4 tm..), tm = t % n_mt fastest; per staged sample it reads one
-// float4 of signs and four q values from shared memory for 16 multiply-adds.  Tiles beyond the
-// block size take further passes over the samples.  (8 x 4 tiles, fewer threads per block, ran
-// slower: the staging latency, not the multiply-adds, sets the pace.)
-
-constexpr size_t BOHU_SMEM_TARGET = 200 * 1024;   // up to a whole split (256 samples) staged at once
-
-QES_HD int bohu_round4(int x) { return (x + 3) & ~3; }
-QES_HD int batch_ohu_tiles(int ns, int nh) { return (bohu_round4(ns + 1) / 4) * (bohu_round4(nh + 1) / 4); }
-// staged samples per pass for rows of (nh + 1) q values and (ns + 1) signs
+// O^H u: a warp takes 16 (complex: 8) hidden units and up to 64 sites at a time (further sites take passes), all samples
+// of the split or, where the problem has few units, a part of them (parts added in a fixed order).  Each q_sm is
+// made by the one lane whose fragment holds it, straight from T in global memory, one step of 16 samples ahead.  The
+// tensor core's own sums stay four steps long; they are added to the float32 accumulators with rounding.
+QES_HD int batch_ohu_ng(int nh, int np) { return (nh + 16 / np - 1) / (16 / np); }    // unit groups
+QES_HD int batch_ohu_parts(int ng) { return ng >= BMM_WARPS ? 1 : BMM_WARPS / ng; }
 template <class T>
-QES_HD int batch_ohu_sc(int ns_max_row, int nh_max_row) {
-  const size_t row = (size_t)bohu_round4(nh_max_row + 1) * sizeof(T) + (size_t)bohu_round4(ns_max_row + 1) * 4;
-  int sc = (int)(BOHU_SMEM_TARGET / row);
-  sc = sc > OHU_SPLIT_SAMPLES ? OHU_SPLIT_SAMPLES : sc;
-  return sc < 4 ? 4 : sc;
+QES_HD size_t batch_ohu_smem(int ns, int nh) {
+  const int ng = batch_ohu_ng(nh, bparts<T>()), parts = batch_ohu_parts(ng);
+  return (size_t)bsmall_align16((int64_t)OHU_SPLIT_SAMPLES * (sizeof(T) + 4 * ((ns + 31) / 32))) +
+         (size_t)bsmall_align16((int64_t)BMM_WARPS * ns * sizeof(T)) + (size_t)(parts - 1) * ng * 34 * 32 * sizeof(float);
 }
 
 template <class T>
-__global__ void __launch_bounds__(bohu_max_threads<T>()) batch_ohu_tile_kernel(const qes_batch_instance* __restrict__ inst,
-                                                                         const int4* __restrict__ items,
-                                                                         const uint32_t* __restrict__ bits,
-                                                                         const T* __restrict__ tt,
-                                                                         const float2* __restrict__ w,
-                                                                         const double* __restrict__ bscal, int mslot,
-                                                                         int skip_done, int SC, int qstride,
-                                                                         int sstride, T* __restrict__ partial) {
+__global__ void __launch_bounds__(BMM_THREADS, 2) batch_ohu_mma_kernel(const qes_batch_instance* __restrict__ inst,
+                                                                       const int4* __restrict__ items,
+                                                                       const uint32_t* __restrict__ bits,
+                                                                       const T* __restrict__ tt,
+                                                                       const float2* __restrict__ w,
+                                                                       const double* __restrict__ bscal,
+                                                                       int own_mean, int skip_done,
+                                                                       T* __restrict__ partial) {
   extern __shared__ __align__(16) uint8_t boh_sm[];
+  constexpr bool CPLX = ScalarTraits<T>::is_complex;
+  constexpr int NP = bparts<T>(), NU = 2 / NP, UG = 16 / NP;  // unit tiles and units of a group: two B tiles
+  __shared__ double mred[BMM_WARPS];
   const int4 it = items[blockIdx.x];
   const double* sc = bscal + (int64_t)it.x * BSC;
   if (skip_done && sc[4] != 0.0) return;
   const qes_batch_instance I = inst[it.x];
   const int ns = I.ns, nh = I.nh, nw = n_words(ns);
-  const int nsp = bohu_round4(ns + 1), nqp = bohu_round4(nh + 1);
-  const int nst = nsp / 4, nmt = nqp / 4, n_tiles = nst * nmt;
   const int64_t rows = batch_rows(I);
-  T* Q = reinterpret_cast<T*>(boh_sm);                                       // [SC][qstride]
-  float* sig = reinterpret_cast<float*>(boh_sm + bsmall_align16((int64_t)SC * qstride * sizeof(T)));   // [SC][sstride]
-  const int tid = threadIdx.x, nthr = blockDim.x;
-  const float mr = (float)sc[mslot], mi = (float)sc[mslot + 1];
-  const float fs = (float)(1.0 / (double)rows);
-  const uint32_t* bw = bits + I.sample_word_off;
-  const T* tb = tt + I.tanh_off;
-  const float2* wb = w + I.sample_off;
   const int64_t sbeg = (int64_t)it.y * OHU_SPLIT_SAMPLES;
-  const int64_t send = min(rows, sbeg + OHU_SPLIT_SAMPLES);
-  // staging coordinates, divided once: Q entry (sl, m) and sign entry (sl, i)
-  const int qm = tid % nqp, qs0 = tid / nqp, qsd = nthr / nqp;
-  const int si = tid % nsp, ss0 = tid / nsp, ssd = nthr / nsp;
-  const int64_t P = (int64_t)ns + nh + (int64_t)ns * nh;
-  T* out = partial + I.sr_part_off + (int64_t)it.y * P;
-  // small problems: the block's threads form G sample groups over the tiles (group g takes the
-  // samples g, g + G, ...), summed in a fixed order at the end; large ones take passes over the tiles
-  const int G = (n_tiles <= nthr) ? nthr / n_tiles : 1;
-  for (int t0 = 0; t0 < n_tiles; t0 += nthr) {
-    const int t = (G > 1) ? tid % n_tiles : t0 + tid;
-    const int grp = (G > 1) ? tid / n_tiles : 0;
-    const bool active = (G > 1) ? grp < G : t < n_tiles;
-    const int tm = active ? t % nmt : 0, ti = active ? t / nmt : 0;
-    T acc[4][4];
+  const int nc = (int)min((int64_t)OHU_SPLIT_SAMPLES, rows - sbeg);
+  const int ng = batch_ohu_ng(nh, NP), parts = batch_ohu_parts(ng);
+  T* us = reinterpret_cast<T*>(boh_sm);                                        // [256], zero past nc
+  uint32_t* ws = reinterpret_cast<uint32_t*>(us + OHU_SPLIT_SAMPLES);          // [256][nw]
+  T* ga = reinterpret_cast<T*>(boh_sm + bsmall_align16((int64_t)OHU_SPLIT_SAMPLES * (sizeof(T) + 4 * nw)));   // [warps][ns]
+  float* red = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(ga) + bsmall_align16((int64_t)BMM_WARPS * ns * sizeof(T)));
+  const int tid = threadIdx.x, lane = tid & 31, wv = tid >> 5, g = lane >> 2, t = lane & 3;
+  const uint32_t* bw = bits + I.sample_word_off + sbeg * nw;
+  const T* tb = tt + I.tanh_off + sbeg * nh;
+  const float2* wb = w + I.sample_off;
+  T* out = partial + I.sr_part_off + (int64_t)it.y * batch_P(I);
+  for (int e = tid; e < OHU_SPLIT_SAMPLES * nw; e += BMM_THREADS) ws[e] = e < nc * nw ? bw[e] : 0u;
+  float mr, mi;
+  if (own_mean) {
+    double sr = 0, si = 0;
+#pragma unroll 8
+    for (int64_t k = tid; k < rows; k += BMM_THREADS) { sr += wb[k].x; si += wb[k].y; }
+    mr = (float)(block_allsum(sr, mred) / (double)rows);
+    mi = CPLX ? (float)(block_allsum(si, mred) / (double)rows) : 0.f;
+  } else {
+    mr = (float)sc[9];
+    mi = (float)sc[10];
+  }
+  const float fs = (float)(1.0 / (double)rows);
+  for (int sl = tid; sl < OHU_SPLIT_SAMPLES; sl += BMM_THREADS) {
+    const float2 wv2 = sl < nc ? wb[sbeg + sl] : make_float2(mr, mi);
+    us[sl] = from_c(make_float2((wv2.x - mr) * fs, (wv2.y - mi) * fs), T());
+  }
+  __syncthreads();
+  // g_a: lane = site, the warp's 32 samples
+  for (int wd = 0; wd < nw; ++wd) {
+    T s = ScalarTraits<T>::zero();
+#pragma unroll 8
+    for (int sl = 32 * wv; sl < 32 * wv + 32; ++sl)
+      s = fma_s(((ws[sl * nw + wd] >> lane) & 1u) ? 1.f : -1.f, us[sl], s);
+    if (32 * wd + lane < ns) ga[wv * ns + 32 * wd + lane] = s;
+  }
+  const int part = ng >= BMM_WARPS ? 0 : wv / ng;
+  const bool warp_on = part < parts;
+  const int nk = (nc + 15) / 16, per = (nk + parts - 1) / parts;
+  const int k0 = min(nk, part * per), k1 = min(nk, k0 + per);
+  for (int gi = ng >= BMM_WARPS ? wv : wv % ng; gi < ng; gi += ng >= BMM_WARPS ? BMM_WARPS : ng) {
+    for (int mb = 0; mb < ns; mb += 64) {
+      const int MT = min(4, (ns - mb + 15) / 16);
+      float sum[4][2][4], gb[2] = {0.f, 0.f};
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
+      for (int mt = 0; mt < 4; ++mt)
 #pragma unroll
-      for (int b = 0; b < 4; ++b) acc[a][b] = ScalarTraits<T>::zero();
-    for (int64_t c0 = sbeg; c0 < send; c0 += SC) {
-      const int nc = (int)min((int64_t)SC, send - c0);
-      // staging in batches of SB rows per thread: the global loads of a batch are issued together
-      constexpr int SB = ScalarTraits<T>::is_complex ? 8 : 4;   // real: within the 64-register budget
-      if (qs0 < qsd) {
-        for (int sl0 = qs0; sl0 < SC; sl0 += SB * qsd) {
-          T tv[SB];
-          float2 wv[SB];
+        for (int j = 0; j < 2; ++j)
 #pragma unroll
-          for (int b = 0; b < SB; ++b) {
-            const int sl = sl0 + b * qsd;
-            const bool ok = sl < nc;
-            wv[b] = ok ? wb[c0 + sl] : make_float2(0.f, 0.f);
-            tv[b] = (ok && qm < nh) ? tb[(c0 + sl) * nh + qm] : ScalarTraits<T>::zero();
-          }
+          for (int x = 0; x < 4; ++x) sum[mt][j][x] = 0.f;
+      if (warp_on) {
+        T tv[NU][4];
+        auto fetch = [&](int ks) {
 #pragma unroll
-          for (int b = 0; b < SB; ++b) {
-            const int sl = sl0 + b * qsd;
-            if (sl < SC) {
-              T q = ScalarTraits<T>::zero();
-              if (sl < nc) {
-                const T u = from_c(make_float2((wv[b].x - mr) * fs, (wv[b].y - mi) * fs), T());
-                if (qm < nh) q = mulx(conjx(tv[b]), u);
-                else if (qm == nh) q = u;                                  // virtual unit: g_a
-              }
-              Q[sl * qstride + qm] = q;
+          for (int j = 0; j < NU; ++j) {
+            const int m = gi * UG + 8 * j + g;
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+              const int sl = 16 * ks + 4 * t + x;
+              tv[j][x] = (ks < k1 && sl < nc && m < nh) ? tb[(int64_t)sl * nh + m] : ScalarTraits<T>::zero();
             }
           }
-        }
-      }
-      if (ss0 < ssd) {
-        for (int sl0 = ss0; sl0 < SC; sl0 += SB * ssd) {
-          uint32_t wd[SB];
+        };
+        fetch(k0);
+        for (int kc = k0; kc < k1; kc += 4) {
+          float d[4][2][4];
 #pragma unroll
-          for (int b = 0; b < SB; ++b) {
-            const int sl = sl0 + b * ssd;
-            wd[b] = (sl < nc && si < ns) ? bw[(c0 + sl) * nw + (si >> 5)] : 0u;
-          }
+          for (int mt = 0; mt < 4; ++mt)
 #pragma unroll
-          for (int b = 0; b < SB; ++b) {
-            const int sl = sl0 + b * ssd;
-            if (sl < SC) {
-              float sg = 0.f;
-              if (sl < nc) {
-                if (si < ns) sg = ((wd[b] >> (si & 31)) & 1u) ? 1.f : -1.f;
-                else if (si == ns) sg = 1.f;                               // virtual site: g_b
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+              for (int x = 0; x < 4; ++x) d[mt][j][x] = 0.f;
+#pragma unroll 1
+          for (int ks = kc; ks < min(k1, kc + 4); ++ks) {
+            uint2 B[2][3];
+#pragma unroll
+            for (int j = 0; j < NU; ++j) {
+              T q[4];
+#pragma unroll
+              for (int x = 0; x < 4; ++x) q[x] = mulx(conjx(tv[j][x]), us[16 * ks + 4 * t + x]);
+#pragma unroll
+              for (int c = 0; c < NP; ++c) {
+                uint32_t lo[3], hi[3];
+                const float q0 = part_of(q[0], c), q1 = part_of(q[1], c), q2 = part_of(q[2], c), q3 = part_of(q[3], c);
+                gb[j * NP + c] += (q0 + q1) + (q2 + q3);
+                split3(q0, q1, lo);
+                split3(q2, q3, hi);
+#pragma unroll
+                for (int k = 0; k < 3; ++k) B[j * NP + c][k] = make_uint2(lo[k], hi[k]);
               }
-              sig[sl * sstride + si] = sg;
+            }
+            fetch(ks + 1);
+#pragma unroll
+            for (int wd = 0; wd < 2; ++wd) {
+              if (2 * wd >= MT) break;
+              uint32_t y[4];                                  // this lane's four samples, site g of each byte on top
+#pragma unroll
+              for (int x = 0; x < 4; ++x) y[x] = ws[(16 * ks + 4 * t + x) * nw + (mb >> 5) + wd] << (7 - g);
+#pragma unroll
+              for (int h = 0; h < 2; ++h) {
+                if (2 * wd + h >= MT) break;
+                uint32_t A[4];
+                if (h == 0) {
+                  A[0] = sign_pair<0, 0>(y[0], y[1]); A[1] = sign_pair<1, 1>(y[0], y[1]);
+                  A[2] = sign_pair<0, 0>(y[2], y[3]); A[3] = sign_pair<1, 1>(y[2], y[3]);
+                } else {
+                  A[0] = sign_pair<2, 2>(y[0], y[1]); A[1] = sign_pair<3, 3>(y[0], y[1]);
+                  A[2] = sign_pair<2, 2>(y[2], y[3]); A[3] = sign_pair<3, 3>(y[2], y[3]);
+                }
+#pragma unroll
+                for (int k = 2; k >= 0; --k)                  // small parts first
+#pragma unroll
+                  for (int j = 0; j < 2; ++j) mma16816(d[2 * wd + h][j], A, B[j][k]);
+              }
             }
           }
+#pragma unroll
+          for (int mt = 0; mt < 4; ++mt)
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+              for (int x = 0; x < 4; ++x) sum[mt][j][x] += d[mt][j][x];
+        }
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          gb[j] += __shfl_xor_sync(0xffffffffu, gb[j], 1);
+          gb[j] += __shfl_xor_sync(0xffffffffu, gb[j], 2);
         }
       }
-      __syncthreads();
-      if (active) {
-        for (int sl = grp; sl < nc; sl += G) {
-          const float4 s4 = *reinterpret_cast<const float4*>(sig + sl * sstride + 4 * ti);
-          T q[4];
-          if constexpr (ScalarTraits<T>::is_complex) {
-            const float4* qr = reinterpret_cast<const float4*>(Q + sl * qstride + 4 * tm);
-            const float4 q01 = qr[0], q23 = qr[1];
-            q[0] = make_float2(q01.x, q01.y); q[1] = make_float2(q01.z, q01.w);
-            q[2] = make_float2(q23.x, q23.y); q[3] = make_float2(q23.z, q23.w);
-          } else {
-            const float4 q4 = *reinterpret_cast<const float4*>(Q + sl * qstride + 4 * tm);
-            q[0] = q4.x; q[1] = q4.y; q[2] = q4.z; q[3] = q4.w;
+      if (parts > 1) {
+        // parts 1, 2, ... through shared memory, added in order by part 0 (every warp passes here once per mb)
+        if (mb) __syncthreads();
+        if (warp_on && part > 0) {
+          float* o = red + (int64_t)((part - 1) * ng + gi) * 34 * 32 + lane;
+#pragma unroll
+          for (int e = 0; e < 32; ++e) o[32 * e] = sum[e >> 3][(e >> 2) & 1][e & 3];
+          o[32 * 32] = gb[0];
+          o[32 * 33] = gb[1];
+        }
+        __syncthreads();
+        if (part == 0)
+          for (int q = 1; q < parts; ++q) {
+            const float* o = red + (int64_t)((q - 1) * ng + gi) * 34 * 32 + lane;
+#pragma unroll
+            for (int e = 0; e < 32; ++e) sum[e >> 3][(e >> 2) & 1][e & 3] += o[32 * e];
+            gb[0] += o[32 * 32];
+            gb[1] += o[32 * 33];
           }
-          const float sv[4] = {s4.x, s4.y, s4.z, s4.w};
-#pragma unroll
-          for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int b = 0; b < 4; ++b) acc[a][b] = addx(acc[a][b], scal(sv[a], q[b]));
-        }
       }
-      __syncthreads();
-    }
-    if (G > 1) {
-      // group partials through shared memory (the staging buffers are free), group 0 adds them
-      T* gred = reinterpret_cast<T*>(boh_sm);             // [G][n_tiles][16]
-      if (active) {
+      if (part == 0) {
 #pragma unroll
-        for (int a = 0; a < 4; ++a)
+        for (int mt = 0; mt < 4; ++mt)
 #pragma unroll
-          for (int b = 0; b < 4; ++b) gred[((size_t)grp * n_tiles + t) * 16 + a * 4 + b] = acc[a][b];
-      }
-      __syncthreads();
-      if (active && grp == 0) {
-        for (int g = 1; g < G; ++g)
+          for (int r = 0; r < 2; ++r)
 #pragma unroll
-          for (int a = 0; a < 4; ++a)
+            for (int j = 0; j < NU; ++j)
 #pragma unroll
-            for (int b = 0; b < 4; ++b) acc[a][b] = addx(acc[a][b], gred[((size_t)g * n_tiles + t) * 16 + a * 4 + b]);
-      }
-    }
-    if (active && grp == 0) {
+              for (int x = 0; x < 2; ++x) {
+                const int i = mb + 16 * mt + 8 * r + g, m = gi * UG + 8 * j + 2 * t + x;
+                if (i < ns && m < nh) {
+                  T v;
+                  if constexpr (CPLX) v = make_float2(sum[mt][0][2 * r + x], sum[mt][1][2 * r + x]);
+                  else v = sum[mt][j][2 * r + x];
+                  out[ns + nh + (int64_t)i * nh + m] = v;
+                }
+              }
+        if (mb == 0 && t == 0)
 #pragma unroll
-      for (int a = 0; a < 4; ++a) {
-        const int i = 4 * ti + a;
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-          const int m = 4 * tm + b;
-          if (i < ns && m < nh) out[ns + nh + (int64_t)i * nh + m] = acc[a][b];
-          else if (i == ns && m < nh) out[ns + m] = acc[a][b];
-          else if (i < ns && m == nh) out[i] = acc[a][b];
-        }
+          for (int j = 0; j < NU; ++j) {
+            const int m = gi * UG + 8 * j + g;
+            if (m < nh) {
+              T v;
+              if constexpr (CPLX) v = make_float2(gb[0], gb[1]);
+              else v = gb[j];
+              out[ns + m] = v;
+            }
+          }
       }
     }
   }
+  __syncthreads();
+  for (int i = tid; i < ns; i += BMM_THREADS) {
+    T s = ga[i];
+#pragma unroll
+    for (int q = 1; q < BMM_WARPS; ++q) s = addx(s, ga[q * ns + i]);
+    out[i] = s;
+  }
 }
 
-// b = sum of the force partials; x = 0, r = p = b; CG scalars (one block per problem)
+// b = sum of the force partials; x = 0, r = p = b (and p in float32); CG scalars (one block per problem)
 template <class T, class V>
 __global__ void __launch_bounds__(BCG_THREADS) batch_cg_setup_kernel(const qes_batch_instance* __restrict__ inst,
                                                                     const T* __restrict__ partial, double rtol,
                                                                     double atol, V* __restrict__ x, V* __restrict__ r,
-                                                                    V* __restrict__ p, V* __restrict__ bvec,
+                                                                    V* __restrict__ p, T* __restrict__ pf,
                                                                     double* __restrict__ bscal,
                                                                     unsigned int* __restrict__ n_done) {
   const qes_batch_instance I = inst[blockIdx.x];
@@ -3223,10 +3355,10 @@ __global__ void __launch_bounds__(BCG_THREADS) batch_cg_setup_kernel(const qes_b
   for (int64_t k = threadIdx.x; k < P; k += blockDim.x) {
     V g = vzero(V());
     for (int z = 0; z < nz; ++z) g = vadd(g, to_d(part[(int64_t)z * P + k]));
-    bvec[o + k] = g;
     x[o + k] = vzero(V());
     r[o + k] = g;
     p[o + k] = g;
+    pf[o + k] = to_f(g);
     d += vdotc(g, g);
   }
   __shared__ double red[BCG_THREADS / 32];
@@ -3241,55 +3373,79 @@ __global__ void __launch_bounds__(BCG_THREADS) batch_cg_setup_kernel(const qes_b
   }
 }
 
-// y = sum of the matvec partials + shift p; alpha; x += alpha p; r -= alpha y; beta; p = r + beta p
+// y = sum of the matvec partials + shift p; alpha; x += alpha p; r -= alpha y; beta; p = r + beta p.  A cluster of
+// BUPD_CL blocks per problem, each with a quarter of the entries: p and y (then r) stay in shared memory between the
+// three steps, the two dot products meet through the cluster's shared memory in rank order.  Bound by latency: with
+// one block per problem and the vectors read back from global memory it took twice as long.
+constexpr int BUPD_CL = 4, BUPD_THREADS = 512;
 template <class T, class V>
-__global__ void __launch_bounds__(BCG_THREADS) batch_cg_update_kernel(const qes_batch_instance* __restrict__ inst,
-                                                                     const T* __restrict__ partial, double shift,
-                                                                     V* __restrict__ x, V* __restrict__ r,
-                                                                     V* __restrict__ p, V* __restrict__ Ap,
-                                                                     double* __restrict__ bscal,
-                                                                     unsigned int* __restrict__ n_done) {
-  double* sc = bscal + (int64_t)blockIdx.x * BSC;
-  if (sc[4] != 0.0) return;
-  const qes_batch_instance I = inst[blockIdx.x];
+__global__ void __launch_bounds__(BUPD_THREADS) __cluster_dims__(BUPD_CL, 1, 1)
+    batch_cg_update_kernel(const qes_batch_instance* __restrict__ inst, const T* __restrict__ partial, double shift,
+                           V* __restrict__ x, V* __restrict__ r, V* __restrict__ p, T* __restrict__ pf,
+                           double* __restrict__ bscal, unsigned int* __restrict__ n_done) {
+  namespace cgrp = cooperative_groups;
+  cgrp::cluster_group cl = cgrp::this_cluster();
+  extern __shared__ __align__(16) uint8_t bup_sm[];
+  __shared__ double red[BUPD_THREADS / 32], dot[2];
+  const int b = blockIdx.x / BUPD_CL, rank = (int)cl.block_rank();
+  double* sc = bscal + (int64_t)b * BSC;
+  if (sc[4] != 0.0) return;                                   // the same for all blocks of the cluster
+  const double rs = sc[0], th2 = sc[3];
+  const qes_batch_instance I = inst[b];
   const int64_t P = batch_P(I), o = I.param_off;
+  const int64_t per = (P + BUPD_CL - 1) / BUPD_CL, k0 = min(P, per * rank), n = min(P, k0 + per) - k0;
+  V* ps = reinterpret_cast<V*>(bup_sm);
+  V* ys = ps + per;
   const int nz = batch_nsplit(I);
-  const T* part = partial + I.sr_part_off;
-  __shared__ double red[BCG_THREADS / 32];
+  const T* part = partial + I.sr_part_off + k0;
   double d = 0.0;
   // the split loads of an element are issued together (fixed summation order)
-  for (int64_t k = threadIdx.x; k < P; k += blockDim.x) {
-    const V pk = p[o + k];
+  for (int64_t k = threadIdx.x; k < n; k += BUPD_THREADS) {
+    const V pk = p[o + k0 + k];
     V g = vzero(V());
     int z = 0;
     for (; z + 8 <= nz; z += 8) {
       T q[8];
 #pragma unroll
-      for (int b = 0; b < 8; ++b) q[b] = part[(int64_t)(z + b) * P + k];
+      for (int e = 0; e < 8; ++e) q[e] = part[(int64_t)(z + e) * P + k];
 #pragma unroll
-      for (int b = 0; b < 8; ++b) g = vadd(g, to_d(q[b]));
+      for (int e = 0; e < 8; ++e) g = vadd(g, to_d(q[e]));
     }
     for (; z < nz; ++z) g = vadd(g, to_d(part[(int64_t)z * P + k]));
     g = vadd(g, vscale(shift, pk));
-    Ap[o + k] = g;
+    ps[k] = pk;
+    ys[k] = g;
     d += vdotc(pk, g);
   }
-  const double pap = block_allsum(d, red);
-  const double alpha = (pap > 0.0) ? sc[0] / pap : 0.0;
+  auto cluster_sum = [&](double v, int slot) {
+    v = block_allsum(v, red);
+    if (threadIdx.x == 0) dot[slot] = v;
+    cl.sync();
+    double s = 0.0;
+    for (int q = 0; q < BUPD_CL; ++q) s += *cl.map_shared_rank(&dot[slot], q);
+    return s;
+  };
+  const double pap = cluster_sum(d, 0);
+  const double alpha = (pap > 0.0) ? rs / pap : 0.0;
   double e = 0.0;
-  for (int64_t k = threadIdx.x; k < P; k += blockDim.x) {
-    x[o + k] = vadd(x[o + k], vscale(alpha, p[o + k]));
-    const V rk = vadd(r[o + k], vscale(-alpha, Ap[o + k]));
-    r[o + k] = rk;
+  for (int64_t k = threadIdx.x; k < n; k += BUPD_THREADS) {
+    x[o + k0 + k] = vadd(x[o + k0 + k], vscale(alpha, ps[k]));
+    const V rk = vadd(r[o + k0 + k], vscale(-alpha, ys[k]));
+    r[o + k0 + k] = rk;
+    ys[k] = rk;
     e += vdotc(rk, rk);
   }
-  const double rr_new = block_allsum(e, red);
-  const double beta = (sc[0] > 0.0) ? rr_new / sc[0] : 0.0;
-  const bool conv = rr_new <= sc[3];
+  const double rr_new = cluster_sum(e, 1);
+  const double beta = (rs > 0.0) ? rr_new / rs : 0.0;
+  const bool conv = rr_new <= th2;
   if (!conv)
-    for (int64_t k = threadIdx.x; k < P; k += blockDim.x) p[o + k] = vadd(r[o + k], vscale(beta, p[o + k]));
-  __syncthreads();
-  if (threadIdx.x == 0) {
+    for (int64_t k = threadIdx.x; k < n; k += BUPD_THREADS) {
+      const V pk = vadd(ys[k], vscale(beta, ps[k]));
+      p[o + k0 + k] = pk;
+      pf[o + k0 + k] = to_f(pk);
+    }
+  cl.sync();                                                  // the others have read dot and the scalars
+  if (rank == 0 && threadIdx.x == 0) {
     sc[1] = pap; sc[7] = alpha; sc[2] = rr_new; sc[8] = beta; sc[0] = rr_new;
     sc[5] += 1.0;
     if (conv) {
@@ -3304,7 +3460,7 @@ struct BatchSRWork {
   unsigned int* n_done; // [1] (+pad)
   float2* w;            // [n_samples_total]
   void* partial;        // [sr_part_total] of T
-  void *r, *p, *Ap, *b; // [n_params_total] of V each
+  void *r, *p, *Ap, *pf; // [n_params_total] of V each (pf: p in float32)
 };
 
 static size_t batch_sr_layout(int dtype, int n_inst, int64_t n_params_total, int64_t n_samples_total,
@@ -3322,7 +3478,7 @@ static size_t batch_sr_layout(int dtype, int n_inst, int64_t n_params_total, int
   W.r = take((size_t)n_params_total * vs);
   W.p = take((size_t)n_params_total * vs);
   W.Ap = take((size_t)n_params_total * vs);
-  W.b = take((size_t)n_params_total * vs);
+  W.pf = take((size_t)n_params_total * vs);
   if (L) *L = W;
   return off;
 }
@@ -3335,40 +3491,39 @@ extern "C" int qes_batch_sr_workspace_bytes(int dtype, int n_inst, int64_t n_par
   return QES_OK;
 }
 
-template <class T, class V>
-static int launch_batch_ov(int n_ov, int threads, size_t smem, const qes_batch_instance* inst, const int4* items,
-                           const uint32_t* bits, const T* tt, const V* p, float2* w, const double* bscal,
+template <class T>
+static int launch_batch_ov(int n_ov, size_t smem, const qes_batch_instance* inst, const int4* items,
+                           const uint32_t* bits, const T* tt, const T* pf, float2* w, const double* bscal,
                            cudaStream_t st) {
-  QES_CUDA_CHECK(cudaFuncSetAttribute(batch_ov_tile_kernel<T, V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem));
-  const int pf = qes_prof_begin(QES_PROF_OV, st);
-  batch_ov_tile_kernel<T, V><<<n_ov, threads, smem, st>>>(inst, items, bits, tt, p, w, bscal);
-  qes_prof_end(pf, st);
+  QES_CUDA_CHECK(cudaFuncSetAttribute(batch_ov_mma_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int pr = qes_prof_begin(QES_PROF_OV, st);
+  batch_ov_mma_kernel<T><<<n_ov, BMM_THREADS, smem, st>>>(inst, items, bits, tt, pf, w, bscal);
+  qes_prof_end(pr, st);
   return QES_OK;
 }
 
 template <class T>
-static int launch_batch_ohu(int n_ohu, int threads, int SC, int qstride, int sstride, size_t smem,
-                            const qes_batch_instance* inst, const int4* items, const uint32_t* bits, const T* tt,
-                            const float2* w, const double* bscal, int skip_done, T* partial, cudaStream_t st) {
-  QES_CUDA_CHECK(cudaFuncSetAttribute(batch_ohu_tile_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+static int launch_batch_ohu(int n_ohu, size_t smem, const qes_batch_instance* inst, const int4* items,
+                            const uint32_t* bits, const T* tt, const float2* w, const double* bscal, int own_mean,
+                            int skip_done, T* partial, cudaStream_t st) {
+  QES_CUDA_CHECK(cudaFuncSetAttribute(batch_ohu_mma_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)smem));
-  const int pf = qes_prof_begin(QES_PROF_OHU, st);
-  batch_ohu_tile_kernel<T><<<n_ohu, threads, smem, st>>>(inst, items, bits, tt, w, bscal, 9, skip_done, SC, qstride,
-                                                         sstride, partial);
-  qes_prof_end(pf, st);
+  const int pr = qes_prof_begin(QES_PROF_OHU, st);
+  batch_ohu_mma_kernel<T><<<n_ohu, BMM_THREADS, smem, st>>>(inst, items, bits, tt, w, bscal, own_mean, skip_done,
+                                                              partial);
+  qes_prof_end(pr, st);
   return QES_OK;
 }
 
 struct BatchGraphKey {
   const void* inst; const void* ov_items; const void* ohu_items; const void* bits; const void* tt; const void* x;
   const void* bscal;
-  int n_inst, n_ov, n_ohu, chunk, cplx, ov_threads, ohu_threads, ohu_sc, ohu_qstride, ohu_sstride, pad0, pad1;
-  int64_t ov_smem, ohu_smem;
+  int n_inst, n_ov, n_ohu, chunk, cplx, own_mean;
+  int64_t ov_smem, ohu_smem, upd_smem;
   double shift;
   bool operator==(const BatchGraphKey& o) const { return std::memcmp(this, &o, sizeof(*this)) == 0; }
 };
-static_assert(sizeof(BatchGraphKey) == 7 * sizeof(void*) + 12 * 4 + 2 * 8 + 8, "BatchGraphKey has padding bytes");
+static_assert(sizeof(BatchGraphKey) == 7 * sizeof(void*) + 6 * 4 + 3 * 8 + 8, "BatchGraphKey has padding bytes");
 struct BatchGraphSlot {
   bool init = false;
   cudaStream_t cs = nullptr;
@@ -3388,51 +3543,42 @@ static int batch_sr_cg_t(int n_inst, const qes_batch_instance* inst, int n_ov, c
   using V = typename VecT<T>::type;
   constexpr bool CPLX = ScalarTraits<T>::is_complex;
   T* partial = (T*)L.partial;
-  V* r = (V*)L.r; V* p = (V*)L.p; V* Ap = (V*)L.Ap; V* b = (V*)L.b;
+  V* r = (V*)L.r; V* p = (V*)L.p; T* pf = (T*)L.pf;
   // the shapes pick the kernel variants: read the descriptors once
   std::vector<qes_batch_instance> hi(n_inst);
   QES_CUDA_CHECK(cudaMemcpyAsync(hi.data(), inst, n_inst * sizeof(qes_batch_instance), cudaMemcpyDeviceToHost, st));
   QES_CUDA_CHECK(cudaStreamSynchronize(st));
-  int max_nh = 1, max_ns = 1, max_tiles = 1;
-  size_t ov_smem = 0;
+  size_t ov_smem = 0, ohu_smem = 0, upd_smem = 0;
+  int64_t max_rows = 0;
   for (const auto& d : hi) {
     if (d.ns <= 0 || d.nh <= 0 || d.nh > 512 || d.ns >= 512 || (int64_t)d.ns * d.nh > (CPLX ? 8192 : 16384)) {
       qes_set_last_message("qes_batch_sr_solve_cg: a problem exceeds ns*nh <= 16384 (real) / 8192 (complex), "
                            "nh <= 512");
       return QES_ERR_SIZE;
     }
-    max_nh = std::max(max_nh, d.nh);
-    max_ns = std::max(max_ns, d.ns);
-    max_tiles = std::max(max_tiles, batch_ohu_tiles(d.ns, d.nh));
+    const int64_t P = (int64_t)d.ns + d.nh + (int64_t)d.ns * d.nh;
     ov_smem = std::max(ov_smem, batch_ov_smem<T>(d.ns, d.nh));
+    ohu_smem = std::max(ohu_smem, batch_ohu_smem<T>(d.ns, d.nh));
+    upd_smem = std::max(upd_smem, (size_t)((P + BUPD_CL - 1) / BUPD_CL) * 2 * sizeof(V));
+    max_rows = std::max(max_rows, (int64_t)d.n_chains * d.num_samples);
   }
-  // O^H u: one block size for every split (enough threads for the largest problem's tiles)
-  const int ohu_qstride = bohu_round4(max_nh + 1), ohu_sstride = bohu_round4(max_ns + 1);
-  // at least one thread per staged row entry (q values and signs), at most 1024 (real) / 512
-  // (complex); tiles beyond take further passes
-  const int ohu_threads =
-      std::min(bohu_max_threads<T>(), (std::max({max_tiles, ohu_qstride, ohu_sstride}) + 31) / 32 * 32);
-  const int ohu_sc = batch_ohu_sc<T>(max_ns, max_nh);
-  const size_t ohu_smem = std::max((size_t)bsmall_align16((int64_t)ohu_sc * ohu_qstride * sizeof(T)) +
-                                       (size_t)ohu_sc * ohu_sstride * sizeof(float),
-                                   (size_t)ohu_threads * 16 * sizeof(T));      // sample-group partials
-  // O v: enough threads for the staging rows (BOV_ROWS signs, nh + ... V columns) and the tiles
-  const int ov_threads = std::min(bohu_max_threads<T>(),
-                                  (std::max({(BOV_ROWS / 4) * (bov_round4(max_nh) / 4), bov_round4(max_nh), BOV_ROWS}) +
-                                   31) / 32 * 32);
-  auto ov = [&](const V* vec) -> int {
-    return launch_batch_ov<T, V>(n_ov, ov_threads, ov_smem, inst, ov_items, bits, tt, vec, L.w, L.bscal, st);
+  // the mean of w: every O^H u block reads all rows of its problem, which grows with the square of the rows; beyond
+  // BMEAN_ROWS (64 blocks of 128 KB each from L2) one launch per iteration does it
+  const int own_mean = max_rows <= BMEAN_ROWS ? 1 : 0;
+  QES_CUDA_CHECK(cudaFuncSetAttribute(batch_cg_update_kernel<T, V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)upd_smem));
+  auto ov = [&]() -> int {
+    return launch_batch_ov<T>(n_ov, ov_smem, inst, ov_items, bits, tt, pf, L.w, L.bscal, st);
   };
-  auto ohu = [&](const float2* g, int skip) -> int {
-    return launch_batch_ohu<T>(n_ohu, ohu_threads, ohu_sc, ohu_qstride, ohu_sstride, ohu_smem, inst, ohu_items, bits,
-                               tt, g, L.bscal, skip, partial, st);
+  auto ohu = [&](const float2* g, int mean, int skip) -> int {
+    return launch_batch_ohu<T>(n_ohu, ohu_smem, inst, ohu_items, bits, tt, g, L.bscal, mean, skip, partial, st);
   };
   int rc;
   QES_CUDA_CHECK(cudaMemsetAsync(L.n_done, 0, sizeof(unsigned int), st));
   // force: mean of E_loc, O^H (E - mean) / rows, then CG set-up
   batch_mean_kernel<<<n_inst, BCG_THREADS, 0, st>>>(inst, eloc, L.bscal, 9, 0);
-  if ((rc = ohu(eloc, 0))) return rc;
-  batch_cg_setup_kernel<T, V><<<n_inst, BCG_THREADS, 0, st>>>(inst, partial, opt->rtol, opt->atol, x, r, p, b,
+  if ((rc = ohu(eloc, 0, 0))) return rc;
+  batch_cg_setup_kernel<T, V><<<n_inst, BCG_THREADS, 0, st>>>(inst, partial, opt->rtol, opt->atol, x, r, p, pf,
                                                               L.bscal, L.n_done);
   QES_LAUNCH_CHECK_N(3);
   const int check = opt->check_every > 0 ? opt->check_every : 8;
@@ -3443,19 +3589,22 @@ static int batch_sr_cg_t(int n_inst, const qes_batch_instance* inst, int n_ov, c
   auto run_chunk = [&](int nrun) -> int {
     for (int q = 0; q < nrun; ++q) {
       int r2;
-      if ((r2 = ov(p))) return r2;
-      batch_mean_kernel<<<n_inst, BCG_THREADS, 0, st>>>(inst, L.w, L.bscal, 9, 1);
-      if ((r2 = ohu(L.w, 1))) return r2;
+      if ((r2 = ov())) return r2;
+      if (!own_mean) {
+        batch_mean_kernel<<<n_inst, BCG_THREADS, 0, st>>>(inst, L.w, L.bscal, 9, 1);
+        QES_LAUNCH_CHECK();
+      }
+      if ((r2 = ohu(L.w, own_mean, 1))) return r2;
       const int pfr = qes_prof_begin(QES_PROF_REDUCE, st);
-      batch_cg_update_kernel<T, V><<<n_inst, BCG_THREADS, 0, st>>>(inst, partial, opt->shift, x, r, p, Ap, L.bscal,
-                                                                   L.n_done);
+      batch_cg_update_kernel<T, V><<<n_inst * BUPD_CL, BUPD_THREADS, upd_smem, st>>>(inst, partial, opt->shift, x, r, p,
+                                                                                     pf, L.bscal, L.n_done);
       qes_prof_end(pfr, st);
-      QES_LAUNCH_CHECK_N(4);
+      QES_LAUNCH_CHECK_N(3);
     }
     return QES_OK;
   };
   // Full chunks run as one CUDA graph on a private stream (captured once per launch configuration
-  // and set of buffers, then replayed): four launches per lockstep iteration otherwise
+  // and set of buffers, then replayed): three launches per lockstep iteration otherwise
   int dev = 0;
   QES_CUDA_CHECK(cudaGetDevice(&dev));
   const bool graphs = g_use_graphs.load() != 0 && !qes_prof_on() && dev >= 0 && dev < kMaxGraphDevices;
@@ -3473,8 +3622,8 @@ static int batch_sr_cg_t(int n_inst, const qes_batch_instance* inst, int n_ov, c
         gs.init = true;
       }
       const BatchGraphKey key{inst, ov_items, ohu_items, bits, tt, x, L.bscal, n_inst, n_ov, n_ohu, nrun,
-                              CPLX ? 1 : 0, ov_threads, ohu_threads, ohu_sc, ohu_qstride, ohu_sstride, 0, 0,
-                              (int64_t)ov_smem, (int64_t)ohu_smem, opt->shift};
+                              CPLX ? 1 : 0, own_mean, (int64_t)ov_smem, (int64_t)ohu_smem,
+                              (int64_t)upd_smem, opt->shift};
       if (gs.exec == nullptr || !(gs.key == key)) {
         if (gs.exec) {
           cudaGraphExecDestroy(gs.exec);

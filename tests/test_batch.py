@@ -132,3 +132,41 @@ def test_batch_autotune_persists_choice(tmp_path):
     B2 = NQSBatch(models, alpha=2, dtype="float32", s_numchains=64, s_numsamples=2, autotune=False,
                   warps_per_block=1, blocks_per_sm=1)
     assert B2.autotune_sampler(cache=str(cache)) == tuple(best)
+
+
+# (chain lengths, alpha, chains, samples): hidden units and sites at the edges of the 16 x 8 tiles and the 32-site words, rows
+# at those of a warp's 32 and the 256 samples of O^H u; several passes over the sites; the largest shared
+# memory; more rows than the blocks of O^H u sum themselves
+@pytest.mark.parametrize("dtype,Ls,alpha,chains,nsamp", [
+    ("float32", [2, 7, 8, 9, 16, 33], 1.0, 37, 9), ("float32", [31, 32, 64], 2.0, 16, 16),
+    ("float32", [500, 17], 0.06, 13, 5), ("float32", [128], 1.0, 8, 17), ("float32", [6], 2.0, 2050, 8),
+    ("float32", [33], 15.0, 8, 8), ("complex64", [16], 32.0, 8, 5),
+    ("complex64", [2, 7, 8, 9, 24], 1.5, 37, 9), ("complex64", [400, 20], 0.05, 13, 5), ("complex64", [64], 2.0, 43, 3)])
+def test_batched_solve_at_tile_edges(dtype, Ls, alpha, chains, nsamp):
+    models = [tfim_chain(L, 1.1) for L in Ls]
+    B = NQSBatch(models, alpha=alpha, dtype=dtype, seeds=list(range(5, 5 + len(Ls))), s_numchains=chains,
+                 s_numsamples=nsamp, init_scale=0.05, autotune=False, warps_per_block=4, blocks_per_sm=2)
+    B.sample()
+    B.forward()
+    B.local_energy()
+    shift, rtol = 0.05, 1e-6
+    x, _ = B.sr_solve(shift=shift, rtol=rtol, maxiter=2000, rhs_prefactor=1.0)
+    xs = x.cpu().numpy()
+    for b, L in enumerate(Ls):
+        bits, _ = B.samples(b)
+        sig = 2.0 * dv.unpack_states(bits, L).cpu().numpy()
+        t = B.tanh_theta(b).cpu().numpy()
+        t = t.astype(np.complex128 if dtype == "complex64" else np.float64).reshape(len(sig), -1)
+        O = np.concatenate([sig.astype(t.dtype), t, (sig[:, :, None] * t[:, None, :]).reshape(len(sig), -1)], axis=1)
+        O = O - O.mean(0)
+        n = len(sig)
+        e = B.local_energies(b).cpu().numpy().astype(np.complex128).reshape(-1)
+        e = e if dtype == "complex64" else e.real
+        F = O.conj().T @ (e - e.mean()) / n
+        xb = xs[int(B.param_off[b]):int(B.param_off[b]) + O.shape[1]]
+        r = O.conj().T @ (O @ xb) / n + shift * xb - F
+        G = O @ O.conj().T / n if n <= O.shape[1] else O.conj().T @ O / n
+        kappa = np.linalg.norm(G, 2) / shift + 1.0
+        # the CG's own bar, and float32 sums of up to max(n, L, nh) terms in an operator of condition kappa
+        tol = rtol + 4.0 * np.sqrt(max(n, L, t.shape[1])) * 2.0 ** -24 * kappa
+        assert np.linalg.norm(r) <= tol * np.linalg.norm(F), (L, np.linalg.norm(r) / np.linalg.norm(F), tol)
