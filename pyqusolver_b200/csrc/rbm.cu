@@ -247,16 +247,19 @@ extern "C" int qes_rbm_move_tables(int dtype, int ns, int nh, const void* a, con
 // forward: theta, tanh(theta), log psi
 // ----------------------------------------------------------------------------
 // Register-tiled contraction: a block of 32 x 8 threads takes 8 RS samples and walks the hidden units 128 at a
-// time, a thread accumulating RS samples x 4 units.  Per 32 sites the block stages the spins as +-1 floats
-// and the W rows in shared memory, so that a site costs a thread 2 or 3 16-byte loads for 4 RS (real) or
+// time, a thread accumulating RS samples x 4 units: real, units 4 lane ..; complex, lane, lane + 32, ..., since
+// there tanh and log cosh, not the multiply-adds, are most of the work and a last pass of few units then skips them
+// by the 32 (2,000 samples of 36 sites x 144 units: 28.5 -> 18.8 us with log psi).  Per 32 sites the block stages the
+// spins as +-1 floats and the W rows in shared memory, so that a site costs a thread 2 or 3 16-byte loads for 4 RS (real) or
 // 8 RS (complex) multiply-adds (one thread per unit with the signs taken from the spin words needed five
 // integer and select instructions per multiply-add).  theta accumulates b, then the sites in order, each
-// product exact, so its value does not depend on the tiling.  A warp holds all units of its RS samples: log
-// psi needs one warp sum.  Bound by FP32 issue; log cosh is evaluated only where log psi is asked for.
+// product exact, so its value does not depend on the tiling.  log psi (LP) does: its terms are added as 256 threads
+// with units t, t + 256, ... would, then 32 at a time by butterflies, then the eight sums in order; a thread
+// holds the sums of its four units of both 128-unit halves.  Bound by FP32 issue.
 // W slices are copied a slice ahead (asynchronous copies into two buffers).
-// Measured (B200, 16,384 samples), the one-thread-per-unit form / this one: 20x20 x 1,600 real, tanh 2.68 / 0.64 ms,
-// log psi 2.40 / 0.67 ms (0.28 ms at the FP32 rate; 0.81 / 0.83 ms with single-buffered slices), 10x10 x 200
-// complex 189 / 130 us.
+// Measured (B200), the one-thread-per-unit form / this one: 16,384 samples of 20x20 x 1,600 real, tanh 2.41 / 0.62 ms,
+// log psi 2.40 / 0.82 ms (0.28 ms at the FP32 rate; 0.81 / 0.83 ms with single-buffered slices), of 10x10 x 200
+// complex, tanh 184 / 86 us, log psi 166 / 134 us; 4,096 samples of 16 x 32 real, 8.7 / 4.1 us.
 constexpr int FWD_SB = 16;               // samples per block of the batched form (RS = 2)
 constexpr int FWD_TX = 32, FWD_TY = 8;
 constexpr int FWD_THREADS = FWD_TX * FWD_TY;
@@ -272,12 +275,21 @@ QES_D float2 fma_sign<float2>(float sg, float2 w, float2 acc) {
   return make_float2(fmaf(sg, w.x, acc.x), fmaf(sg, w.y, acc.y));
 }
 
+QES_D float shfl_xor_val(float v, int o) { return __shfl_xor_sync(0xffffffffu, v, o); }
+QES_D float2 shfl_xor_val(float2 v, int o) {
+  return make_float2(__shfl_xor_sync(0xffffffffu, v.x, o), __shfl_xor_sync(0xffffffffu, v.y, o));
+}
+QES_D float shfl_val(float v, int l) { return __shfl_sync(0xffffffffu, v, l); }
+QES_D float2 shfl_val(float2 v, int l) {
+  return make_float2(__shfl_sync(0xffffffffu, v.x, l), __shfl_sync(0xffffffffu, v.y, l));
+}
+
 // dynamic shared memory of a block: W slices and signs, double-buffered
 template <class T, int RS>
 constexpr int fwd_smem() { return 2 * FWD_K * (FWD_U * (int)sizeof(T) + FWD_TY * RS * 4); }
 
-// one block of 8 RS samples starting at row s0; VEC: W rows start on 16-byte boundaries
-template <class T, int RS, bool VEC>
+// one block of 8 RS samples starting at row s0; VEC: W rows start on 16-byte boundaries; LP: log psi asked for
+template <class T, int RS, bool VEC, bool LP>
 QES_D void rbm_forward_block(uint8_t* smem, int64_t s0, int ns, int nh, int64_t n_samples,
                              const uint32_t* __restrict__ bits, const T* __restrict__ a, const T* __restrict__ b,
                              const T* __restrict__ W, T* __restrict__ theta_out, T* __restrict__ tanh_out,
@@ -287,9 +299,14 @@ QES_D void rbm_forward_block(uint8_t* smem, int64_t s0, int ns, int nh, int64_t 
   float* sg_all = reinterpret_cast<float*>(smem + 2 * FWD_K * FWD_U * sizeof(T));       // [2][FWD_K][TS]
   const int nw = n_words(ns);
   const int tid = threadIdx.x, lane = tid & 31, row = tid >> 5;
-  T lsum[RS];
+  constexpr bool CPLX = ScalarTraits<T>::is_complex;
+  T lsum[LP ? RS : 1][2][4];                  // of the virtual threads 128 h + (unit of c)
 #pragma unroll
-  for (int q = 0; q < RS; ++q) lsum[q] = ScalarTraits<T>::zero();
+  for (int q = 0; q < (LP ? RS : 1); ++q)
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) lsum[q][h][c] = ScalarTraits<T>::zero();
   // 16-byte stores where every row's groups of 4 units start on a 16-byte boundary
   const bool vec = nh % 4 == 0 && ((reinterpret_cast<uintptr_t>(theta_out) | reinterpret_cast<uintptr_t>(tanh_out)) & 15) == 0;
   // slice q = (unit pass, spin word): W by asynchronous copies, the spins of row tid % TS as +-1
@@ -323,11 +340,12 @@ QES_D void rbm_forward_block(uint8_t* smem, int64_t s0, int ns, int nh, int64_t 
   if (total > 1) next_word = spin_word(1);
   int q_sl = 0;
   for (int u0 = 0; u0 < nh; u0 += FWD_U) {
-    const int m0 = u0 + 4 * lane;
+    const int m0 = u0 + (CPLX ? 1 : 4) * lane;                // unit c: m0 + c, complex m0 + 32 c
+    constexpr int MC = CPLX ? 32 : 1;
     T acc[RS][4];
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
-      const T bm = (m0 + c < nh) ? b[m0 + c] : ScalarTraits<T>::zero();
+      const T bm = (m0 + MC * c < nh) ? b[m0 + MC * c] : ScalarTraits<T>::zero();
 #pragma unroll
       for (int q = 0; q < RS; ++q) acc[q][c] = bm;
     }
@@ -339,16 +357,14 @@ QES_D void rbm_forward_block(uint8_t* smem, int64_t s0, int ns, int nh, int64_t 
         stage(q_sl + 1, buf ^ 1, next_word);
         if (q_sl + 2 < total) next_word = spin_word(q_sl + 2);
       }
-      const T* ws = ws_all + buf * FWD_K * FWD_U + 4 * lane;
+      const T* ws = ws_all + buf * FWD_K * FWD_U + (CPLX ? 1 : 4) * lane;
       const float* sg = sg_all + buf * FWD_K * TS + RS * row;
 #pragma unroll 8
       for (int il = 0; il < FWD_K; ++il) {
         T w[4];
-        if constexpr (ScalarTraits<T>::is_complex) {
-          const float4 w01 = reinterpret_cast<const float4*>(ws + il * FWD_U)[0];
-          const float4 w23 = reinterpret_cast<const float4*>(ws + il * FWD_U)[1];
-          w[0] = make_float2(w01.x, w01.y); w[1] = make_float2(w01.z, w01.w);
-          w[2] = make_float2(w23.x, w23.y); w[3] = make_float2(w23.z, w23.w);
+        if constexpr (CPLX) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) w[c] = ws[il * FWD_U + 32 * c];
         } else {
           const float4 w4 = *reinterpret_cast<const float4*>(ws + il * FWD_U);
           w[0] = w4.x; w[1] = w4.y; w[2] = w4.z; w[3] = w4.w;
@@ -374,65 +390,86 @@ QES_D void rbm_forward_block(uint8_t* smem, int64_t s0, int ns, int nh, int64_t 
     for (int q = 0; q < RS; ++q) {
       const int64_t s = s0 + RS * row + q;
       if (s < n_samples) {
-        T t[4];
-        if (tanh_out) {
-#pragma unroll
-          for (int c = 0; c < 4; ++c) t[c] = tanhx(acc[q][c]);
-        }
         const int64_t o = s * nh + m0;
-        if (vec && m0 < nh) {
-          constexpr int NV = (int)sizeof(T) / 4;             // 16-byte vectors of 4 units
-#pragma unroll
-          for (int z = 0; z < NV; ++z) {
-            if (theta_out) reinterpret_cast<float4*>(theta_out + o)[z] = reinterpret_cast<const float4*>(acc[q])[z];
-            if (tanh_out) reinterpret_cast<float4*>(tanh_out + o)[z] = reinterpret_cast<const float4*>(t)[z];
-          }
-        } else {
+        if (CPLX || !vec) {
 #pragma unroll
           for (int c = 0; c < 4; ++c)
-            if (m0 + c < nh) {
-              if (theta_out) theta_out[o + c] = acc[q][c];
-              if (tanh_out) tanh_out[o + c] = t[c];
+            if (m0 + MC * c < nh) {
+              if (theta_out) theta_out[o + MC * c] = acc[q][c];
+              if (tanh_out) tanh_out[o + MC * c] = tanhx(acc[q][c]);
             }
-        }
-        if (logpsi_out) {
+        } else if (m0 < nh) {                                  // 16-byte vectors of 4 units
+          if (theta_out) *reinterpret_cast<float4*>(theta_out + o) = *reinterpret_cast<const float4*>(acc[q]);
+          if (tanh_out) {
+            T t[4];
 #pragma unroll
-          for (int c = 0; c < 4; ++c)
-            if (m0 + c < nh) lsum[q] = addx(lsum[q], log_cosh(acc[q][c]));
+            for (int c = 0; c < 4; ++c) t[c] = tanhx(acc[q][c]);
+            *reinterpret_cast<float4*>(tanh_out + o) = *reinterpret_cast<const float4*>(t);
+          }
+        }
+        if constexpr (LP) {
+          if (logpsi_out) {
+            const bool odd = (u0 / FWD_U) & 1;
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+              if (m0 + MC * c < nh) {
+                const T l = log_cosh(acc[q][c]);
+                if (odd) lsum[q][1][c] = addx(lsum[q][1][c], l);
+                else lsum[q][0][c] = addx(lsum[q][0][c], l);
+              }
+          }
         }
       }
     }
   }
-  if (!logpsi_out) return;
+  if constexpr (LP) {
+    if (!logpsi_out) return;
 #pragma unroll
-  for (int q = 0; q < RS; ++q) {
-    const int64_t s = s0 + RS * row + q;
-    T v = lsum[q];
-    if (s < n_samples) {
-      const uint32_t* w = bits + s * nw;
-      for (int i = lane; i < ns; i += 32) v = fma_sign(sigma_of(w, i), a[i], v);
+    for (int q = 0; q < RS; ++q) {
+      const int64_t s = s0 + RS * row + q;
+      T v = ScalarTraits<T>::zero();
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        T x[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          x[c] = lsum[q][h][c];
+          if (s < n_samples)
+            for (int i = 128 * h + (CPLX ? lane + 32 * c : 4 * lane + c); i < ns; i += 256)
+              x[c] = fma_sign(sigma_of(bits + s * nw, i), a[i], x[c]);
+#pragma unroll
+          for (int o = CPLX ? 16 : 4; o > 0; o >>= 1) x[c] = addx(x[c], shfl_xor_val(x[c], o));
+        }
+        if constexpr (CPLX) {                                  // the four sums of 32, in every lane
+#pragma unroll
+          for (int c = 0; c < 4; ++c) v = addx(v, x[c]);
+        } else {                                               // threads 16, 8 and 4 apart above; 2 and 1 apart here
+          const T e = addx(addx(x[0], x[2]), addx(x[1], x[3]));
+#pragma unroll
+          for (int g = 0; g < 4; ++g) v = addx(v, shfl_val(e, 8 * g));
+        }
+      }
+      if (lane == 0 && s < n_samples) logpsi_out[s] = v;
     }
-    v = warp_sum(v);
-    if (lane == 0 && s < n_samples) logpsi_out[s] = v;
   }
 }
 
-template <class T, int RS, bool VEC>
+template <class T, int RS, bool VEC, bool LP>
 __global__ void __launch_bounds__(FWD_THREADS, 2) rbm_forward_kernel(
     int ns, int nh, int64_t n_samples, const uint32_t* __restrict__ bits, const T* __restrict__ a,
     const T* __restrict__ b, const T* __restrict__ W, T* __restrict__ theta_out, T* __restrict__ tanh_out,
     T* __restrict__ logpsi_out) {
   extern __shared__ __align__(16) uint8_t fwd_sm[];
-  rbm_forward_block<T, RS, VEC>(fwd_sm, (int64_t)blockIdx.x * FWD_TY * RS, ns, nh, n_samples, bits, a, b, W, theta_out,
+  rbm_forward_block<T, RS, VEC, LP>(fwd_sm, (int64_t)blockIdx.x * FWD_TY * RS, ns, nh, n_samples, bits, a, b, W, theta_out,
                                 tanh_out, logpsi_out);
 }
 
-template <class T, int RS>
+template <class T, int RS, bool LP>
 static int launch_forward_rs(int ns, int nh, int64_t n, const uint32_t* bits, const T* a, const T* b, const T* W,
                              T* theta_out, T* tanh_out, T* logpsi_out, cudaStream_t st) {
   const unsigned grid = (unsigned)((n + FWD_TY * RS - 1) / (FWD_TY * RS));
   const bool vec = nh % (16 / (int)sizeof(T)) == 0 && (reinterpret_cast<uintptr_t>(W) & 15) == 0;
-  auto kern = vec ? rbm_forward_kernel<T, RS, true> : rbm_forward_kernel<T, RS, false>;
+  auto kern = vec ? rbm_forward_kernel<T, RS, true, LP> : rbm_forward_kernel<T, RS, false, LP>;
   constexpr int smem = fwd_smem<T, RS>();
   QES_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   kern<<<grid, FWD_THREADS, smem, st>>>(ns, nh, n, bits, a, b, W, theta_out, tanh_out, logpsi_out);
@@ -440,16 +477,26 @@ static int launch_forward_rs(int ns, int nh, int64_t n, const uint32_t* bits, co
   return QES_OK;
 }
 
-// samples per thread: the most that leave a block for every SM, down to one
+// samples per thread: the most that leave a block for every SM, down to one; half as many at most with log psi,
+// whose eight sums per sample live in registers
 template <class T>
 static int launch_forward(int ns, int nh, int64_t n, const uint32_t* bits, const T* a, const T* b, const T* W,
                           T* theta_out, T* tanh_out, T* logpsi_out, cudaStream_t st) {
+  constexpr int MAX = ScalarTraits<T>::is_complex ? 4 : 8;
   auto blocks = [&](int rs) { return (n + FWD_TY * rs - 1) / (FWD_TY * rs); };
-  if constexpr (!ScalarTraits<T>::is_complex)
-    if (blocks(8) >= 148) return launch_forward_rs<T, 8>(ns, nh, n, bits, a, b, W, theta_out, tanh_out, logpsi_out, st);
-  if (blocks(4) >= 148) return launch_forward_rs<T, 4>(ns, nh, n, bits, a, b, W, theta_out, tanh_out, logpsi_out, st);
-  if (blocks(2) >= 148) return launch_forward_rs<T, 2>(ns, nh, n, bits, a, b, W, theta_out, tanh_out, logpsi_out, st);
-  return launch_forward_rs<T, 1>(ns, nh, n, bits, a, b, W, theta_out, tanh_out, logpsi_out, st);
+#define QES_FWD(RS, LP) launch_forward_rs<T, RS, LP>(ns, nh, n, bits, a, b, W, theta_out, tanh_out, logpsi_out, st)
+  if (logpsi_out) {
+    if (blocks(MAX / 2) >= 148) return QES_FWD(MAX / 2, true);
+    if constexpr (MAX / 2 > 2)
+      if (blocks(2) >= 148) return QES_FWD(2, true);
+    return QES_FWD(1, true);
+  }
+  if (blocks(MAX) >= 148) return QES_FWD(MAX, false);
+  if constexpr (MAX > 4)
+    if (blocks(4) >= 148) return QES_FWD(4, false);
+  if (blocks(2) >= 148) return QES_FWD(2, false);
+  return QES_FWD(1, false);
+#undef QES_FWD
 }
 
 extern "C" int qes_rbm_forward(int dtype, int ns, int nh, int64_t n_samples, const uint32_t* bits, const void* a,
@@ -641,7 +688,7 @@ __global__ void __launch_bounds__(FWD_THREADS) batch_forward_kernel(const qes_ba
   const T* W = b + I.nh;
   const int64_t rows = (int64_t)I.n_chains * I.num_samples;
   extern __shared__ __align__(16) uint8_t fwd_sm[];
-  rbm_forward_block<T, 2, false>(fwd_sm, (int64_t)it.y * FWD_SB, I.ns, I.nh, rows, bits + I.sample_word_off, a, b, W,
+  rbm_forward_block<T, 2, false, true>(fwd_sm, (int64_t)it.y * FWD_SB, I.ns, I.nh, rows, bits + I.sample_word_off, a, b, W,
                        nullptr, tanh_out ? tanh_out + I.tanh_off : nullptr,
                        logpsi_out ? logpsi_out + I.sample_off : nullptr);
 }
