@@ -462,6 +462,14 @@ int qes_rbm_forward_tc(int dtype, int ns, int nh, int64_t n_samples, const uint3
                        const void* a, const void* b, const void* W, void* theta_out,
                        void* tanh_out, void* logpsi_out, void* workspace, size_t workspace_bytes,
                        void* stream);
+/* The same without waiting for the device: the status word (int, 0 = good,
+ * else QES_ERR_TIMEOUT's outputs must not be used) is left at
+ * workspace + *status_offset, for the caller to read once the stream has
+ * passed.  The workspace belongs to the call until then.                    */
+int qes_rbm_forward_tc_nowait(int dtype, int ns, int nh, int64_t n_samples, const uint32_t* bits,
+                              const void* a, const void* b, const void* W, void* theta_out,
+                              void* tanh_out, void* logpsi_out, void* workspace, size_t workspace_bytes,
+                              size_t* status_offset, void* stream);
 /* Keep the tensor-core operand tiles resident in L2 across CG iterations
  * through a persisting access-policy window on the solve's streams (1; the
  * window and the persisting lines are released after each solve) or not (0,

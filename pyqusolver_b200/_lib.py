@@ -137,6 +137,8 @@ SIGNATURES = {
     "qes_sr_set_barrier_test": [C.c_uint, C.c_uint],
     "qes_rbm_forward_tc_workspace_bytes": [C.c_int, C.c_int, C.c_int, _i64, C.POINTER(_sz)],
     "qes_rbm_forward_tc": [C.c_int, C.c_int, C.c_int, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _sz, _vp],
+    "qes_rbm_forward_tc_nowait": [C.c_int, C.c_int, C.c_int, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _sz,
+                                  C.POINTER(_sz), _vp],
     "qes_set_l2_persist": [C.c_int],
     "qes_profile_enable": [C.c_int],
     "qes_profile_read": [C.c_int, C.POINTER(C.c_double), C.POINTER(C.c_longlong), C.c_int],

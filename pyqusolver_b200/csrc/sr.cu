@@ -1774,13 +1774,8 @@ static int sr_prepare(int dtype, int64_t n_samples, const uint32_t* bits, const 
   return tc_prepare_step(dtype, L.td, n_samples, bits, tt, L.tw, st);
 }
 
-// Reads the tensor-core status word and, inside a CG solve (cg_words: counter[4] was zeroed at the
-// start of the solve), the grid-barrier error word of the fused CG kernel; synchronises the stream.
-static int sr_check_status(const SRWork& L, cudaStream_t st, bool cg_words) {
-  int h[2] = {0, 0};
-  if (L.tc) QES_CUDA_CHECK(cudaMemcpyAsync(&h[0], L.tw.status, sizeof(int), cudaMemcpyDeviceToHost, st));
-  if (cg_words) QES_CUDA_CHECK(cudaMemcpyAsync(&h[1], L.counter + 4, sizeof(int), cudaMemcpyDeviceToHost, st));
-  QES_CUDA_CHECK(cudaStreamSynchronize(st));
+// tensor-core status word, grid-barrier error word -> return code
+static int sr_status_code(const int (&h)[2]) {
   if (h[0] != 0) {
     qes_set_last_message("SR tensor-core matvec: a bounded device wait gave up");
     return QES_ERR_TIMEOUT;
@@ -1790,6 +1785,16 @@ static int sr_check_status(const SRWork& L, cudaStream_t st, bool cg_words) {
     return QES_ERR_TIMEOUT;
   }
   return QES_OK;
+}
+
+// Reads the tensor-core status word and, inside a CG solve (cg_words: counter[4] was zeroed at the
+// start of the solve), the grid-barrier error word of the fused CG kernel; synchronises the stream.
+static int sr_check_status(const SRWork& L, cudaStream_t st, bool cg_words) {
+  int h[2] = {0, 0};
+  if (L.tc) QES_CUDA_CHECK(cudaMemcpyAsync(&h[0], L.tw.status, sizeof(int), cudaMemcpyDeviceToHost, st));
+  if (cg_words) QES_CUDA_CHECK(cudaMemcpyAsync(&h[1], L.counter + 4, sizeof(int), cudaMemcpyDeviceToHost, st));
+  QES_CUDA_CHECK(cudaStreamSynchronize(st));
+  return sr_status_code(h);
 }
 
 extern "C" int qes_sr_matvec_weighted(int dtype, int ns, int nh, int64_t n_samples, const uint32_t* bits,
@@ -2022,9 +2027,15 @@ static int sr_cg_persistent_t(int ns, int nh, int64_t n_samples, const uint32_t*
                   L.x, L.b, x_out, L.scal, L.partial, L.pvz, L.slots, L.tw.status, (int*)(L.counter + 4)};
   int rc = pcg_solve(dtype, L.pd, n_samples, a, st);
   if (rc) return rc;
+  // the scalars and both status words in one read (they are free of use at [14]): each read waits for the device
   double hs[16] = {0}, true_rr = -1.0;
+  QES_CUDA_CHECK(cudaMemcpyAsync(L.scal + 14, L.tw.status, sizeof(int), cudaMemcpyDeviceToDevice, st));
+  QES_CUDA_CHECK(cudaMemcpyAsync((int*)(L.scal + 14) + 1, L.counter + 4, sizeof(int), cudaMemcpyDeviceToDevice, st));
   QES_CUDA_CHECK(cudaMemcpyAsync(hs, L.scal, 16 * sizeof(double), cudaMemcpyDeviceToHost, st));
-  if ((rc = sr_check_status(L, st, true))) return rc;      // synchronises the stream
+  QES_CUDA_CHECK(cudaStreamSynchronize(st));
+  int words[2];
+  std::memcpy(words, &hs[14], sizeof(words));
+  if ((rc = sr_status_code(words))) return rc;
   if (opt->maxiter > 0 && !opt->skip_true_residual) {
     if ((rc = sr_prepare(dtype, n_samples, bits, tt, L, st))) return rc;
     if ((rc = sr_matvec_t<T>(ns, nh, n_samples, bits, tt, opt->shift, (const V*)L.x, (V*)L.Ap, nullptr, L, st, false)))

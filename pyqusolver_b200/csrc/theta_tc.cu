@@ -278,7 +278,7 @@ extern "C" int qes_rbm_forward_tc_workspace_bytes(int dtype, int ns, int nh, int
 
 template <class T>
 static int forward_tc_t(const ThetaDims& d, int64_t n, const uint32_t* bits, const T* a, const T* b, const T* W,
-                        T* theta_out, T* tanh_out, T* logpsi_out, char* ws, cudaStream_t st) {
+                        T* theta_out, T* tanh_out, T* logpsi_out, char* ws, cudaStream_t st, bool wait) {
   size_t ow, ol, os;
   theta_ws(d, n, sizeof(T), &ow, &ol, &os);
   uint16_t* sig = reinterpret_cast<uint16_t*>(ws);
@@ -296,6 +296,7 @@ static int forward_tc_t(const ThetaDims& d, int64_t n, const uint32_t* bits, con
     theta_logpsi_kernel<T><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(d.ns, d.nnc, n, bits, a, lsum, logpsi_out);
     QES_LAUNCH_CHECK();
   }
+  if (!wait) return QES_OK;                                   // the caller reads the word
   int h = 0;
   QES_CUDA_CHECK(cudaMemcpyAsync(&h, status, sizeof(int), cudaMemcpyDeviceToHost, st));
   QES_CUDA_CHECK(cudaStreamSynchronize(st));
@@ -306,9 +307,9 @@ static int forward_tc_t(const ThetaDims& d, int64_t n, const uint32_t* bits, con
   return QES_OK;
 }
 
-extern "C" int qes_rbm_forward_tc(int dtype, int ns, int nh, int64_t n_samples, const uint32_t* bits, const void* a,
-                                  const void* b, const void* W, void* theta_out, void* tanh_out, void* logpsi_out,
-                                  void* workspace, size_t workspace_bytes, void* stream) {
+static int forward_tc(int dtype, int ns, int nh, int64_t n_samples, const uint32_t* bits, const void* a, const void* b,
+                      const void* W, void* theta_out, void* tanh_out, void* logpsi_out, void* workspace,
+                      size_t workspace_bytes, void* stream, size_t* status_offset) {
   QES_ARG_CHECK(ns > 0 && nh > 0 && n_samples >= 0, "qes_rbm_forward_tc: bad sizes");
   QES_ARG_CHECK(dtype == QES_DTYPE_F32 || dtype == QES_DTYPE_C64, "qes_rbm_forward_tc: bad dtype");
   if (n_samples == 0) return QES_OK;
@@ -318,15 +319,32 @@ extern "C" int qes_rbm_forward_tc(int dtype, int ns, int nh, int64_t n_samples, 
     qes_set_last_message("qes_rbm_forward_tc: shapes outside the tensor-core forward's limits");
     return QES_ERR_SIZE;
   }
-  size_t x, y, z;
+  size_t x, y, z = 0;
   if (workspace_bytes < theta_ws(d, n_samples, dtype == QES_DTYPE_C64 ? 8 : 4, &x, &y, &z)) {
     qes_set_last_message("qes_rbm_forward_tc: workspace too small");
     return QES_ERR_WORKSPACE;
   }
+  if (status_offset) *status_offset = z;
   cudaStream_t st = (cudaStream_t)stream;
   if (dtype == QES_DTYPE_F32)
     return forward_tc_t<float>(d, n_samples, bits, (const float*)a, (const float*)b, (const float*)W,
-                               (float*)theta_out, (float*)tanh_out, (float*)logpsi_out, (char*)workspace, st);
+                               (float*)theta_out, (float*)tanh_out, (float*)logpsi_out, (char*)workspace, st, status_offset == nullptr);
   return forward_tc_t<float2>(d, n_samples, bits, (const float2*)a, (const float2*)b, (const float2*)W,
-                              (float2*)theta_out, (float2*)tanh_out, (float2*)logpsi_out, (char*)workspace, st);
+                              (float2*)theta_out, (float2*)tanh_out, (float2*)logpsi_out, (char*)workspace, st, status_offset == nullptr);
+}
+
+extern "C" int qes_rbm_forward_tc(int dtype, int ns, int nh, int64_t n_samples, const uint32_t* bits, const void* a,
+                                  const void* b, const void* W, void* theta_out, void* tanh_out, void* logpsi_out,
+                                  void* workspace, size_t workspace_bytes, void* stream) {
+  return forward_tc(dtype, ns, nh, n_samples, bits, a, b, W, theta_out, tanh_out, logpsi_out, workspace, workspace_bytes,
+                    stream, nullptr);
+}
+
+extern "C" int qes_rbm_forward_tc_nowait(int dtype, int ns, int nh, int64_t n_samples, const uint32_t* bits,
+                                         const void* a, const void* b, const void* W, void* theta_out, void* tanh_out,
+                                         void* logpsi_out, void* workspace, size_t workspace_bytes,
+                                         size_t* status_offset, void* stream) {
+  QES_ARG_CHECK(status_offset && n_samples > 0, "qes_rbm_forward_tc_nowait: bad args");
+  return forward_tc(dtype, ns, nh, n_samples, bits, a, b, W, theta_out, tanh_out, logpsi_out, workspace, workspace_bytes,
+                    stream, status_offset);
 }

@@ -135,6 +135,29 @@ def rbm_forward_step(flat_params, ns, nh, bits, theta=False, tanh=True, logpsi=T
     return rbm_forward(flat_params, ns, nh, bits, theta=theta, tanh=tanh, logpsi=logpsi, tensor_cores=tc)
 
 
+def rbm_tanh_nowait(flat_params, ns, nh, bits):
+    """tanh(theta) as rbm_forward_step gives it, without waiting for the device, and the status word of its
+    bounded waits (int32 device tensor of one entry, for ``check_forward_status``; None on the CUDA cores).
+    The workspace is the call's own: another thread or stream may run a forward meanwhile."""
+    n = int(bits.shape[0])
+    if not forward_uses_tensor_cores(flat_params, ns, nh, n):
+        return rbm_forward(flat_params, ns, nh, bits, theta=False, tanh=True, logpsi=False)[1], None
+    a, b, W = split_params(flat_params, ns, nh)
+    tn = torch.empty((n, nh), dtype=flat_params.dtype, device=flat_params.device)
+    nb, off = C.c_size_t(0), C.c_size_t(0)
+    call("qes_rbm_forward_tc_workspace_bytes", dtype_code(flat_params), ns, nh, n, C.byref(nb))
+    ws = torch.empty((int(nb.value),), dtype=torch.uint8, device=flat_params.device)
+    call("qes_rbm_forward_tc_nowait", dtype_code(flat_params), ns, nh, n, ptr(bits), ptr(a), ptr(b), ptr(W), None,
+         ptr(tn), None, ptr(ws), int(ws.numel()), C.byref(off), stream_ptr())
+    return tn, ws[off.value:off.value + 4].view(torch.int32)
+
+
+def check_forward_status(word):
+    """Raises what qes_rbm_forward_tc returns for this status word (a host number)."""
+    if word:
+        raise _lib.QESError(_lib.QES_ERR_TIMEOUT, "qes_rbm_forward_tc: a bounded device wait gave up")
+
+
 def log_derivatives(flat_params, ns, nh, bits, tanh_theta, out=None):
     n = int(bits.shape[0])
     P = n_params(ns, nh)

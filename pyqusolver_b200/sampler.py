@@ -86,6 +86,7 @@ class VMCSampler:
             raise ValueError(f"initial state {initstate!r} is not supported")
         self._tables = None
         self._tables_version = -1
+        self._flip_moves = None                                 # (sites, kinds) of the single-flip tables
         self._pt_betas = None
         self._n_replicas = 1
         self._pt_round = 0
@@ -228,8 +229,10 @@ class VMCSampler:
         if self._tables is not None and self._tables_version == net.version:
             return self._tables
         if self._rule == _lib.RULE_LOCAL:
-            sites = torch.arange(net.ns, dtype=torch.int32, device=net.device)
-            kinds = torch.full((net.ns,), _lib.MOVE_FLIP1, dtype=torch.int32, device=net.device)
+            if self._flip_moves is None:
+                self._flip_moves = (torch.arange(net.ns, dtype=torch.int32, device=net.device),
+                                    torch.full((net.ns,), _lib.MOVE_FLIP1, dtype=torch.int32, device=net.device))
+            sites, kinds = self._flip_moves
             fC, fS, _ = dv.move_tables(net.flat, net.ns, net.nh, sites, sites, kinds, move_major=True)
             self._tables = ((fC, fS), None)
         else:

@@ -6,8 +6,9 @@ import torch
 
 from oracle import lattice as olat, hamiltonian as oH, rbm as orbm, estimator as oest
 import pyqusolver_b200 as qb
-from pyqusolver_b200 import device as dv
+from pyqusolver_b200 import _lib, device as dv
 from pyqusolver_b200.rbm import RBM
+from pyqusolver_b200.tdvp import TDVP
 
 pytestmark = pytest.mark.gpu
 
@@ -81,3 +82,27 @@ def test_log_derivative_rows(cplx, ns, nh, n):
     wide = torch.full((n, dv.n_params(ns, nh) + 3), 7.0, dtype=tn.dtype, device="cuda")       # rows of a wider array
     dv.log_derivatives(net.flat, ns, nh, bits, tn, out=wide)
     assert torch.equal(wide[:, :-3], ref) and bool((wide[:, -3:] == 7.0).all())
+
+
+@pytest.mark.parametrize("dtype,ns,nh,n", [("float32", 5, 3, 1), ("float32", 63, 126, 700), ("complex64", 33, 40, 129)])
+def test_forward_without_wait_is_the_forward(dtype, ns, nh, n):
+    net = RBM((ns,), n_hidden=nh, dtype=dtype, seed=ns, init_scale=0.1)
+    bits = dv.pack_states(np.where(np.random.default_rng(nh).random((n, ns)) < 0.5, 0.5, -0.5))
+    tn, status = dv.rbm_tanh_nowait(net.flat, ns, nh, bits)
+    _, ref, _ = dv.rbm_forward_step(net.flat, ns, nh, bits, theta=False, tanh=True, logpsi=False)
+    assert torch.equal(tn, ref)
+    assert status is None or int(status.item()) == 0
+
+
+def test_a_failed_forward_updates_nothing(monkeypatch):
+    model = qb.TransverseFieldIsing(qb.SquareLattice(1, 8), j=1.0, hx=1.0, hz=0.0)
+    nqs = qb.NQS("rbm", model, alpha=1.0, dtype="float32", seed=1, s_numchains=64, s_numsamples=4)
+    tdvp = TDVP(rhs_prefactor=-1.0, sr_diag_shift=1e-2)
+    nqs.train_step(lr=0.01, tdvp=tdvp)
+    weights, solution = nqs.net.flat.clone(), tdvp._solution
+    real = dv.rbm_tanh_nowait
+    monkeypatch.setattr(dv, "rbm_tanh_nowait", lambda *a: (real(*a)[0], torch.ones(1, dtype=torch.int32, device="cuda")))
+    with pytest.raises(_lib.QESError) as err:
+        nqs.train_step(lr=0.01, tdvp=tdvp)
+    assert err.value.code == _lib.QES_ERR_TIMEOUT
+    assert torch.equal(nqs.net.flat, weights) and tdvp._solution is solution
