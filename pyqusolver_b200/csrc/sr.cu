@@ -2850,9 +2850,27 @@ extern "C" int qes_sr_solve_minsr(int dtype, int ns, int nh, int64_t n_samples, 
 // vector-Jacobian product of log psi:  grad = O^H g  (no centring, no 1/Ns)
 // ----------------------------------------------------------------------------
 template <class T>
+static int launch_vjp_mma(int ns, int nh, int64_t n_samples, const uint32_t* bits, const T* tt, const float2* g, T* partial,
+                          cudaStream_t st);
+constexpr int VJP_MAX_NS = 512;
+
+// Up to VJP_MAX_NS sites (the spin words and the sums of g_a of a block's 512 samples in shared memory) on the tensor cores at
+// float32 precision (vjp_mma_kernel); the float64 form, the CUDA-core form where it is asked for and longer rows
+// on the CUDA cores.  16,384 samples of 100 sites x 200 complex units with the
+// sum over the splits: 49 us against 161; error against 64 bits 1.8e-7 against 4.0e-7 (5 to 400 sites).
+template <class T>
 static int vjp_t(int ns, int nh, int64_t n_samples, const uint32_t* bits, const T* tt, const float2* g,
                  typename VecT<T>::type* out, const SRWork& L, cudaStream_t st) {
   using V = typename VecT<T>::type;
+  const int64_t nsplit = (n_samples + PT_SPLIT - 1) / PT_SPLIT;
+  if (!L.fp64 && g_sr_impl.load() != 1 && ns <= VJP_MAX_NS && nh <= 65536 && nsplit <= 65535) {
+    const int64_t P = (int64_t)ns + nh + (int64_t)ns * nh;
+    if (int rc = launch_vjp_mma<T>(ns, nh, n_samples, bits, tt, g, (T*)L.partial, st)) return rc;
+    if (int rc = launch_reduce_splits<T, V>(P, (int)nsplit, L.partial, 0.0, nullptr, out, nullptr, nullptr, L.counter, st))
+      return rc;
+    QES_LAUNCH_CHECK();
+    return QES_OK;
+  }
   return apply_ohu<T, V>(ns, nh, n_samples, bits, tt, g, nullptr, 1.0, L, 0.0, nullptr, out, nullptr, st);
 }
 
@@ -3126,6 +3144,134 @@ __global__ void __launch_bounds__(BMM_THREADS, 2) batch_ov_mma_kernel(const qes_
   }
 }
 
+// O^H u of unit group gi (16, complex 8, units) and the sites from mb (up to 64), steps [k0, k1) of 16 samples, by one warp:
+// us the samples' u (zero past nc), ws their spin words, tb their rows of T.  sum: D fragments; gb: sum_s q of unit g of
+// either B tile (complex: Re and Im)
+template <class T>
+QES_D void ohu_mma_sites(int ns, int nh, int nw, int nc, int gi, int mb, int k0, int k1, const T* __restrict__ tb,
+                         const T* us, const uint32_t* ws, float (&sum)[4][2][4], float (&gb)[2]) {
+  constexpr int NP = bparts<T>(), NU = 2 / NP, UG = 16 / NP;  // unit tiles and units of a group: two B tiles
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, MT = min(4, (ns - mb + 15) / 16);
+#pragma unroll
+  for (int mt = 0; mt < 4; ++mt)
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int x = 0; x < 4; ++x) sum[mt][j][x] = 0.f;
+  gb[0] = gb[1] = 0.f;
+  T tv[NU][4];
+  auto fetch = [&](int ks) {
+#pragma unroll
+    for (int j = 0; j < NU; ++j) {
+      const int m = gi * UG + 8 * j + g;
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        const int sl = 16 * ks + 4 * t + x;
+        tv[j][x] = (ks < k1 && sl < nc && m < nh) ? tb[(int64_t)sl * nh + m] : ScalarTraits<T>::zero();
+      }
+    }
+  };
+  fetch(k0);
+  for (int kc = k0; kc < k1; kc += 4) {
+    float d[4][2][4];
+#pragma unroll
+    for (int mt = 0; mt < 4; ++mt)
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int x = 0; x < 4; ++x) d[mt][j][x] = 0.f;
+#pragma unroll 1
+    for (int ks = kc; ks < min(k1, kc + 4); ++ks) {
+      uint2 B[2][3];
+#pragma unroll
+      for (int j = 0; j < NU; ++j) {
+        T q[4];
+#pragma unroll
+        for (int x = 0; x < 4; ++x) q[x] = mulx(conjx(tv[j][x]), us[16 * ks + 4 * t + x]);
+#pragma unroll
+        for (int c = 0; c < NP; ++c) {
+          uint32_t lo[3], hi[3];
+          const float q0 = part_of(q[0], c), q1 = part_of(q[1], c), q2 = part_of(q[2], c), q3 = part_of(q[3], c);
+          gb[j * NP + c] += (q0 + q1) + (q2 + q3);
+          split3(q0, q1, lo);
+          split3(q2, q3, hi);
+#pragma unroll
+          for (int k = 0; k < 3; ++k) B[j * NP + c][k] = make_uint2(lo[k], hi[k]);
+        }
+      }
+      fetch(ks + 1);
+#pragma unroll
+      for (int wd = 0; wd < 2; ++wd) {
+        if (2 * wd >= MT) break;
+        uint32_t y[4];                                  // this lane's four samples, site g of each byte on top
+#pragma unroll
+        for (int x = 0; x < 4; ++x) y[x] = ws[(16 * ks + 4 * t + x) * nw + (mb >> 5) + wd] << (7 - g);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          if (2 * wd + h >= MT) break;
+          uint32_t A[4];
+          if (h == 0) {
+            A[0] = sign_pair<0, 0>(y[0], y[1]); A[1] = sign_pair<1, 1>(y[0], y[1]);
+            A[2] = sign_pair<0, 0>(y[2], y[3]); A[3] = sign_pair<1, 1>(y[2], y[3]);
+          } else {
+            A[0] = sign_pair<2, 2>(y[0], y[1]); A[1] = sign_pair<3, 3>(y[0], y[1]);
+            A[2] = sign_pair<2, 2>(y[2], y[3]); A[3] = sign_pair<3, 3>(y[2], y[3]);
+          }
+#pragma unroll
+          for (int k = 2; k >= 0; --k)                  // small parts first
+#pragma unroll
+            for (int j = 0; j < 2; ++j) mma16816(d[2 * wd + h][j], A, B[j][k]);
+        }
+      }
+    }
+#pragma unroll
+    for (int mt = 0; mt < 4; ++mt)
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int x = 0; x < 4; ++x) sum[mt][j][x] += d[mt][j][x];
+  }
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    gb[j] += __shfl_xor_sync(0xffffffffu, gb[j], 1);
+    gb[j] += __shfl_xor_sync(0xffffffffu, gb[j], 2);
+  }
+}
+template <class T>
+QES_D void ohu_mma_store(int ns, int nh, int gi, int mb, const float (&sum)[4][2][4], const float (&gb)[2],
+                         T* __restrict__ out) {
+  constexpr bool CPLX = ScalarTraits<T>::is_complex;
+  constexpr int NP = bparts<T>(), NU = 2 / NP, UG = 16 / NP;
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+#pragma unroll
+  for (int mt = 0; mt < 4; ++mt)
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+      for (int j = 0; j < NU; ++j)
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+          const int i = mb + 16 * mt + 8 * r + g, m = gi * UG + 8 * j + 2 * t + x;
+          if (i < ns && m < nh) {
+            T v;
+            if constexpr (CPLX) v = make_float2(sum[mt][0][2 * r + x], sum[mt][1][2 * r + x]);
+            else v = sum[mt][j][2 * r + x];
+            out[ns + nh + (int64_t)i * nh + m] = v;
+          }
+        }
+  if (mb == 0 && t == 0)
+#pragma unroll
+    for (int j = 0; j < NU; ++j) {
+      const int m = gi * UG + 8 * j + g;
+      if (m < nh) {
+        T v;
+        if constexpr (CPLX) v = make_float2(gb[0], gb[1]);
+        else v = gb[j];
+        out[ns + m] = v;
+      }
+    }
+}
+
 // O^H u: a warp takes 16 (complex: 8) hidden units and up to 64 sites at a time (further sites take passes), all samples
 // of the split or, where the problem has few units, a part of them (parts added in a fixed order).  Each q_sm is
 // made by the one lane whose fragment holds it, straight from T in global memory, one step of 16 samples ahead.  The
@@ -3150,7 +3296,7 @@ __global__ void __launch_bounds__(BMM_THREADS, 2) batch_ohu_mma_kernel(const qes
                                                                        T* __restrict__ partial) {
   extern __shared__ __align__(16) uint8_t boh_sm[];
   constexpr bool CPLX = ScalarTraits<T>::is_complex;
-  constexpr int NP = bparts<T>(), NU = 2 / NP, UG = 16 / NP;  // unit tiles and units of a group: two B tiles
+  constexpr int NP = bparts<T>();
   __shared__ double mred[BMM_WARPS];
   const int4 it = items[blockIdx.x];
   const double* sc = bscal + (int64_t)it.x * BSC;
@@ -3165,7 +3311,7 @@ __global__ void __launch_bounds__(BMM_THREADS, 2) batch_ohu_mma_kernel(const qes
   uint32_t* ws = reinterpret_cast<uint32_t*>(us + OHU_SPLIT_SAMPLES);          // [256][nw]
   T* ga = reinterpret_cast<T*>(boh_sm + bsmall_align16((int64_t)OHU_SPLIT_SAMPLES * (sizeof(T) + 4 * nw)));   // [warps][ns]
   float* red = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(ga) + bsmall_align16((int64_t)BMM_WARPS * ns * sizeof(T)));
-  const int tid = threadIdx.x, lane = tid & 31, wv = tid >> 5, g = lane >> 2, t = lane & 3;
+  const int tid = threadIdx.x, lane = tid & 31, wv = tid >> 5;
   const uint32_t* bw = bits + I.sample_word_off + sbeg * nw;
   const T* tb = tt + I.tanh_off + sbeg * nh;
   const float2* wb = w + I.sample_off;
@@ -3202,92 +3348,9 @@ __global__ void __launch_bounds__(BMM_THREADS, 2) batch_ohu_mma_kernel(const qes
   const int k0 = min(nk, part * per), k1 = min(nk, k0 + per);
   for (int gi = ng >= BMM_WARPS ? wv : wv % ng; gi < ng; gi += ng >= BMM_WARPS ? BMM_WARPS : ng) {
     for (int mb = 0; mb < ns; mb += 64) {
-      const int MT = min(4, (ns - mb + 15) / 16);
-      float sum[4][2][4], gb[2] = {0.f, 0.f};
-#pragma unroll
-      for (int mt = 0; mt < 4; ++mt)
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-#pragma unroll
-          for (int x = 0; x < 4; ++x) sum[mt][j][x] = 0.f;
+      float sum[4][2][4], gb[2];
       if (warp_on) {
-        T tv[NU][4];
-        auto fetch = [&](int ks) {
-#pragma unroll
-          for (int j = 0; j < NU; ++j) {
-            const int m = gi * UG + 8 * j + g;
-#pragma unroll
-            for (int x = 0; x < 4; ++x) {
-              const int sl = 16 * ks + 4 * t + x;
-              tv[j][x] = (ks < k1 && sl < nc && m < nh) ? tb[(int64_t)sl * nh + m] : ScalarTraits<T>::zero();
-            }
-          }
-        };
-        fetch(k0);
-        for (int kc = k0; kc < k1; kc += 4) {
-          float d[4][2][4];
-#pragma unroll
-          for (int mt = 0; mt < 4; ++mt)
-#pragma unroll
-            for (int j = 0; j < 2; ++j)
-#pragma unroll
-              for (int x = 0; x < 4; ++x) d[mt][j][x] = 0.f;
-#pragma unroll 1
-          for (int ks = kc; ks < min(k1, kc + 4); ++ks) {
-            uint2 B[2][3];
-#pragma unroll
-            for (int j = 0; j < NU; ++j) {
-              T q[4];
-#pragma unroll
-              for (int x = 0; x < 4; ++x) q[x] = mulx(conjx(tv[j][x]), us[16 * ks + 4 * t + x]);
-#pragma unroll
-              for (int c = 0; c < NP; ++c) {
-                uint32_t lo[3], hi[3];
-                const float q0 = part_of(q[0], c), q1 = part_of(q[1], c), q2 = part_of(q[2], c), q3 = part_of(q[3], c);
-                gb[j * NP + c] += (q0 + q1) + (q2 + q3);
-                split3(q0, q1, lo);
-                split3(q2, q3, hi);
-#pragma unroll
-                for (int k = 0; k < 3; ++k) B[j * NP + c][k] = make_uint2(lo[k], hi[k]);
-              }
-            }
-            fetch(ks + 1);
-#pragma unroll
-            for (int wd = 0; wd < 2; ++wd) {
-              if (2 * wd >= MT) break;
-              uint32_t y[4];                                  // this lane's four samples, site g of each byte on top
-#pragma unroll
-              for (int x = 0; x < 4; ++x) y[x] = ws[(16 * ks + 4 * t + x) * nw + (mb >> 5) + wd] << (7 - g);
-#pragma unroll
-              for (int h = 0; h < 2; ++h) {
-                if (2 * wd + h >= MT) break;
-                uint32_t A[4];
-                if (h == 0) {
-                  A[0] = sign_pair<0, 0>(y[0], y[1]); A[1] = sign_pair<1, 1>(y[0], y[1]);
-                  A[2] = sign_pair<0, 0>(y[2], y[3]); A[3] = sign_pair<1, 1>(y[2], y[3]);
-                } else {
-                  A[0] = sign_pair<2, 2>(y[0], y[1]); A[1] = sign_pair<3, 3>(y[0], y[1]);
-                  A[2] = sign_pair<2, 2>(y[2], y[3]); A[3] = sign_pair<3, 3>(y[2], y[3]);
-                }
-#pragma unroll
-                for (int k = 2; k >= 0; --k)                  // small parts first
-#pragma unroll
-                  for (int j = 0; j < 2; ++j) mma16816(d[2 * wd + h][j], A, B[j][k]);
-              }
-            }
-          }
-#pragma unroll
-          for (int mt = 0; mt < 4; ++mt)
-#pragma unroll
-            for (int j = 0; j < 2; ++j)
-#pragma unroll
-              for (int x = 0; x < 4; ++x) sum[mt][j][x] += d[mt][j][x];
-        }
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          gb[j] += __shfl_xor_sync(0xffffffffu, gb[j], 1);
-          gb[j] += __shfl_xor_sync(0xffffffffu, gb[j], 2);
-        }
+        ohu_mma_sites<T>(ns, nh, nw, nc, gi, mb, k0, k1, tb, us, ws, sum, gb);
       }
       if (parts > 1) {
         // parts 1, 2, ... through shared memory, added in order by part 0 (every warp passes here once per mb)
@@ -3310,33 +3373,7 @@ __global__ void __launch_bounds__(BMM_THREADS, 2) batch_ohu_mma_kernel(const qes
           }
       }
       if (part == 0) {
-#pragma unroll
-        for (int mt = 0; mt < 4; ++mt)
-#pragma unroll
-          for (int r = 0; r < 2; ++r)
-#pragma unroll
-            for (int j = 0; j < NU; ++j)
-#pragma unroll
-              for (int x = 0; x < 2; ++x) {
-                const int i = mb + 16 * mt + 8 * r + g, m = gi * UG + 8 * j + 2 * t + x;
-                if (i < ns && m < nh) {
-                  T v;
-                  if constexpr (CPLX) v = make_float2(sum[mt][0][2 * r + x], sum[mt][1][2 * r + x]);
-                  else v = sum[mt][j][2 * r + x];
-                  out[ns + nh + (int64_t)i * nh + m] = v;
-                }
-              }
-        if (mb == 0 && t == 0)
-#pragma unroll
-          for (int j = 0; j < NU; ++j) {
-            const int m = gi * UG + 8 * j + g;
-            if (m < nh) {
-              T v;
-              if constexpr (CPLX) v = make_float2(gb[0], gb[1]);
-              else v = gb[j];
-              out[ns + m] = v;
-            }
-          }
+        ohu_mma_store<T>(ns, nh, gi, mb, sum, gb, out);
       }
     }
   }
@@ -3347,6 +3384,68 @@ __global__ void __launch_bounds__(BMM_THREADS, 2) batch_ohu_mma_kernel(const qes
     for (int q = 1; q < BMM_WARPS; ++q) s = addx(s, ga[q * ns + i]);
     out[i] = s;
   }
+}
+
+// O^H g of one problem (the vector-Jacobian product of log psi): block (z, y) takes the PT_SPLIT samples of split z, its warps
+// the pairs (unit group, 64 sites) 8 y ..; the blocks y = 0 also g_a.  partial: [split][P].
+template <class T>
+__global__ void __launch_bounds__(BMM_THREADS, 2) vjp_mma_kernel(int ns, int nh, int64_t n_samples,
+                                                                 const uint32_t* __restrict__ bits,
+                                                                 const T* __restrict__ tt, const float2* __restrict__ g,
+                                                                 T* __restrict__ partial) {
+  extern __shared__ __align__(16) uint8_t vjp_sm[];
+  const int nw = n_words(ns), tid = threadIdx.x, lane = tid & 31, wv = tid >> 5;
+  const int64_t sbeg = (int64_t)blockIdx.x * PT_SPLIT;
+  const int nc = (int)min((int64_t)PT_SPLIT, n_samples - sbeg);
+  T* us = reinterpret_cast<T*>(vjp_sm);                                        // [PT_SPLIT], zero past nc
+  uint32_t* ws = reinterpret_cast<uint32_t*>(us + PT_SPLIT);                   // [PT_SPLIT][nw]
+  T* ga = reinterpret_cast<T*>(vjp_sm + bsmall_align16((int64_t)PT_SPLIT * (sizeof(T) + 4 * nw)));     // [warps][ns], y = 0
+  const uint32_t* bw = bits + sbeg * nw;
+  for (int e = tid; e < PT_SPLIT * nw; e += BMM_THREADS) ws[e] = e < nc * nw ? bw[e] : 0u;
+  for (int sl = tid; sl < PT_SPLIT; sl += BMM_THREADS) us[sl] = sl < nc ? from_c(g[sbeg + sl], T()) : ScalarTraits<T>::zero();
+  __syncthreads();
+  const int64_t P = (int64_t)ns + nh + (int64_t)ns * nh;
+  T* out = partial + (int64_t)blockIdx.x * P;
+  const int ng = batch_ohu_ng(nh, bparts<T>());
+  const int64_t pair = (int64_t)blockIdx.y * BMM_WARPS + wv;
+  const int gi = (int)(pair % ng), mb = (int)min((int64_t)ns, 64 * (pair / ng));
+  if (mb < ns) {
+    float sum[4][2][4], gb[2];
+    ohu_mma_sites<T>(ns, nh, nw, nc, gi, mb, 0, (nc + 15) / 16, tt + sbeg * nh, us, ws, sum, gb);
+    ohu_mma_store<T>(ns, nh, gi, mb, sum, gb, out);
+  }
+  if (blockIdx.y != 0) return;
+  constexpr int SW = PT_SPLIT / BMM_WARPS;                    // samples per warp; lane = site
+  for (int wd = 0; wd < nw; ++wd) {
+    T s = ScalarTraits<T>::zero();
+#pragma unroll 8
+    for (int sl = SW * wv; sl < SW * wv + SW; ++sl)
+      s = fma_s(((ws[sl * nw + wd] >> lane) & 1u) ? 1.f : -1.f, us[sl], s);
+    if (32 * wd + lane < ns) ga[wv * ns + 32 * wd + lane] = s;
+  }
+  __syncthreads();
+  for (int i = tid; i < ns; i += BMM_THREADS) {
+    T s = ga[i];
+#pragma unroll
+    for (int q = 1; q < BMM_WARPS; ++q) s = addx(s, ga[q * ns + i]);
+    out[i] = s;
+  }
+}
+
+template <class T>
+static int launch_vjp_mma(int ns, int nh, int64_t n_samples, const uint32_t* bits, const T* tt, const float2* g, T* partial,
+                          cudaStream_t st) {
+  const int64_t pairs = (int64_t)batch_ohu_ng(nh, bparts<T>()) * ((ns + 63) / 64);
+  const int64_t gy = (pairs + BMM_WARPS - 1) / BMM_WARPS;
+  const size_t smem = (size_t)bsmall_align16((int64_t)PT_SPLIT * (sizeof(T) + 4 * n_words(ns))) +
+                      (size_t)BMM_WARPS * ns * sizeof(T);
+  QES_CUDA_CHECK(cudaFuncSetAttribute(vjp_mma_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int pf = qes_prof_begin(QES_PROF_OHU, st);
+  vjp_mma_kernel<T><<<dim3((unsigned)((n_samples + PT_SPLIT - 1) / PT_SPLIT), (unsigned)gy), BMM_THREADS, smem, st>>>(
+      ns, nh, n_samples, bits, tt, g, partial);
+  QES_LAUNCH_CHECK();
+  qes_prof_end(pf, st);
+  return QES_OK;
 }
 
 // b = sum of the force partials; x = 0, r = p = b (and p in float32); CG scalars (one block per problem)

@@ -106,3 +106,22 @@ def test_a_failed_forward_updates_nothing(monkeypatch):
         nqs.train_step(lr=0.01, tdvp=tdvp)
     assert err.value.code == _lib.QES_ERR_TIMEOUT
     assert torch.equal(nqs.net.flat, weights) and tdvp._solution is solution
+
+
+# unit groups of 16 (complex 8), 64 sites per pass, 16 samples per step and 512 per split; past 512 sites the CUDA-core form
+@pytest.mark.parametrize("cplx,ns,nh,n", [(False, 1, 1, 1), (True, 1, 1, 17), (False, 64, 16, 512), (True, 65, 9, 513),
+                                          (False, 33, 17, 1030), (True, 512, 8, 40), (False, 513, 3, 40),
+                                          (False, 130, 140, 31)])
+def test_logpsi_vjp_at_tile_edges(cplx, ns, nh, n):
+    net, st, bits, _ = _problem(cplx, ns, nh, n, 0.2)
+    _, tn, _ = dv.rbm_forward(net.flat, ns, nh, bits, tanh=True, logpsi=False)
+    rng = np.random.default_rng(n)
+    g = (rng.standard_normal(n) + 1j * rng.standard_normal(n)).astype(np.complex64)
+    out = dv.logpsi_vjp(net.flat, ns, nh, bits, tn, torch.tensor(g, device="cuda")).cpu().numpy()
+    t, s, u = tn.cpu().numpy().reshape(n, nh), 2.0 * st, g if cplx else g.real
+    t, u = t.astype(np.complex128 if cplx else np.float64), u.astype(np.complex128 if cplx else np.float64)
+    q = t.conj() * u[:, None]
+    ref = np.concatenate([s.T @ u, q.sum(0), (s.T @ q).reshape(-1)])
+    # products rounded once (complex: three times) and float32 sums of 512 terms: a few 2^-24 of the terms' norm, which the
+    # random signs leave as the result's
+    assert np.linalg.norm(out - ref) <= 1e-6 * np.linalg.norm(ref)
