@@ -6,6 +6,7 @@
 // (i >> 5) is 1 for spin up (s = +0.5, sigma = +1).
 #pragma once
 
+#include <atomic>
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <math.h>
@@ -250,6 +251,24 @@ QES_D double warp_sum(double v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
+
+// ----------------------------------------------------------------------------
+// dynamic shared memory past 48 KB: the attribute is set once per kernel and device (a static of the launch site; the
+// driver call costs 1-2 us, which the smallest batches notice)
+// ----------------------------------------------------------------------------
+struct QesSmemAttr {
+  std::atomic<uint64_t> done{0};
+  cudaError_t set(const void* kernel, int bytes) {
+    if (bytes <= 48 * 1024) return cudaSuccess;
+    int dev = 0;
+    if (cudaError_t e = cudaGetDevice(&dev)) return e;
+    const uint64_t bit = dev < 64 ? 1ull << dev : 0;
+    if (done.load(std::memory_order_relaxed) & bit) return cudaSuccess;
+    if (cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)) return e;
+    done.fetch_or(bit, std::memory_order_relaxed);
+    return cudaSuccess;
+  }
+};
 
 // ----------------------------------------------------------------------------
 // asynchronous copies to shared memory (4, 8 or 16 bytes, both sides aligned to the size)

@@ -471,7 +471,8 @@ static int launch_forward_rs(int ns, int nh, int64_t n, const uint32_t* bits, co
   const bool vec = nh % (16 / (int)sizeof(T)) == 0 && (reinterpret_cast<uintptr_t>(W) & 15) == 0;
   auto kern = vec ? rbm_forward_kernel<T, RS, true, LP> : rbm_forward_kernel<T, RS, false, LP>;
   constexpr int smem = fwd_smem<T, RS>();
-  QES_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  static QesSmemAttr attr[2];
+  QES_CUDA_CHECK(attr[vec].set((const void*)kern, smem));
   kern<<<grid, FWD_THREADS, smem, st>>>(ns, nh, n, bits, a, b, W, theta_out, tanh_out, logpsi_out);
   QES_LAUNCH_CHECK();
   return QES_OK;

@@ -3439,7 +3439,8 @@ static int launch_vjp_mma(int ns, int nh, int64_t n_samples, const uint32_t* bit
   const int64_t gy = (pairs + BMM_WARPS - 1) / BMM_WARPS;
   const size_t smem = (size_t)bsmall_align16((int64_t)PT_SPLIT * (sizeof(T) + 4 * n_words(ns))) +
                       (size_t)BMM_WARPS * ns * sizeof(T);
-  QES_CUDA_CHECK(cudaFuncSetAttribute(vjp_mma_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (smem > 48 * 1024)
+    QES_CUDA_CHECK(cudaFuncSetAttribute(vjp_mma_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int pf = qes_prof_begin(QES_PROF_OHU, st);
   vjp_mma_kernel<T><<<dim3((unsigned)((n_samples + PT_SPLIT - 1) / PT_SPLIT), (unsigned)gy), BMM_THREADS, smem, st>>>(
       ns, nh, n_samples, bits, tt, g, partial);
