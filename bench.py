@@ -851,7 +851,7 @@ def issue_rooflines(cfg, nqs, form, clk):
                                ("local_energy", n * n_moves * net.nh, "sample x move x hidden-unit terms")):
         ms = float(np.mean(form["phase_ms"][phase]))
         tf = units * f_unit / (ms / 1e3) / 1e12
-        out[phase] = {"kernel": "sampler_kernel" if phase == "sample" else "eloc_moves_kernel",
+        out[phase] = {"kernel": "sampler_kernel" if phase == "sample" else "eloc_tile_kernel",
                       "bound": "fp32_issue", "work_units_per_launch": int(units), "unit_definition": what,
                       "flops_per_unit": f_unit, "avg_launch_us": ms * 1e3, "achieved": tf, "peak": peak,
                       "unit": "TFLOP/s", "frac": tf / peak,
@@ -895,7 +895,7 @@ def roofline(cfg, nqs, form):
              "ohu": "tc_ohu_kernel (O^H u, tcgen05)" if tc else "ohu_kernel (O^H u, CUDA cores)",
              "reduce": "reduce_splits_kernel / cg_fused_kernel", "sample": "sampler_kernel",
              "sv": "tc_sv_kernel (S v: O v and O^H u fused, tcgen05)",
-             "local_energy": "eloc_moves_kernel",
+             "local_energy": "eloc_tile_kernel",
              "forward": "theta_tc_kernel (tcgen05)" if dv.forward_uses_tensor_cores(
                  net.flat, net.ns, net.nh, cfg["chains"] * cfg["samples"]) else "rbm_forward_kernel"}
     out = {"kernel": names.get(dom, dom), "launches_timed": cnt, "avg_launch_us": avg_s * 1e6,
@@ -912,14 +912,28 @@ def roofline(cfg, nqs, form):
         # working sets in shared memory and L2: bound by FP32 issue, not by HBM
         ir = issue_rooflines(cfg, nqs, {"phase_ms": phases}, None)[dom]
         ir["share_of_timed_region"] = out["share_of_timed_region"]
+        ir["timed_cg_iteration"] = timed_cg_iteration(cfg, nqs, form, hbm, tc)
         return ir
     else:
         n = cfg["chains"] * cfg["samples"]
         b = n * net.nh * (8 if net.is_complex else 4) + n * ((net.ns + 31) // 32) * 4
         tr = None
     ach = b / avg_s / 1e9
-    out.update({"achieved": ach, "frac": ach / hbm, "algorithmic_bytes_per_launch": int(b), "traffic": tr})
+    out.update({"achieved": ach, "frac": ach / hbm, "algorithmic_bytes_per_launch": int(b), "traffic": tr,
+                "timed_cg_iteration": timed_cg_iteration(cfg, nqs, form, hbm, tc)})
     return out
+
+
+def timed_cg_iteration(cfg, nqs, form, hbm, tc):
+    """The SR phase of the timed (unprofiled) steps per CG iteration.  There the whole solve is one launch
+    (cg_persist_kernel, up to 127 sites) wherever the default tensor-core form fits it; profiled steps run the
+    kernel chain instead, a launch per class."""
+    its, ms = float(np.sum(form["cg_iters"])), float(np.sum(form["phase_ms"]["sr_solve"]))
+    if not its:
+        return None
+    b = kernel_bytes(cfg, nqs, "sv", tc=tc)
+    ach = b / (ms / its / 1e3) / 1e9
+    return {"us": ms / its * 1e3, "algorithmic_bytes": int(b), "achieved": ach, "unit": "GB/s", "frac": ach / hbm}
 
 
 # ---------------------------------------------------------------------------------------- CPU (oracle)

@@ -8,12 +8,12 @@
 // of one complex FMA against per-move tables that depend only on W, so the
 // work is O(K*M) per sample with no transcendental in the inner loop.
 //
-// Mapping: block = 32 moves (threadIdx.x, one warp row) x ELOC_ROWS sample
-// groups (threadIdx.y) of ELOC_SPT samples each.  Tables are stored m-major
-// (Ct[m][k]) so a warp reads 32 consecutive moves of one hidden unit per
-// load; tanh(theta) rows are warp-broadcast.  Each block writes one partial
-// sum per sample (deterministic), reduced by eloc_reduce_kernel together with
-// the diagonal part.
+// One problem runs eloc_tile_kernel (moves x samples in register tiles, tables and tanh rows staged in
+// shared memory), the batched form eloc_moves_block: 32 moves (threadIdx.x, one warp row) x
+// ELOC_ROWS sample groups (threadIdx.y) of ELOC_SPT samples each.  Tables are stored m-major (Ct[m][k])
+// so a warp reads 32 consecutive moves of one hidden unit per load.  Both write one partial sum per 32
+// moves and sample in the same order (bit-identical), reduced by eloc_reduce_kernel together with the
+// diagonal part.
 #include "common.cuh"
 
 #define QES_ARG_CHECK(cond, msg) do { if (!(cond)) { qes_set_last_message(msg); return QES_ERR_ARG; } } while (0)

@@ -2975,13 +2975,18 @@ QES_D void mma16816(float (&d)[4], const uint32_t (&a)[4], uint2 b) {
                : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b.x), "r"(b.y));
 }
-// two floats as three pairs of BF16 (hi + mid + lo is exact: 3 x 8 bits)
+// two floats as three pairs of BF16 (hi + mid + lo is exact: 3 x 8 bits).  A pair with a value past BF16's largest
+// takes a truncated hi, so that finite floats stay finite; of an infinity or a NaN hi is all.
 QES_D void split3(float x, float y, uint32_t (&o)[3]) {
+  constexpr float BF16_MAX = 3.38953139e38f, FLT_LARGEST = 3.402823466e38f;
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(o[k]) : "f"(y), "f"(x));
-    x -= __uint_as_float(o[k] << 16);
-    y -= __uint_as_float(o[k] & 0xffff0000u);
+    if (k == 0 && !(fabsf(x) <= BF16_MAX && fabsf(y) <= BF16_MAX))
+      asm("cvt.rz.bf16x2.f32 %0, %1, %2;" : "=r"(o[0]) : "f"(y), "f"(x));
+    const float rx = x - __uint_as_float(o[k] << 16), ry = y - __uint_as_float(o[k] & 0xffff0000u);
+    x = k > 0 || fabsf(x) <= FLT_LARGEST ? rx : 0.f;
+    y = k > 0 || fabsf(y) <= FLT_LARGEST ? ry : 0.f;
   }
 }
 // bits 8 i + 7 and 8 j + 7 of y as a pair of +-1 in BF16 (set = +1)

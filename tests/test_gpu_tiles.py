@@ -125,3 +125,22 @@ def test_logpsi_vjp_at_tile_edges(cplx, ns, nh, n):
     # products rounded once (complex: three times) and float32 sums of 512 terms: a few 2^-24 of the terms' norm, which the
     # random signs leave as the result's
     assert np.linalg.norm(out - ref) <= 1e-6 * np.linalg.norm(ref)
+
+
+# one sample's infinity or NaN, or the largest float, leaves the same entries finite, infinite and NaN as the CUDA-core form
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan, 3.4e38])
+def test_logpsi_vjp_of_infinities(value):
+    net, st, bits, _ = _problem(False, 20, 24, 70, 0.2)
+    _, tn, _ = dv.rbm_forward(net.flat, 20, 24, bits, tanh=True, logpsi=False)
+    g = torch.ones(70, dtype=torch.complex64, device="cuda")
+    g[33] = value
+    out = dv.logpsi_vjp(net.flat, 20, 24, bits, tn, g)
+    _lib.set_sr_impl(_lib.SR_IMPL_CUDA_CORES)
+    try:
+        ref = dv.logpsi_vjp(net.flat, 20, 24, bits, tn, g)
+    finally:
+        _lib.set_sr_impl(0)
+    assert torch.equal(out.isnan(), ref.isnan()) and torch.equal(out.isinf(), ref.isinf())
+    ok = ref.isfinite()
+    assert (out[ok] - ref[ok]).abs().max() <= 1e-6 * ref[ok].abs().max() if ok.any() else True
+    assert torch.equal(out[ref.isinf()], ref[ref.isinf()])
