@@ -451,6 +451,14 @@ int qes_set_cg_fused_pdl(int on);
  * QES_ERR_TIMEOUT at its next status check; (0, 0) restores the normal
  * barriers.  Process-wide; meant for tests of the time-out path only.      */
 int qes_sr_set_barrier_test(unsigned int extra_arrivals, unsigned int poll_limit);
+/* Test hook of the one-launch CG solve (no reference counterpart), for the
+ * solves that the calling thread starts: in the given pass (-2 the mean row,
+ * -1 the force, 0 .. the iterations) one arrival at the barrier before the
+ * partials are summed (which = 1) or at the one before the next direction is
+ * read (3), or one block's value of a grid-wide sum (2), never comes, and
+ * every wait gives up after `polls` polls, so the solve returns
+ * QES_ERR_TIMEOUT; which = 0 restores the normal waits.                     */
+int qes_sr_set_one_launch_wait_test(int which, int pass, unsigned int polls);
 
 /* RBM forward on the tensor cores: theta = Sigma W + b with W split into
  * three BF16 terms (exact for float32 W) and float32 accumulation; outputs

@@ -26,8 +26,10 @@
 //    one step) the vector is summed in one more exchange.
 //
 // Warps 0-15 compute; warp 16 carries the direction exchange and issues the bulk copies of V, warp 17 the
-// MMAs.  Every wait is bounded: a wait that runs out sets *status or *err, every CTA leaves at its next
-// exchange, and the host reports QES_ERR_TIMEOUT.
+// MMAs.  Every wait is bounded: a wait that runs out sets *status or *err, every CTA leaves after the
+// partials of a pass (or the sums after them) at the latest, and the host reports QES_ERR_TIMEOUT.  The warps meet
+// at kBarAll before every iteration, which is where warps 16 and 17 learn of the end: a CTA that fails in pass -2
+// therefore still builds pass -1's operand, which warp 17 waits for.
 #include "common.cuh"
 #include "sr_pcg.h"
 #include "umma.cuh"
@@ -139,6 +141,8 @@ struct Exchange {
   double* box2;              // [receiver][type][parity][value][kDirect]: subtotals
   unsigned int* count;       // barrier counters, one line each
   int G, nc, cta;
+  uint32_t polls;            // of a wait before it gives up
+  bool mute;                 // test hook: this CTA's value of the next sum is never sent
   int* err;
   int* s_fail;               // shared: written and read by the compute warps inside an exchange only
   const int* s_bad;          // shared: an operand wait gave up (any warp, any time)
@@ -159,8 +163,8 @@ __device__ __forceinline__ void slot_put(double* p, double v) {
 __device__ __forceinline__ void slot_clear(double* p) {
   asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(kEmptySlot) : "memory");
 }
-__device__ __forceinline__ bool slot_wait(const double* p, int* err, double& v) {
-  for (uint32_t it = 0; it < kPollLimit; ++it) {
+__device__ __forceinline__ bool slot_wait(const double* p, uint32_t polls, int* err, double& v) {
+  for (uint32_t it = 0; it < polls; ++it) {
     unsigned long long u;
     asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(u) : "l"(p) : "memory");
     if (u != kEmptySlot) {
@@ -217,18 +221,18 @@ __device__ __forceinline__ bool exchange_sum(const Exchange& X, int type, int pa
     bool good = true;
     const bool direct = X.G <= kDirect;
     if (!direct) {
-      if (lane == 0) slot_put(X.slot1(type, par, warp, X.cta), t);
+      if (lane == 0 && !X.mute) slot_put(X.slot1(type, par, warp, X.cta), t);
       if (X.cta < X.nc) {                                   // senders cta, cta + nc, ...
         const int sender = X.cta + lane * X.nc;
         t = 0.0;
-        if (sender < X.G) good = slot_wait(X.slot1(type, par, warp, sender), X.err, t);
+        if (sender < X.G) good = slot_wait(X.slot1(type, par, warp, sender), X.polls, X.err, t);
         t = warp_sum(t);
       }
     }
-    if (direct || X.cta < X.nc)
+    if (direct ? !X.mute : X.cta < X.nc)
       for (int r = lane; r < X.G; r += 32) slot_put(X.slot2(r, type, par, warp) + X.cta, t);
     t = 0.0;
-    if (lane < X.nc) good = slot_wait(X.slot2(X.cta, type, par, warp) + lane, X.err, t) && good;
+    if (lane < X.nc) good = slot_wait(X.slot2(X.cta, type, par, warp) + lane, X.polls, X.err, t) && good;
     t = warp_sum(t);
     if (!good) *X.s_fail = 1;
     if (lane == 0) X.s_red[16 * kVals + warp] = t;
@@ -252,23 +256,24 @@ __device__ __forceinline__ void exchange_reset(const Exchange& X, int type, int 
 // Grid-wide barrier, one thread of each CTA after its CTA has synchronised: everything that the CTAs wrote
 // to global memory before it is visible after it.  One counter that every CTA polls: 1.2 us on 148 CTAs,
 // against 1.7 us with a separate release flag.
-__device__ __forceinline__ bool grid_arrive_wait(unsigned int* c, unsigned int target, int* err) {
+__device__ __forceinline__ bool grid_arrive_wait(unsigned int* c, unsigned int target, uint32_t polls, int* err) {
   unsigned int v;
   asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(c) : "memory");
   for (uint32_t it = 1;; ++it) {
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(c) : "memory");
     if ((int)(v - target) >= 0) return true;
-    if (it >= kPollLimit || ((it & 1023u) == 0 && *(volatile int*)err != 0)) {
+    if (it >= polls || ((it & 1023u) == 0 && *(volatile int*)err != 0)) {
       atomicCAS(err, 0, 1);
       return false;
     }
   }
 }
-__device__ __forceinline__ bool exchange_barrier(const Exchange& X, int which, unsigned int round) {
+// extra: arrivals that never come (test hook)
+__device__ __forceinline__ bool exchange_barrier(const Exchange& X, int which, unsigned int round, unsigned int extra) {
   bar_sync(kBarCompute, kCompute);
   if (threadIdx.x == 0) {
     if (*(const volatile int*)X.s_bad != 0) *X.s_fail = 1;
-    if (!grid_arrive_wait(X.count + 32 * which, round * (unsigned int)X.G, X.err)) *X.s_fail = 1;
+    if (!grid_arrive_wait(X.count + 32 * which, round * (unsigned int)X.G + extra, X.polls, X.err)) *X.s_fail = 1;
   }
   bar_sync(kBarCompute, kCompute);
   return *(volatile int*)X.s_fail == 0;
@@ -284,7 +289,7 @@ cg_persist_kernel(PcgDims d, int64_t n_samples, const uint32_t* __restrict__ bit
                   double* __restrict__ x_out, double* __restrict__ scal, float4* __restrict__ partial,
                   uint8_t* __restrict__ vz, float* __restrict__ va, double2* __restrict__ wres,
                   double* __restrict__ slots, unsigned int* __restrict__ counters,
-                  int* __restrict__ status, int* __restrict__ err) {
+                  int* __restrict__ status, int* __restrict__ err, PcgWaitTest hook) {
   extern __shared__ __align__(128) uint8_t smem[];
   constexpr bool CPLX = ScalarTraits<T>::is_complex;
   constexpr int H = CPLX ? 2 : 1;
@@ -428,7 +433,7 @@ cg_persist_kernel(PcgDims d, int64_t n_samples, const uint32_t* __restrict__ bit
       }
     }
     const int sg = tid / d.vpc, vl = tid - sg * d.vpc;       // split group and vector of the reduction
-    Exchange X{slots, slots + (size_t)2 * 2 * kVals * G, counters, G, d.nc, cta, err, s_fail, s_bad, s_red};
+    Exchange X{slots, slots + (size_t)2 * 2 * kVals * G, counters, G, d.nc, cta, hook.polls, false, err, s_fail, s_bad, s_red};
     const float fs = (float)(1.0 / (double)n_samples);
     const double inv_n = 1.0 / (double)n_samples;
     float4* part_mine = partial + (int64_t)cta * d.nvec;
@@ -441,6 +446,7 @@ cg_persist_kernel(PcgDims d, int64_t n_samples, const uint32_t* __restrict__ bit
     // pass -2: O^H 1 (conj(O-bar)); pass -1: the force; then the iterations
     for (int it = -2;; ++it) {
       const int par = it & 1;
+      X.mute = hook.which == PcgWaitTest::SUM && it == hook.pass && cta == 0;
       float2 w = make_float2(0.f, 0.f);
       if (it == -2) {
         if (warp < 4 && sval) w = make_float2(1.f, 0.f);
@@ -654,8 +660,9 @@ cg_persist_kernel(PcgDims d, int64_t n_samples, const uint32_t* __restrict__ bit
       } else if (it >= 0 && warp < 3) {
         bar_arrive(kBarLeft, 128);
       }
-      ok = exchange_barrier(X, X_PART, (unsigned int)(it + 3)) && ok;
-      if (!ok) break;
+      ok = exchange_barrier(X, X_PART, (unsigned int)(it + 3),
+                            hook.which == PcgWaitTest::PARTIALS && it == hook.pass ? 1u : 0u) && ok;
+      if (!ok && it > -2) break;                             // from pass -2 by way of pass -1: see the header
       if (it >= 0) {                                         // the previous pass's words: read by everyone
         exchange_reset(X, X_DOTS, par ^ 1);
         exchange_reset(X, X_RR, par ^ 1);
@@ -810,7 +817,9 @@ cg_persist_kernel(PcgDims d, int64_t n_samples, const uint32_t* __restrict__ bit
       bar_sync(kBarAll, kThreadsP);
       if (__shfl_sync(0xffffffffu, *(volatile int*)s_stop, 0) != 0) break;
       ++round;
-      if (lane == 0 && !grid_arrive_wait(counters + 32 * X_DIR, round * (unsigned int)G, err)) *(volatile int*)s_bad = 1;
+      const unsigned int extra = hook.which == PcgWaitTest::DIRECTION && (int)round == hook.pass + 1 ? 1u : 0u;
+      if (lane == 0 && !grid_arrive_wait(counters + 32 * X_DIR, round * (unsigned int)G + extra, hook.polls, err))
+        *(volatile int*)s_bad = 1;
       bar_arrive(kBarGo, kCompute + 32);
       if (lane == 0) {
         asm volatile("fence.proxy.async.global;" ::: "memory");     // other CTAs' stores before the bulk reads
@@ -946,6 +955,16 @@ size_t pcg_operand_bytes(const PcgDims& d) { return (size_t)d.Kz * d.NZ * 4 + (s
 static size_t pcg_box_bytes(const PcgDims& d) {
   return (size_t)4 * kVals * d.G * (1 + kDirect) * sizeof(double);
 }
+// the calling thread's test hook
+static thread_local PcgWaitTest t_wait_test{PcgWaitTest::NONE, 0, kPollLimit};
+extern "C" int qes_sr_set_one_launch_wait_test(int which, int pass, unsigned int polls) {
+  if (which < PcgWaitTest::NONE || which > PcgWaitTest::DIRECTION || (which != PcgWaitTest::NONE && polls == 0)) {
+    qes_set_last_message("qes_sr_set_one_launch_wait_test: which 0 (off), 1 (partials), 2 (sum) or 3 (direction), polls > 0");
+    return QES_ERR_ARG;
+  }
+  t_wait_test = PcgWaitTest{which, pass, which == PcgWaitTest::NONE ? kPollLimit : std::min(polls, kPollLimit)};
+  return QES_OK;
+}
 size_t pcg_slot_bytes(const PcgDims& d) { return pcg_box_bytes(d) + 256 + (size_t)d.G * sizeof(double2); }
 
 template <class T>
@@ -970,7 +989,8 @@ static int pcg_solve_t(const PcgDims& d, int64_t n, const PcgArgs& a, cudaStream
   float* va = reinterpret_cast<float*>(vz + (((size_t)d.Kz * d.NZ * 4 + 127) & ~(size_t)127));
   QES_CUDA_CHECK(cudaLaunchKernelEx(&cfg, cg_persist_kernel<T>, d, n, a.bits, (const T*)a.tt, a.eloc, a.wts, a.shift,
                                     a.rtol, a.atol, a.maxiter, a.prefactor, (double*)a.x, (double*)a.b,
-                                    (double*)a.x_out, a.scal, (float4*)a.partial, vz, va, wres, a.slots, counters, a.status, a.err));
+                                    (double*)a.x_out, a.scal, (float4*)a.partial, vz, va, wres, a.slots, counters, a.status, a.err,
+                                    t_wait_test));
   QES_LAUNCH_CHECK();
   return QES_OK;
 }

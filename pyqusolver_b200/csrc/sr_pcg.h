@@ -22,6 +22,13 @@ struct PcgDims {
   int tmem_cols, smem;
 };
 
+// test hook: the wait that runs out (in pass -2, -1, 0, ...; DIRECTION from pass 0 on) and the polls before it does
+struct PcgWaitTest {
+  enum { NONE = 0, PARTIALS = 1, SUM = 2, DIRECTION = 3 };
+  int which, pass;
+  uint32_t polls;
+};
+
 // whether the shapes admit the persistent kernel, and its tiling
 bool pcg_plan(int dtype, int ns, int nh, int64_t n_samples, PcgDims* d);
 size_t pcg_partial_bytes(const PcgDims& d);

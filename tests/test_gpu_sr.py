@@ -527,3 +527,25 @@ def test_persistent_cg_stops_as_the_rule_says(cplx):
     assert float((x * -1e9 - F).abs().max()) <= 1e-4 * float(F.abs().max())
     _, info = dv.sr_solve_cg(net.flat, ns, nh, bits, tn, eloc, shift=1e-6, rtol=1e-12, maxiter=3)
     assert not info["converged"] and info["iterations"] == 3
+
+
+# pass -2: the mean row, -1: the force, 0 ..: the iterations; on up to 32 blocks and on more (sums by collectors)
+@pytest.mark.parametrize("n", [500, 6000])
+@pytest.mark.parametrize("which,pass_", [(1, -2), (1, -1), (1, 0), (1, 3), (2, -1), (2, 0), (2, 2), (3, 0), (3, 1)])
+def test_persistent_cg_waits_that_run_out_are_reported(which, pass_, n):
+    """A wait for the partials (1), for a block's sum (2) or for the next direction (3) that runs out in any pass ends
+    the solve with QES_ERR_TIMEOUT, and the next solve is the one before."""
+    ns, nh = 20, 41
+    net, bits, tn, eloc = _persistent_problem(True, ns, nh, n)
+    kw = dict(shift=1e-2, rtol=1e-8, maxiter=2000)
+    ref, info_ref = dv.sr_solve_cg(net.flat, ns, nh, bits, tn, eloc, **kw)
+    assert info_ref["iterations"] > 4
+    try:
+        _lib.call("qes_sr_set_one_launch_wait_test", which, pass_, 20000)
+        with pytest.raises(_lib.QESError) as ei:
+            dv.sr_solve_cg(net.flat, ns, nh, bits, tn, eloc, **kw)
+        assert ei.value.code == _lib.QES_ERR_TIMEOUT
+    finally:
+        _lib.call("qes_sr_set_one_launch_wait_test", 0, 0, 0)
+    x, info = dv.sr_solve_cg(net.flat, ns, nh, bits, tn, eloc, **kw)
+    assert torch.equal(x, ref) and info == info_ref
