@@ -455,7 +455,8 @@ int qes_sr_set_barrier_test(unsigned int extra_arrivals, unsigned int poll_limit
  * solves that the calling thread starts: in the given pass (-2 the mean row,
  * -1 the force, 0 .. the iterations) one arrival at the barrier before the
  * partials are summed (which = 1) or at the one before the next direction is
- * read (3), or one block's value of a grid-wide sum (2), never comes, and
+ * read (3), or one block's value of a grid-wide sum (2), or one copy of the
+ * direction operand (4), never comes, and
  * every wait gives up after `polls` polls, so the solve returns
  * QES_ERR_TIMEOUT; which = 0 restores the normal waits.                     */
 int qes_sr_set_one_launch_wait_test(int which, int pass, unsigned int polls);

@@ -29,7 +29,9 @@
 // MMAs.  Every wait is bounded: a wait that runs out sets *status or *err, every CTA leaves after the
 // partials of a pass (or the sums after them) at the latest, and the host reports QES_ERR_TIMEOUT.  The warps meet
 // at kBarAll before every iteration, which is where warps 16 and 17 learn of the end: a CTA that fails in pass -2
-// therefore still builds pass -1's operand, which warp 17 waits for.
+// therefore still builds pass -1's operand, which warp 17 waits for.  A compute warp arrives for an operand stage again
+// only after warp 17 has met its last arrival: warp 17 waits for nothing but copies that are under way (kBarGo comes
+// first) and gives up on all of an iteration's before a compute warp gives up on their products.
 #include "common.cuh"
 #include "sr_pcg.h"
 #include "umma.cuh"
@@ -42,7 +44,8 @@ namespace {
 
 constexpr int kCompute = 512;                    // threads of the compute warps
 constexpr int kThreadsP = kCompute + 64;         // + bulk-copy warp and MMA warp
-constexpr uint32_t kWaitP = 1u << 22;            // try_wait polls before giving up
+constexpr uint32_t kWaitP = 1u << 22;            // try_wait polls of the compute warps before giving up
+constexpr uint32_t kWaitOp = kWaitP >> 4;        // of warps 16 and 17, once per k-step: up to 8 in a row are over first
 constexpr uint32_t kPollLimit = 1u << 22;        // slot polls before giving up
 constexpr size_t kSmemMax = 227 * 1024;
 constexpr unsigned long long kEmptySlot = ~0ull;  // a NaN pattern that no sum produces
@@ -463,7 +466,7 @@ cg_persist_kernel(PcgDims d, int64_t n_samples, const uint32_t* __restrict__ bit
         }
       } else {
         // ---- w = O p: sigma . v_a while the MMAs run, then t . z
-        bar_sync(kBarGo, kCompute + 32);                     // every CTA's operand entries are written
+        bar_sync(kBarGo, kCompute + 64);                     // every CTA's operand entries are written
         float2 acc = make_float2(0.f, 0.f);
         if (cg < nw) {
           float vr = 0.f, vi = 0.f;
@@ -813,6 +816,8 @@ cg_persist_kernel(PcgDims d, int64_t n_samples, const uint32_t* __restrict__ bit
     // ------------------------------------------------------------------ bulk copies of the direction operand
     int g = 2 * nqs;                                         // the two passes before the first iteration
     unsigned int round = 0;
+    uint32_t last_ph = ~0u;                                  // per stage, phase of its last copy (none: passed)
+    const int skip = hook.which == PcgWaitTest::COPY && cta == 0 ? g + hook.pass * (nks + nqs) : -1;   // test hook
     for (;;) {
       bar_sync(kBarAll, kThreadsP);
       if (__shfl_sync(0xffffffffu, *(volatile int*)s_stop, 0) != 0) break;
@@ -820,22 +825,29 @@ cg_persist_kernel(PcgDims d, int64_t n_samples, const uint32_t* __restrict__ bit
       const unsigned int extra = hook.which == PcgWaitTest::DIRECTION && (int)round == hook.pass + 1 ? 1u : 0u;
       if (lane == 0 && !grid_arrive_wait(counters + 32 * X_DIR, round * (unsigned int)G + extra, hook.polls, err))
         *(volatile int*)s_bad = 1;
-      bar_arrive(kBarGo, kCompute + 32);
+      bar_arrive(kBarGo, kCompute + 64);
       if (lane == 0) {
         asm volatile("fence.proxy.async.global;" ::: "memory");     // other CTAs' stores before the bulk reads
         for (int c = 0; c < nks; ++c) {
           const int u = g + c, st = u % S;
-          if (u >= S && !umma::mbar_wait(&empty[st], ((u / S) - 1) & 1, kWaitP)) {
+          if (u >= S && !umma::mbar_wait(&empty[st], ((u / S) - 1) & 1, kWaitOp)) {
             gave_up();
             break;
           }
+          if (u == skip) continue;
           umma::mbar_arrive_expect_tx(&full[st], stage_bytes);
           umma::bulk_g2s(sB + (size_t)st * stage_bytes, vz + (size_t)c * stage_bytes, stage_bytes, &full[st]);
+          last_ph ^= 1u << st;
         }
       }
       g += nks + nqs;
       __syncwarp();
     }
+    if (lane == 0) {                                         // no copy outlives the block, whoever gave up
+#pragma unroll 1
+      for (int st = 0; st < S; ++st) umma::mbar_wait(&full[st], (last_ph >> st) & 1u, kWaitOp);
+    }
+    __syncwarp();
   } else {
     // ------------------------------------------------------------------ MMA issue
     const int n_parts = NZ > 256 ? 2 : 1;
@@ -858,10 +870,11 @@ cg_persist_kernel(PcgDims d, int64_t n_samples, const uint32_t* __restrict__ bit
       if (it >= 0) {
         bar_sync(kBarAll, kThreadsP);
         if (__shfl_sync(0xffffffffu, *(volatile int*)s_stop, 0) != 0) break;
+        bar_sync(kBarGo, kCompute + 64);
         if (lane == 0) {
           for (int c = 0; c < nks; ++c) {
             const int st = (g + c) % S;
-            if (!umma::mbar_wait(&full[st], (fph >> st) & 1u, kWaitP)) {
+            if (!umma::mbar_wait(&full[st], (fph >> st) & 1u, kWaitOp)) {
               gave_up();
             }
             fph ^= 1u << st;
@@ -958,8 +971,9 @@ static size_t pcg_box_bytes(const PcgDims& d) {
 // the calling thread's test hook
 static thread_local PcgWaitTest t_wait_test{PcgWaitTest::NONE, 0, kPollLimit};
 extern "C" int qes_sr_set_one_launch_wait_test(int which, int pass, unsigned int polls) {
-  if (which < PcgWaitTest::NONE || which > PcgWaitTest::DIRECTION || (which != PcgWaitTest::NONE && polls == 0)) {
-    qes_set_last_message("qes_sr_set_one_launch_wait_test: which 0 (off), 1 (partials), 2 (sum) or 3 (direction), polls > 0");
+  if (which < PcgWaitTest::NONE || which > PcgWaitTest::COPY || (which != PcgWaitTest::NONE && polls == 0)) {
+    qes_set_last_message("qes_sr_set_one_launch_wait_test: which 0 (off), 1 (partials), 2 (sum), 3 (direction) or 4 (copy), "
+                         "polls > 0");
     return QES_ERR_ARG;
   }
   t_wait_test = PcgWaitTest{which, pass, which == PcgWaitTest::NONE ? kPollLimit : std::min(polls, kPollLimit)};

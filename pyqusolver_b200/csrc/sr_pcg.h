@@ -22,9 +22,9 @@ struct PcgDims {
   int tmem_cols, smem;
 };
 
-// test hook: the wait that runs out (in pass -2, -1, 0, ...; DIRECTION from pass 0 on) and the polls before it does
+// test hook: the wait that runs out (in pass -2, -1, 0, ...; DIRECTION and COPY from pass 0 on) and the polls before it does
 struct PcgWaitTest {
-  enum { NONE = 0, PARTIALS = 1, SUM = 2, DIRECTION = 3 };
+  enum { NONE = 0, PARTIALS = 1, SUM = 2, DIRECTION = 3, COPY = 4 };
   int which, pass;
   uint32_t polls;
 };

@@ -549,3 +549,22 @@ def test_persistent_cg_waits_that_run_out_are_reported(which, pass_, n):
         _lib.call("qes_sr_set_one_launch_wait_test", 0, 0, 0)
     x, info = dv.sr_solve_cg(net.flat, ns, nh, bits, tn, eloc, **kw)
     assert torch.equal(x, ref) and info == info_ref
+
+
+@pytest.mark.parametrize("cplx,ns,nh,n,pass_", [(True, 20, 41, 6000, 0), (False, 48, 15, 2049, 2), (True, 100, 200, 16384, 1)])
+def test_persistent_cg_operand_copy_that_never_lands(cplx, ns, nh, n, pass_):
+    """A copy of the direction operand that never lands: the warp that waits for it gives up on every k-step before the
+    warps behind it do, so that no barrier is passed twice; the solve reports QES_ERR_TIMEOUT, the next is the one
+    before.  (100 x 200: two operand stages for seven k-steps.)"""
+    net, bits, tn, eloc = _persistent_problem(cplx, ns, nh, n)
+    kw = dict(shift=1e-2, rtol=1e-8, maxiter=8, allow_not_converged=True)
+    ref, info_ref = dv.sr_solve_cg(net.flat, ns, nh, bits, tn, eloc, **kw)
+    try:
+        _lib.call("qes_sr_set_one_launch_wait_test", 4, pass_, 1000)
+        with pytest.raises(_lib.QESError) as ei:
+            dv.sr_solve_cg(net.flat, ns, nh, bits, tn, eloc, **kw)
+        assert ei.value.code == _lib.QES_ERR_TIMEOUT
+    finally:
+        _lib.call("qes_sr_set_one_launch_wait_test", 0, 0, 0)
+    x, info = dv.sr_solve_cg(net.flat, ns, nh, bits, tn, eloc, **kw)
+    assert torch.equal(x, ref) and info == info_ref
