@@ -3633,13 +3633,13 @@ static int launch_batch_ohu(int n_ohu, size_t smem, const qes_batch_instance* in
 
 struct BatchGraphKey {
   const void* inst; const void* ov_items; const void* ohu_items; const void* bits; const void* tt; const void* x;
-  const void* bscal;
+  const void *bscal, *n_done, *w, *partial, *r, *p, *pf;     // offsets in the workspace follow from the totals
   int n_inst, n_ov, n_ohu, chunk, cplx, own_mean;
   int64_t ov_smem, ohu_smem, upd_smem;
   double shift;
   bool operator==(const BatchGraphKey& o) const { return std::memcmp(this, &o, sizeof(*this)) == 0; }
 };
-static_assert(sizeof(BatchGraphKey) == 7 * sizeof(void*) + 6 * 4 + 3 * 8 + 8, "BatchGraphKey has padding bytes");
+static_assert(sizeof(BatchGraphKey) == 13 * sizeof(void*) + 6 * 4 + 3 * 8 + 8, "BatchGraphKey has padding bytes");
 struct BatchGraphSlot {
   bool init = false;
   cudaStream_t cs = nullptr;
@@ -3737,7 +3737,8 @@ static int batch_sr_cg_t(int n_inst, const qes_batch_instance* inst, int n_ov, c
         QES_CUDA_CHECK(cudaEventCreateWithFlags(&gs.ev_out, cudaEventDisableTiming));
         gs.init = true;
       }
-      const BatchGraphKey key{inst, ov_items, ohu_items, bits, tt, x, L.bscal, n_inst, n_ov, n_ohu, nrun,
+      const BatchGraphKey key{inst, ov_items, ohu_items, bits, tt, x, L.bscal, L.n_done, L.w, partial, r, p, pf,
+                              n_inst, n_ov, n_ohu, nrun,
                               CPLX ? 1 : 0, own_mean, (int64_t)ov_smem, (int64_t)ohu_smem,
                               (int64_t)upd_smem, opt->shift};
       if (gs.exec == nullptr || !(gs.key == key)) {

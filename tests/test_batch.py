@@ -170,3 +170,41 @@ def test_batched_solve_at_tile_edges(dtype, Ls, alpha, chains, nsamp):
         # the CG's own bar, and float32 sums of up to max(n, L, nh) terms in an operator of condition kappa
         tol = rtol + 4.0 * np.sqrt(max(n, L, t.shape[1])) * 2.0 ** -24 * kappa
         assert np.linalg.norm(r) <= tol * np.linalg.norm(F), (L, np.linalg.norm(r) / np.linalg.norm(F), tol)
+
+
+def test_batched_solves_of_other_row_counts_through_the_same_buffers():
+    """Two batches that agree in everything but their rows (200 and 250 per problem), solved in turn through the same
+    device buffers and workspace: the graph of CG chunks captured for one is not replayed for the other, whose
+    vectors lie elsewhere in the workspace."""
+    models = [tfim_chain(L, 1.1) for L in (14, 15)]
+    batches = []
+    for nsamp in (4, 5):
+        B = NQSBatch(models, alpha=1.0, dtype="float32", seeds=[3, 4], s_numchains=50, s_numsamples=nsamp,
+                     init_scale=0.1, autotune=False, warps_per_block=4, blocks_per_sm=2)
+        B.sample()
+        B.forward()
+        B.local_energy()
+        batches.append(B)
+    names = ("inst", "items_ov", "items_ohu", "sample_bits", "tanh", "eloc", "x", "sr_ws")
+    own = [{k: getattr(B, k) for k in names} for B in batches]
+    size = {k: max(o[k].numel() for o in own) for k in names}
+    shared = {k: torch.zeros(2 * size[k], dtype=own[0][k].dtype, device=own[0][k].device) for k in names}
+
+    def solve(q):
+        B = batches[q]
+        for k in names:
+            src = own[q][k]
+            dst = shared[k][:src.numel()].view(src.shape)
+            dst.copy_(src)
+            setattr(B, k, shared[k] if k == "sr_ws" else dst)
+        x, res = B.sr_solve(shift=1e-2, rtol=0.0, maxiter=12, check_every=4)
+        return x.clone(), [r.iterations for r in res]
+
+    try:
+        _lib.call("qes_set_cg_graphs", 0)
+        ref = [solve(q) for q in (0, 1)]
+    finally:
+        _lib.call("qes_set_cg_graphs", 1)
+    for q in (0, 1, 0):
+        x, its = solve(q)
+        assert its == ref[q][1] and torch.equal(x, ref[q][0]), q
