@@ -253,19 +253,22 @@ QES_D double warp_sum(double v) {
 }
 
 // ----------------------------------------------------------------------------
-// dynamic shared memory past 48 KB: the attribute is set once per kernel and device (a static of the launch site; the
-// driver call costs 1-2 us, which the smallest batches notice)
+// dynamic shared memory past 48 KB: the attribute is set once per kernel and device, to the most that any launch of the
+// kernel asks for (a static of the launch site; the driver call costs 1-2 us, which the smallest batches notice).  It is
+// one value for all host threads, hence a constant: set per call to the launch's own size, one thread's smaller size could come
+// between another's set and its launch, which then fails.
 // ----------------------------------------------------------------------------
 struct QesSmemAttr {
   std::atomic<uint64_t> done{0};
-  cudaError_t set(const void* kernel, int bytes) {
-    if (bytes <= 48 * 1024) return cudaSuccess;
+  template <int BYTES, class K>
+  cudaError_t set(K* kernel) {
+    if (BYTES <= 48 * 1024) return cudaSuccess;
     int dev = 0;
     if (cudaError_t e = cudaGetDevice(&dev)) return e;
     const uint64_t bit = dev < 64 ? 1ull << dev : 0;
-    if (done.load(std::memory_order_relaxed) & bit) return cudaSuccess;
-    if (cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)) return e;
-    done.fetch_or(bit, std::memory_order_relaxed);
+    if (done.load(std::memory_order_acquire) & bit) return cudaSuccess;
+    if (cudaError_t e = cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BYTES)) return e;
+    done.fetch_or(bit, std::memory_order_release);
     return cudaSuccess;
   }
 };

@@ -389,7 +389,7 @@ static int launch_eloc_tiles(int ns, int nh, int64_t n, const uint32_t* bits, co
   constexpr size_t smem = eloc_tile_smem<T, RS>();
   auto kern = vec ? eloc_tile_kernel<T, RS, true> : eloc_tile_kernel<T, RS, false>;
   static QesSmemAttr attr[2];
-  QES_CUDA_CHECK(attr[vec].set((const void*)kern, (int)smem));
+  QES_CUDA_CHECK(attr[vec].set<(int)smem>(kern));
   kern<<<dim3(eloc_kblocks(K), (unsigned)nsb), ELT_THREADS, smem, st>>>(ns, nh, n, bits, tt, K, ham->move_i, ham->move_j,
                                                                        ham->move_kind, (const float4*)ham->move_coef, Ct,
                                                                        St, A, partial);

@@ -472,7 +472,7 @@ static int launch_forward_rs(int ns, int nh, int64_t n, const uint32_t* bits, co
   auto kern = vec ? rbm_forward_kernel<T, RS, true, LP> : rbm_forward_kernel<T, RS, false, LP>;
   constexpr int smem = fwd_smem<T, RS>();
   static QesSmemAttr attr[2];
-  QES_CUDA_CHECK(attr[vec].set((const void*)kern, smem));
+  QES_CUDA_CHECK(attr[vec].set<smem>(kern));
   kern<<<grid, FWD_THREADS, smem, st>>>(ns, nh, n, bits, a, b, W, theta_out, tanh_out, logpsi_out);
   QES_LAUNCH_CHECK();
   return QES_OK;
@@ -702,8 +702,8 @@ extern "C" int qes_batch_rbm_forward(int dtype, int n_inst, const qes_batch_inst
   if (n_items == 0) return QES_OK;
   QES_ARG_CHECK(inst && items && params && sample_bits, "qes_batch_rbm_forward: null pointer");
   cudaStream_t st = (cudaStream_t)stream;
-  QES_CUDA_CHECK(cudaFuncSetAttribute(batch_forward_kernel<float2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      fwd_smem<float2, 2>()));
+  static QesSmemAttr attr;
+  QES_CUDA_CHECK((attr.set<fwd_smem<float2, 2>()>(batch_forward_kernel<float2>)));
   if (dtype == QES_DTYPE_F32)
     batch_forward_kernel<float><<<n_items, FWD_THREADS, fwd_smem<float, 2>(), st>>>(inst, (const int4*)items, (const float*)params,
                                                                   sample_bits, (float*)tanh_out, (float*)logpsi_out);

@@ -516,9 +516,10 @@ static int launch_sampler_kernel(unsigned grid, size_t smem, const qes_sampler_c
                                  const void* pairC, const void* pairS, uint32_t* chain_bits, uint64_t* chain_step,
                                  int32_t* proposed, int32_t* accepted, uint32_t* sample_bits, void* sample_logpsi,
                                  void* last_logpsi, const float* chain_beta, cudaStream_t st) {
-  if (SM)
-    QES_CUDA_CHECK(cudaFuncSetAttribute(sampler_kernel<T, MPL, RULE, SM, MINB>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (SM) {
+    static QesSmemAttr attr;                                  // nh <= 32 MPL
+    QES_CUDA_CHECK((attr.set<SMP_WARPS * 2 * 32 * MPL * (int)sizeof(T)>(sampler_kernel<T, MPL, RULE, SM, MINB>)));
+  }
   sampler_kernel<T, MPL, RULE, SM, MINB><<<grid, 32 * SMP_WARPS, smem, st>>>(
       *cfg, (const T*)a, (const T*)b, (const T*)W, (const T*)flipC, (const T*)flipS, nbr, nbr_pair, pi, pj,
       (const T*)pairC, (const T*)pairS, chain_bits, chain_step, proposed, accepted, sample_bits,

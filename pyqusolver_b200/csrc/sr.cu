@@ -677,15 +677,9 @@ static int launch_reduce_splits(int64_t P, int nsplit, const void* partial, doub
   if constexpr (!IsF64<T>::value) {
     const size_t bulk_smem = (size_t)nsplit * (size_t)cv * 16;
     if (vec && g_reduce_bulk.load() != 0 && bulk_smem <= kReduceBulkSmem) {
-      static bool attr_set = false;                        // per process (the attribute is per function)
-      if (!attr_set) {
-        QES_CUDA_CHECK(cudaFuncSetAttribute(reduce_splits_bulk_kernel<T, V, false>,
-                                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kReduceBulkSmem));
-        QES_CUDA_CHECK(cudaFuncSetAttribute(reduce_splits_bulk_kernel<T, V, true>,
-                                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kReduceBulkSmem));
-        attr_set = true;
-      }
       auto kern = cg ? reduce_splits_bulk_kernel<T, V, true> : reduce_splits_bulk_kernel<T, V, false>;
+      static QesSmemAttr attr[2];
+      QES_CUDA_CHECK(attr[cg].set<(int)kReduceBulkSmem>(kern));
       QES_CUDA_CHECK(qes_launch_pdl(kern, dim3(grid), dim3(RS_THREADS), bulk_smem, st, P, nsplit, (int)cv,
                                     (const T*)partial, shift, p, y, dot_part, scal, counter, cg_done, pold, sold,
                                     counter ? (int*)(counter + 4) : (int*)nullptr));
@@ -2954,6 +2948,7 @@ __global__ void __launch_bounds__(BCG_THREADS) batch_mean_kernel(const qes_batch
 template <class T>
 constexpr int bparts() { return ScalarTraits<T>::is_complex ? 2 : 1; }   // real numbers per T
 constexpr int BMM_THREADS = 256, BMM_WARPS = BMM_THREADS / 32;
+constexpr int BATCH_SMEM_MAX = 224 * 1024;       // of the block's 227 KB; at ns * nh <= 16384 (8192) at most 200,832 bytes (O p)
 constexpr int64_t BMEAN_ROWS = 16384;            // up to here every ohu block sums its problem's w itself
 
 QES_HD int64_t bsmall_align16(int64_t bytes) { return (bytes + 15) & ~(int64_t)15; }
@@ -3444,8 +3439,9 @@ static int launch_vjp_mma(int ns, int nh, int64_t n_samples, const uint32_t* bit
   const int64_t gy = (pairs + BMM_WARPS - 1) / BMM_WARPS;
   const size_t smem = (size_t)bsmall_align16((int64_t)PT_SPLIT * (sizeof(T) + 4 * n_words(ns))) +
                       (size_t)BMM_WARPS * ns * sizeof(T);
-  if (smem > 48 * 1024)
-    QES_CUDA_CHECK(cudaFuncSetAttribute(vjp_mma_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  constexpr int most = PT_SPLIT * ((int)sizeof(T) + VJP_MAX_NS / 8) + BMM_WARPS * VJP_MAX_NS * (int)sizeof(T);
+  static QesSmemAttr attr;
+  QES_CUDA_CHECK(attr.set<most>(vjp_mma_kernel<T>));
   const int pf = qes_prof_begin(QES_PROF_OHU, st);
   vjp_mma_kernel<T><<<dim3((unsigned)((n_samples + PT_SPLIT - 1) / PT_SPLIT), (unsigned)gy), BMM_THREADS, smem, st>>>(
       ns, nh, n_samples, bits, tt, g, partial);
@@ -3611,7 +3607,8 @@ template <class T>
 static int launch_batch_ov(int n_ov, size_t smem, const qes_batch_instance* inst, const int4* items,
                            const uint32_t* bits, const T* tt, const T* pf, float2* w, const double* bscal,
                            cudaStream_t st) {
-  QES_CUDA_CHECK(cudaFuncSetAttribute(batch_ov_mma_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  static QesSmemAttr attr;
+  QES_CUDA_CHECK(attr.set<BATCH_SMEM_MAX>(batch_ov_mma_kernel<T>));
   const int pr = qes_prof_begin(QES_PROF_OV, st);
   batch_ov_mma_kernel<T><<<n_ov, BMM_THREADS, smem, st>>>(inst, items, bits, tt, pf, w, bscal);
   qes_prof_end(pr, st);
@@ -3622,8 +3619,8 @@ template <class T>
 static int launch_batch_ohu(int n_ohu, size_t smem, const qes_batch_instance* inst, const int4* items,
                             const uint32_t* bits, const T* tt, const float2* w, const double* bscal, int own_mean,
                             int skip_done, T* partial, cudaStream_t st) {
-  QES_CUDA_CHECK(cudaFuncSetAttribute(batch_ohu_mma_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem));
+  static QesSmemAttr attr;
+  QES_CUDA_CHECK(attr.set<BATCH_SMEM_MAX>(batch_ohu_mma_kernel<T>));
   const int pr = qes_prof_begin(QES_PROF_OHU, st);
   batch_ohu_mma_kernel<T><<<n_ohu, BMM_THREADS, smem, st>>>(inst, items, bits, tt, w, bscal, own_mean, skip_done,
                                                               partial);
@@ -3681,8 +3678,8 @@ static int batch_sr_cg_t(int n_inst, const qes_batch_instance* inst, int n_ov, c
   // the mean of w: every O^H u block reads all rows of its problem, which grows with the square of the rows; beyond
   // BMEAN_ROWS (64 blocks of 128 KB each from L2) one launch per iteration does it
   const int own_mean = max_rows <= BMEAN_ROWS ? 1 : 0;
-  QES_CUDA_CHECK(cudaFuncSetAttribute(batch_cg_update_kernel<T, V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)upd_smem));
+  static QesSmemAttr upd_attr;
+  QES_CUDA_CHECK((upd_attr.set<BATCH_SMEM_MAX>(batch_cg_update_kernel<T, V>)));
   auto ov = [&]() -> int {
     return launch_batch_ov<T>(n_ov, ov_smem, inst, ov_items, bits, tt, pf, L.w, L.bscal, st);
   };

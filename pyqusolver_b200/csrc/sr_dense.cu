@@ -732,8 +732,9 @@ int dense_gram_t(int ns, int nh, int64_t n, const uint32_t* bits, const typename
   dense_x_tiles_kernel<V><<<(unsigned)std::min<int64_t>((items + 255) / 256, 4 * 1184), 256, 0, st>>>(
       ns, nh, n, (int)W.rows, W.n_rb, W.nK, bits, tt, probs, (const V*)W.obar, W.xt);
   QES_LAUNCH_CHECK_N(3);
-  const size_t smem = (size_t)GSTAGES * 4 * GR * GK * 2 + 8 * (2 * GSTAGES + 1) + 16;
-  QES_CUDA_CHECK(cudaFuncSetAttribute(dense_gram_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  constexpr size_t smem = (size_t)GSTAGES * 4 * GR * GK * 2 + 8 * (2 * GSTAGES + 1) + 16;
+  static QesSmemAttr attr;
+  QES_CUDA_CHECK(attr.set<(int)smem>(dense_gram_kernel));
   const int64_t tiles = (int64_t)W.n_rb * (W.n_rb + 1) / 2;
   QES_ARG_CHECK(tiles < (1ll << 31), "dense SR: too many Gram tiles");
   const int pf = qes_prof_begin(QES_PROF_GRAM, st);
@@ -777,10 +778,10 @@ int dense_solve_t(int ns, int nh, int64_t n, const uint32_t* bits, const typenam
   conj_copy_kernel<V><<<vg, 256, 0, st>>>(P, (const V*)W.F, y);
   QES_LAUNCH_CHECK_N(2);
   // blocked Cholesky with the row F^H below the matrix
-  const size_t sm_block = (size_t)CB * LP * sizeof(V);
-  QES_CUDA_CHECK(cudaFuncSetAttribute(chol_panel_kernel<V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)sm_block));
-  QES_CUDA_CHECK(cudaFuncSetAttribute(chol_inv_kernel<V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_block));
+  constexpr size_t sm_block = (size_t)CB * LP * sizeof(V);
+  static QesSmemAttr panel_attr, inv_attr;
+  QES_CUDA_CHECK(panel_attr.set<(int)sm_block>(chol_panel_kernel<V>));
+  QES_CUDA_CHECK(inv_attr.set<(int)sm_block>(chol_inv_kernel<V>));
   const int64_t n_rows = P + 1;
   const int pfc = qes_prof_begin(QES_PROF_CHOL, st);
   chol_diag_kernel<V><<<1, 256, 0, st>>>(A, P, 0, (int)std::min<int64_t>(CB, P), W.flags);

@@ -988,7 +988,8 @@ static int pcg_solve_t(const PcgDims& d, int64_t n, const PcgArgs& a, cudaStream
   QES_CUDA_CHECK(cudaMemsetAsync(a.slots, 0xff, pcg_box_bytes(d), st));
   QES_CUDA_CHECK(cudaMemsetAsync(counters, 0, 256, st));
   QES_CUDA_CHECK(cudaMemsetAsync(a.status, 0, sizeof(int), st));
-  QES_CUDA_CHECK(cudaFuncSetAttribute(cg_persist_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, d.smem));
+  static QesSmemAttr attr;
+  QES_CUDA_CHECK(attr.set<(int)kSmemMax>(cg_persist_kernel<T>));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)d.G);
   cfg.blockDim = dim3(kThreadsP);

@@ -2118,18 +2118,14 @@ TcWork tc_layout(const TcDims& d, char* base) {
 
 template <class T, class V>
 static int tc_set_attrs() {
-  QES_CUDA_CHECK(cudaFuncSetAttribute(tc_ov_kernel<T, V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)kTcSmemLimit));
-  QES_CUDA_CHECK(cudaFuncSetAttribute(tc_ohu_kernel<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)kTcSmemLimit));
-  QES_CUDA_CHECK(cudaFuncSetAttribute(tc_ohu_kernel<T, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)kTcSmemLimit));
-  QES_CUDA_CHECK(cudaFuncSetAttribute(tc_ohu_big_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)kTcSmemLimit));
-  QES_CUDA_CHECK(cudaFuncSetAttribute(tc_sv_kernel<T, V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)kTcSmemLimit));
-  QES_CUDA_CHECK(cudaFuncSetAttribute(tc_ovz_kernel<T, V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)kTcSmemLimit));
+  constexpr int most = (int)kTcSmemLimit;
+  static QesSmemAttr attr[6];
+  QES_CUDA_CHECK((attr[0].set<most>(tc_ov_kernel<T, V>)));
+  QES_CUDA_CHECK((attr[1].set<most>(tc_ohu_kernel<T, 1>)));
+  QES_CUDA_CHECK((attr[2].set<most>(tc_ohu_kernel<T, 2>)));
+  QES_CUDA_CHECK(attr[3].set<most>(tc_ohu_big_kernel<T>));
+  QES_CUDA_CHECK((attr[4].set<most>(tc_sv_kernel<T, V>)));
+  QES_CUDA_CHECK((attr[5].set<most>(tc_ovz_kernel<T, V>)));
   return QES_OK;
 }
 

@@ -286,7 +286,8 @@ static int forward_tc_t(const ThetaDims& d, int64_t n, const uint32_t* bits, con
   T* lsum = reinterpret_cast<T*>(ws + ol);
   int* status = reinterpret_cast<int*>(ws + os);
   QES_CUDA_CHECK(cudaMemsetAsync(status, 0, sizeof(int), st));
-  QES_CUDA_CHECK(cudaFuncSetAttribute(theta_tc_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, d.smem));
+  static QesSmemAttr attr;
+  QES_CUDA_CHECK(attr.set<(int)kSmemLimit>(theta_tc_kernel<T>));
   theta_sig_rows_kernel<<<1184, 256, 0, st>>>(d, n, bits, sig);
   theta_w_terms_kernel<T><<<296, 256, 0, st>>>(d, W, wt);
   theta_tc_kernel<T><<<dim3(d.n_tiles, d.nnc), kThr, d.smem, st>>>(d, n, sig, wt, b, theta_out, tanh_out,

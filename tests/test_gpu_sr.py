@@ -568,3 +568,49 @@ def test_persistent_cg_operand_copy_that_never_lands(cplx, ns, nh, n, pass_):
         _lib.call("qes_sr_set_one_launch_wait_test", 0, 0, 0)
     x, info = dv.sr_solve_cg(net.flat, ns, nh, bits, tn, eloc, **kw)
     assert torch.equal(x, ref) and info == info_ref
+
+
+def _loop_in_threads(calls, rounds):
+    """Each call in its own thread on its own stream, `rounds` times; the results of the last round, or the error."""
+    import threading
+    out, errs = [None] * len(calls), []
+    gate = threading.Barrier(len(calls))
+
+    def work(q):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                gate.wait()
+                for _ in range(rounds):
+                    out[q] = calls[q]()
+                torch.cuda.synchronize()
+        except Exception as e:
+            errs.append(e)
+
+    ts = [threading.Thread(target=work, args=(q,)) for q in range(len(calls))]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not errs, errs
+    return out
+
+
+def test_solves_of_other_shapes_from_two_threads():
+    """The one-launch solve, and log psi's backward, of two shapes that need different amounts of shared memory, from two
+    threads on streams of their own: no call fails, and every result is that of a call alone."""
+    solves, vjps = [], []
+    for cplx, ns, nh, n in [(True, 60, 100, 3000), (True, 16, 40, 500)]:
+        net, bits, tn, eloc = _persistent_problem(cplx, ns, nh, n)
+        ws = dv.sr_workspace(dv.dtype_code(net.flat), ns, nh, n, bits.device)
+        solves.append(lambda a=(net.flat, ns, nh, bits, tn, eloc), ws=ws:
+                      dv.sr_solve_cg(*a, shift=1e-2, rtol=0.0, maxiter=1, workspace=ws, true_residual=False)[0])
+    for cplx, ns, nh, n in [(True, 500, 8, 600), (True, 410, 8, 600)]:
+        net, bits, tn, _ = _persistent_problem(cplx, ns, nh, n)
+        g = torch.as_tensor(np.random.default_rng(1).normal(size=n) + 0j).to(torch.complex64).cuda()
+        ws = dv.sr_workspace(dv.dtype_code(net.flat), ns, nh, n, bits.device)
+        vjps.append(lambda a=(net.flat, ns, nh, bits, tn, g), ws=ws: dv.logpsi_vjp(*a, workspace=ws))
+    for large, small in (solves, vjps):
+        alone = [large(), small()]
+        torch.cuda.synchronize()
+        first, *_, last = _loop_in_threads([large, small], 2000)
+        assert torch.equal(first, alone[0]) and torch.equal(last, alone[1])

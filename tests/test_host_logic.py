@@ -297,3 +297,17 @@ def test_oracle_fast_log_psi_matches_numpy_path():
         finally:
             fast.disable()
         assert np.allclose(got, ref, rtol=0, atol=1e-11)
+
+
+def test_shared_memory_limits_are_compile_time_constants():
+    """A kernel's limit of dynamic shared memory is one value for all host threads, so no launch may set it to its own
+    size: every limit goes through QesSmemAttr::set, whose size is a template argument."""
+    src = os.path.join(ROOT, "pyqusolver_b200", "csrc")
+    calls = []
+    for name in sorted(os.listdir(src)):
+        with open(os.path.join(src, name)) as f:
+            text = f.read()
+        calls += [(name, m.group(1)) for m in re.finditer(r"cudaFuncSetAttribute\(([^;]*)\)", text)]
+    assert [c[0] for c in calls] == ["common.cuh"] and "BYTES" in calls[0][1]
+    with open(os.path.join(src, "common.cuh")) as f:
+        assert re.search(r"template <int BYTES, class K>\s*cudaError_t set\(", f.read())
