@@ -445,6 +445,13 @@ int qes_set_cg_xrp(int on);
  * kernel's tail (TFIM-16 CG iteration 18.8 -> 18.3 us).  Same kernel, same
  * sums: bit-identical results.                                            */
 int qes_set_cg_fused_pdl(int on);
+/* The whole CG solve (no start vector, no preconditioner) as one cooperative
+ * launch: 1 (the default) where the shapes admit it and no tiling or product
+ * is asked for through the qes_sr_set_* calls above; 2 wherever the shapes
+ * admit it, those calls then choosing among the kernels of the other solves;
+ * 0 never; negative: no change.  *previous (may be NULL) gets the mode before
+ * the call.  Process-wide.                                                  */
+int qes_sr_set_one_launch(int mode, int* previous);
 /* Test hook of the fused CG kernel's grid barriers (no reference
  * counterpart): (1, polls) makes every barrier wait for one arrival that
  * never comes and give up after `polls` polls, so a solve returns

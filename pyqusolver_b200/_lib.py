@@ -135,6 +135,7 @@ SIGNATURES = {
     "qes_set_cg_fused_pdl": [C.c_int],
     "qes_sr_set_prefetch": [C.c_int],
     "qes_sr_set_barrier_test": [C.c_uint, C.c_uint],
+    "qes_sr_set_one_launch": [C.c_int, C.POINTER(C.c_int)],
     "qes_sr_set_one_launch_wait_test": [C.c_int, C.c_int, C.c_uint],
     "qes_rbm_forward_tc_workspace_bytes": [C.c_int, C.c_int, C.c_int, _i64, C.POINTER(_sz)],
     "qes_rbm_forward_tc": [C.c_int, C.c_int, C.c_int, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _sz, _vp],

@@ -2008,6 +2008,19 @@ static int sr_jacobi_t(int ns, int nh, int64_t n_samples, const uint32_t* bits, 
   return QES_OK;
 }
 
+// The one-launch solve (1: where the shapes admit it and no tiling or product is asked for through qes_sr_set_*; 2: wherever
+// the shapes admit it, so that a tiling chosen for one shape does not take it from the others; 0: never)
+static std::atomic<int> g_one_launch{1};
+extern "C" int qes_sr_set_one_launch(int mode, int* previous) {
+  if (mode > 2) {
+    qes_set_last_message("qes_sr_set_one_launch: mode 0..2, or negative to ask for the present one");
+    return QES_ERR_ARG;
+  }
+  const int old = mode < 0 ? g_one_launch.load() : g_one_launch.exchange(mode);
+  if (previous) *previous = old;
+  return QES_OK;
+}
+
 // CG of the unweighted start x = 0 without a preconditioner as one launch (sr_pcg.cu)
 template <class T>
 static int sr_cg_persistent_t(int ns, int nh, int64_t n_samples, const uint32_t* bits, const T* tt, const float2* eloc,
@@ -2066,7 +2079,8 @@ static int sr_cg_t(int ns, int nh, int64_t n_samples, const uint32_t* bits, cons
   int rc;
   // one persistent kernel for the force and all iterations, where the shapes admit it and no other form of
   // the solve is asked for
-  if (L.pcg && L.tc && tc_default_form() && !x0 && opt->precond == QES_PRECOND_NONE && g_cg_fused.load() == 1 &&
+  const int one_launch = g_one_launch.load();
+  if (L.pcg && L.tc && (one_launch == 2 || (one_launch == 1 && tc_default_form())) && !x0 && opt->precond == QES_PRECOND_NONE && g_cg_fused.load() == 1 &&
       g_cg_single.load() == 0 && g_bar_extra.load() == 0 && g_l2_persist.load() == 0 && !qes_prof_on())
     return sr_cg_persistent_t<T>(ns, nh, n_samples, bits, tt, eloc, opt, x_out, res, L, st);
   rc = sr_prepare(dtype, n_samples, bits, tt, L, st);

@@ -614,3 +614,49 @@ def test_solves_of_other_shapes_from_two_threads():
         torch.cuda.synchronize()
         first, *_, last = _loop_in_threads([large, small], 2000)
         assert torch.equal(first, alone[0]) and torch.equal(last, alone[1])
+
+
+def _solve_launches(a):
+    before = _lib.launch_count(reset=False)
+    x, info = dv.sr_solve_cg(*a, shift=1e-2, rtol=1e-8, maxiter=40, true_residual=False)
+    return _lib.launch_count(reset=False) - before, x
+
+
+def test_tuned_tiling_leaves_the_one_launch_solve_on(tmp_path):
+    """A tiling tuned for (or read back from a file for) a shape that the one-launch CG does not fit leaves that solve to the
+    shapes that it does fit; a file written when the default candidate was another solver is not read; an explicit
+    switch, and a tiling set by hand, still turn it off."""
+    from pyqusolver_b200 import autotune
+    net, bits, tn, eloc = _persistent_problem(True, 16, 40, 500)
+    small = (net.flat, net.ns, net.nh, bits, tn, eloc)
+    big, bbits, btn, _ = _persistent_problem(False, 140, 40, 600)                 # more than 127 sites
+    cache = tmp_path / "tune.json"
+    other = (2, 32, 148, 0, 0, 0, 1)
+    ref_n, ref = _solve_launches(small)
+    assert ref_n == 1
+    try:
+        for _ in range(2):                                                        # timed, then from the file
+            r = autotune.tune_sr_tiling(big, bbits, btn, repeats=1, iters=2, cache=str(cache),
+                                        candidates=None if cache.exists() else [other])
+            assert tuple(r["choice"]) == other
+            n, x = _solve_launches(small)
+            assert n == 1 and torch.equal(x, ref)
+        assert r["cached"]
+        import json
+        table = json.loads(cache.read_text())
+        (key, entry), = table.items()
+        assert key.startswith("sr_cg_iter8|")
+        cache.write_text(json.dumps({key.replace("iter8", "iter7"): dict(entry, choice=[1, 0, 0, 0, 0, 0, 1])}))
+        r = autotune.tune_sr_tiling(big, bbits, btn, repeats=1, iters=2, cache=str(cache))
+        assert not r["cached"]
+        autotune.apply_tiling(*autotune.DEFAULT_TILING)
+        _lib.call("qes_sr_set_one_launch", 0, None)
+        autotune.apply_tiling(*other)
+        assert _solve_launches(small)[0] > 1                                      # switched off: stays off
+        _lib.call("qes_sr_set_one_launch", 1, None)
+        assert _solve_launches(small)[0] > 1                                      # a tiling asked for by hand
+    finally:
+        _lib.call("qes_sr_set_one_launch", 1, None)
+        autotune.apply_tiling(*autotune.DEFAULT_TILING)
+    n, x = _solve_launches(small)
+    assert n == 1 and torch.equal(x, ref)
