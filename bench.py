@@ -13,7 +13,9 @@ fused local energy, float64 statistics, structured SR CG, float64 update.
 Synthetic data: random-init parameters and random Sz = 0 starting chains.
 
 value = samples/s of the whole job (N GPUs x 16,384 samples per step / time);
-vmc_steps_per_s is reported beside it.  With --gpus N > 1 every rank runs its
+vmc_steps_per_s is reported beside it.  Standard output holds one JSON line with
+the headline figures (below 2,000 characters, so that it survives a log's tail);
+the whole report, a JSON line too, goes to standard error, or to --report FILE.  With --gpus N > 1 every rank runs its
 own independent VMC (replicas, weak scaling, no collective on the data path).
 """
 
@@ -55,6 +57,43 @@ CONFIGS = {
                       chains=4096, samples=4, rule="LOCAL", sweep=400, shift=1e-4, lr=0.01, rtol=1e-8, maxiter=1000,
                       init="RND"),
 }
+
+
+def _short(o):
+    """Floats to nine significant digits."""
+    if isinstance(o, float):
+        return float(f"{o:.9g}")
+    if isinstance(o, dict):
+        return {k: _short(v) for k, v in o.items()}
+    return [_short(v) for v in o] if isinstance(o, (list, tuple)) else o
+
+
+def headline(line):
+    """The part of a report that goes to standard output: what identifies and states the measurement whole, of the
+    rest a figure each."""
+    rest = ("forms", "issue_rooflines", "sr_tiling", "accuracy", "accuracy_ed_j1j2_6x6", "accuracy_matched_fp64",
+            "accuracy_matched_fp64_other", "other_configs", "dense_sr", "roofline", "cpu_baseline")
+    out = {k: v for k, v in line.items() if k not in rest}
+    keep = {"roofline": ("kernel", "bound", "avg_launch_us", "achieved", "peak", "unit", "frac"),
+            "cpu_baseline": ("value", "unit", "cores", "kind")}
+    for k, names in keep.items():
+        if line.get(k):
+            out[k] = {n: line[k][n] for n in names if n in line[k]}
+    if "mixed_over_plain_steps_per_s" in line.get("forms", {}):
+        out["mixed_over_plain_steps_per_s"] = line["forms"]["mixed_over_plain_steps_per_s"]
+    oc = line.get("other_configs", {})
+    if oc:
+        out["other_vmc_steps_per_s"] = {n: (c.get("mixed") or c)["vmc_steps_per_s"] for n, c in oc.items()}
+    return _short(out)
+
+
+def print_report(line, args):
+    if args.report:
+        with open(args.report, "w") as f:
+            f.write(json.dumps(line) + "\n")
+    else:
+        print(json.dumps(line), file=sys.stderr, flush=True)
+    print(json.dumps(headline(line)), flush=True)
 
 
 def env_rank():
@@ -463,7 +502,7 @@ def run_batch(args, cfg, rank, world, local_rank):
         line["cpu_baseline"] = cpu_baseline(cfg, budget_s=args.cpu_budget)
     replicas.finish(dist)
     if rank == 0:
-        print(json.dumps(line))
+        print_report(line, args)
 
 
 def batch_accuracy(B, cfg, epochs, Ls):
@@ -618,7 +657,7 @@ def run_ours(args, cfg, rank, world, local_rank):
         line["cpu_baseline"] = cpu_baseline(cfg, budget_s=args.cpu_budget)
     replicas.finish(dist)
     if rank == 0:
-        print(json.dumps(line))
+        print_report(line, args)
 
 
 def config_summary(name, steps, warmup, flush):
@@ -1070,6 +1109,7 @@ def main():
     ap.add_argument("--config", default="heis10x10", choices=sorted(CONFIGS))
     ap.add_argument("--impl", default="ours", choices=["ours", "reference"])
     ap.add_argument("--no-cpu-baseline", action="store_true")
+    ap.add_argument("--report", default="", help="file for the whole report (default: standard error)")
     ap.add_argument("--forms", default="plain_fp32,mixed", help="comma list of plain_fp32, mixed (mixed is required)")
     ap.add_argument("--cpu-budget", type=float, default=20.0)
     ap.add_argument("--ed-epochs", type=int, default=1500,

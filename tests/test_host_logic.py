@@ -311,3 +311,31 @@ def test_shared_memory_limits_are_compile_time_constants():
     assert [c[0] for c in calls] == ["common.cuh"] and "BYTES" in calls[0][1]
     with open(os.path.join(src, "common.cuh")) as f:
         assert re.search(r"template <int BYTES, class K>\s*cudaError_t set\(", f.read())
+
+
+def test_bench_headline_fits_a_log_tail():
+    """bench.py's standard output is one line of the headline figures, below 2,000 characters whatever the report holds."""
+    import json
+    import bench
+    f = 1234567.891234567
+    phases = {p: f for p in ("sample", "forward", "local_energy", "stats", "sr_solve", "update")}
+    form = dict(phases, vmc_steps_per_s=f)
+    summary = {"mixed": form, "plain_fp32": form, "roofline": {"x": "y" * 900}}
+    line = {"metric": bench.METRIC, "value": f, "unit": "samples/s", "n_gpus": 1, "steps": 20, "warmup": 5, "ms_per_step": f,
+            "vmc_steps_per_s": f, "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "c64",
+            "data": "synthetic (random-init RBM, random Sz=0 chains)", "config": {"workload": "w" * 400}, "phase_ms": phases,
+            "cg_iterations_mean": f, "energy_mean_last": f, "gpu_launches": 400, "clocks": {"sm_mhz": f, "sm_max_mhz": f, "reasons": []},
+            "e2e": {"value": f, "unit": "samples/s", "h2d_bytes_per_step": 1, "d2h_bytes_per_step": 1, "ms_per_step": f},
+            "forms": {"mixed": dict(phases), "plain_fp32": dict(phases), "mixed_over_plain_steps_per_s": f},
+            "roofline": {"kernel": "k" * 60, "bound": "hbm", "avg_launch_us": f, "achieved": f, "peak": f, "unit": "GB/s", "frac": f,
+                         "detail": "d" * 2000}, "issue_rooflines": {"sample": "s" * 900}, "sr_tiling": {"c": "t" * 1200},
+            "accuracy_matched_fp64": {"per_epoch": ["e" * 400] * 20}, "dense_sr": {"d": "s" * 1500},
+            "other_configs": {n: summary for n in ("tfim16", "j1j2_6x6", "tfim20x20", "tfim_batch64")},
+            "cpu_baseline": {"value": f, "unit": "samples/s", "cores": 16, "kind": "port", "sample": "s" * 300}}
+    text = json.dumps(bench.headline(line))
+    assert len(text) < 2000
+    got = json.loads(text)
+    for k in ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better", "scaling", "vs_baseline",
+              "dtype", "data", "config", "gpu_launches", "clocks", "e2e"):
+        assert k in got
+    assert got["value"] == pytest.approx(f, rel=1e-5) and got["config"] == line["config"]
