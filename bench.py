@@ -952,7 +952,7 @@ def roofline(cfg, nqs, form):
         ir = issue_rooflines(cfg, nqs, {"phase_ms": phases}, None)[dom]
         ir["share_of_timed_region"] = out["share_of_timed_region"]
         ir["timed_cg_iteration"] = timed_cg_iteration(cfg, nqs, form, hbm, tc)
-        return ir
+        return solve_roofline(cfg, nqs, form, hbm, src, tc, ir)
     else:
         n = cfg["chains"] * cfg["samples"]
         b = n * net.nh * (8 if net.is_complex else 4) + n * ((net.ns + 31) // 32) * 4
@@ -960,7 +960,7 @@ def roofline(cfg, nqs, form):
     ach = b / avg_s / 1e9
     out.update({"achieved": ach, "frac": ach / hbm, "algorithmic_bytes_per_launch": int(b), "traffic": tr,
                 "timed_cg_iteration": timed_cg_iteration(cfg, nqs, form, hbm, tc)})
-    return out
+    return solve_roofline(cfg, nqs, form, hbm, src, tc, out)
 
 
 def timed_cg_iteration(cfg, nqs, form, hbm, tc):
@@ -972,7 +972,22 @@ def timed_cg_iteration(cfg, nqs, form, hbm, tc):
         return None
     b = kernel_bytes(cfg, nqs, "sv", tc=tc)
     ach = b / (ms / its / 1e3) / 1e9
-    return {"us": ms / its * 1e3, "algorithmic_bytes": int(b), "achieved": ach, "unit": "GB/s", "frac": ach / hbm}
+    return {"us": ms / its * 1e3, "algorithmic_bytes": int(b), "achieved": ach, "unit": "GB/s", "frac": ach / hbm,
+            "one_launch": form["launches"] < its}          # the chain launches three kernels and more per iteration
+
+
+def solve_roofline(cfg, nqs, form, hbm, src, tc, chain):
+    """The timed steps' solve as one launch, per CG iteration, where it is the longest phase; chain: the roofline of the
+    profiled steps, whose solves are a chain of kernels."""
+    cg = timed_cg_iteration(cfg, nqs, form, hbm, tc)
+    phases = {p: float(np.sum(v)) for p, v in form["phase_ms"].items()}
+    if cg is None or not cg["one_launch"] or max(phases, key=phases.get) != "sr_solve":
+        return chain
+    return {"kernel": "cg_persist_kernel (SR solve as one launch, figures per CG iteration)",
+            "launches_timed": len(form["cg_iters"]), "avg_launch_us": cg["us"],
+            "share_of_timed_region": phases["sr_solve"] / sum(phases.values()), "bound": "hbm", "peak": hbm,
+            "unit": "GB/s", "peak_source": src, "achieved": cg["achieved"], "frac": cg["frac"],
+            "algorithmic_bytes_per_iteration": cg["algorithmic_bytes"], "profiled_chain": chain}
 
 
 # ---------------------------------------------------------------------------------------- CPU (oracle)
