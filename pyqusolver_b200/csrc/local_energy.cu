@@ -124,7 +124,10 @@ QES_D void eloc_moves_block(int kb, int64_t sb, int ns, int nh, int64_t n_sample
 // product's exponent (biased, so that it cannot carry into the sign).
 // Factors, roundings and the order of the sum over the 32 moves are those of the form above, so the energies
 // are bit-identical to it: in a stochastic-reconfiguration step even the last bits of E_loc reach the
-// weights through the near-null directions of S.
+// weights through the near-null directions of S.  Products run at 2^8 times the form above's and are renormalised only
+// once they have left 1 .. 2^16, so that they never lose digits to underflow where that form would not; one that overflows
+// where it need not (a chunk's factors multiply up to 2^112 .. 2^127) comes out as infinite or NaN and is taken again
+// the way of the form above.
 // Bound by the FP32 and integer pipes: 2 multiply-adds and 1 xor per real factor, 8 and 2 per complex one.
 // Measured (B200, 16,384 samples unless stated), the form above / this one: 20x20 TFIM x 1,600 real 3.81 / 1.51 ms
 // (0.57 ms at the FP32 rate), TFIM-100 x 200 real 173 / 88 us, 10x10 x 200 complex 452 / 401 us, 6x6 J1-J2 x 144
@@ -136,8 +139,27 @@ constexpr int ELT_COLS = 8;              // thread columns: 32 moves
 constexpr int ELT_ROWS = 32;             // thread rows
 constexpr int ELT_THREADS = ELT_COLS * ELT_ROWS;
 constexpr uint32_t ELT_EX0 = 1u << 30;   // bias of the exponent field
+constexpr int ELT_UP = 8;                // products carry this power of two
+constexpr float ELT_SCALE = 256.f;       // 2^ELT_UP
 
 QES_D float xor_sign(float t, uint32_t v) { return __uint_as_float(__float_as_uint(t) ^ (v & 0x80000000u)); }
+// the product over all units of move k and one sample (t its row of T), renormalised every ELOC_RENORM units
+QES_D float mul_fixed(float a, float b) { return a * b; }
+QES_D float2 mul_fixed(float2 a, float2 b) {
+  return make_float2(__fmaf_rn(a.x, b.x, -__fmul_rn(a.y, b.y)), __fmaf_rn(a.x, b.y, __fmul_rn(a.y, b.x)));
+}
+template <class T>
+__device__ __noinline__ T eloc_product(int nh, int K, int k, const T* __restrict__ Ct, const T* __restrict__ St,
+                                       const T* __restrict__ t, float g, int* ex_out) {
+  T acc = ScalarTraits<T>::one();
+  int ex = 0;
+  for (int m = 0; m < nh; ++m) {
+    acc = mul_fixed(acc, ratio_factor(Ct[(int64_t)m * K + k], g, t[m], St[(int64_t)m * K + k]));
+    if (m % ELOC_RENORM == ELOC_RENORM - 1) renorm(acc, ex);
+  }
+  *ex_out = ex;
+  return acc;
+}
 // VEC: rows of C, S and T start on 16-byte boundaries every 4 (real) / 2 (complex) elements
 template <class T, int RS, bool VEC>
 __global__ void __launch_bounds__(ELT_THREADS, ScalarTraits<T>::is_complex ? 3 : 2) eloc_tile_kernel(
@@ -226,7 +248,7 @@ __global__ void __launch_bounds__(ELT_THREADS, ScalarTraits<T>::is_complex ? 3 :
       const bool ok = kval && s < n_samples;
       const uint32_t* w = bits + (ok ? s : 0) * nw;
       const uint32_t bi = bit_of(w, i), bj = bit_of(w, j);
-      v[a][q] = (bi << 31) | ELT_EX0;                                // g = -sigma_i: negative for spin up
+      v[a][q] = (bi << 31) | (ELT_EX0 - ELT_UP);                     // g = -sigma_i: negative for spin up
       const bool on = ok && (kind == QES_MOVE_FLIP1 || ((kind == QES_MOVE_PAIR_ANTI) == (bi != bj)));
       act |= (on ? 1u : 0u) << (a * RS + q);
     }
@@ -236,7 +258,7 @@ __global__ void __launch_bounds__(ELT_THREADS, ScalarTraits<T>::is_complex ? 3 :
   for (int a = 0; a < ELT_K; ++a)
 #pragma unroll
     for (int q = 0; q < RS; ++q) {
-      accr[a][q] = 1.f;
+      accr[a][q] = ELT_SCALE;
       acci[a][q] = 0.f;
     }
   store_cs(0);
@@ -287,15 +309,15 @@ __global__ void __launch_bounds__(ELT_THREADS, ScalarTraits<T>::is_complex ? 3 :
         }
       }
     }
-    // power-of-two renormalisation (exact) of a thread whose products have left 2^-7 .. 2^9: most never do.
-    // An exponent e in [120, 135] has e + 8 = 1000xxxx in binary.
+    // power-of-two renormalisation (exact) of a thread whose products have left 1 .. 2^16: most never do.
+    // An exponent e in [127, 142] has e + 1 = 1000xxxx in binary.
     uint32_t far = 0;
 #pragma unroll
     for (int a = 0; a < ELT_K; ++a)
 #pragma unroll
       for (int q = 0; q < RS; ++q) {
         const float m = CPLX ? fmaxf(fabsf(accr[a][q]), fabsf(acci[a][q])) : accr[a][q];
-        far |= (__float_as_uint(m) + (8u << 23)) ^ 0x40000000u;
+        far |= (__float_as_uint(m) + (1u << 23)) ^ 0x40000000u;
       }
     if (far & 0x78000000u) {
 #pragma unroll
@@ -306,12 +328,13 @@ __global__ void __launch_bounds__(ELT_THREADS, ScalarTraits<T>::is_complex ? 3 :
           if constexpr (CPLX) {
             float2 z = make_float2(accr[a][q], acci[a][q]);
             renorm(z, ex);
-            accr[a][q] = z.x;
-            acci[a][q] = z.y;
+            accr[a][q] = ELT_SCALE * z.x;
+            acci[a][q] = ELT_SCALE * z.y;
           } else {
             renorm(accr[a][q], ex);
+            accr[a][q] *= ELT_SCALE;
           }
-          v[a][q] += (uint32_t)ex;                                   // |sum| < 2^30: no carry into the sign bit
+          v[a][q] += (uint32_t)(ex - ELT_UP);                        // (a zero or infinity: not read)  |sum| < 2^30: no carry into the sign bit
         }
     }
     if (ch + 1 < nchunk) {
@@ -343,14 +366,18 @@ __global__ void __launch_bounds__(ELT_THREADS, ScalarTraits<T>::is_complex ? 3 :
         const float sig = -g;
         const float2 coef = make_float2(cf.x + sig * cf.z, cf.y + sig * cf.w);
         const float2 z = to_c(scal(2.f * g, Ak));
+        const float size = CPLX ? fabsf(accr[a][q]) + fabsf(acci[a][q]) : fabsf(accr[a][q]);
+        const bool again = !(size > 0.f && size <= 3.402823466e38f);
         if constexpr (CPLX) {
           float2 acc = make_float2(accr[a][q], acci[a][q]);
+          if (again) acc = eloc_product(nh, K, k, Ct, St, tanh_theta + (s0 + ELT_ROWS * q + row) * nh, g, &ex);
           renorm(acc, ex);
           const float lx = __fmul_rn(0.69314718055994531f, (float)ex);
           const float2 x = expx(make_float2(__fadd_rn(z.x, lx), z.y));
           e = coef * (x * acc);
         } else {
           float acc = accr[a][q];
+          if (again) acc = eloc_product(nh, K, k, Ct, St, tanh_theta + (s0 + ELT_ROWS * q + row) * nh, g, &ex);
           renorm(acc, ex);
           const float lx = __fmul_rn(0.69314718055994531f, (float)ex);
           const float m = expf(__fadd_rn(z.x, lx)) * acc;

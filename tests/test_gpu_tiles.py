@@ -144,3 +144,60 @@ def test_logpsi_vjp_of_infinities(value):
     ok = ref.isfinite()
     assert (out[ok] - ref[ok]).abs().max() <= 1e-6 * ref[ok].abs().max() if ok.any() else True
     assert torch.equal(out[ref.isinf()], ref[ref.isinf()])
+
+
+# flip of site 0: the first 16 factors multiply to 2^8.5, the next 16 to 2^grow; the visible bias brings the ratio back into range.  One to
+# four samples per thread.
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("n", [40, 3000, 30000])
+@pytest.mark.parametrize("grow", [100.0, 115.0, 121.6])
+def test_local_energy_of_products_near_the_float_range(cplx, n, grow):
+    ns, nh = 33, 32
+    model = qb.TransverseFieldIsing(qb.SquareLattice(1, ns), j=1.0, hx=0.7, hz=0.0)
+    rng = np.random.default_rng(int(grow))
+    W = 0.01 * rng.normal(size=(ns, nh))
+    W[0, :16], W[0, 16:] = 0.5 * 8.5 / 16 * np.log(2), 0.5 * grow / 16 * np.log(2)
+    a = np.zeros(ns)
+    a[0] = -30.0 * np.log(2)
+    flat = torch.as_tensor(np.concatenate([a, np.full(nh, 80.0), W.reshape(-1)])).cuda()
+    flat = flat.to(torch.complex64 if cplx else torch.float32)
+    st = np.where(rng.random((n, ns)) < 0.5, 0.5, -0.5)
+    st[:, 0] = -0.5
+    bits = dv.pack_states(st)
+    tn = torch.ones((n, nh), dtype=flat.dtype, device="cuda")                 # tanh(80 + ...) in float32
+    h = dv.DeviceHamiltonian(model.lower())
+    tables = dv.move_tables(flat, ns, nh, h.move_i, h.move_j, h.move_kind, move_major=False)
+    e = dv.local_energy(flat, ns, nh, bits, tn, h, tables).cpu().numpy()
+    # with tanh = 1 the ratio of a flip is exp(-2 sigma (a + sum_m W_m)), from the float32 parameters; site 0's is 2^48 and
+    # more, beside which the other terms vanish
+    f = flat.real.double().cpu().numpy()
+    ref = float(h.move_coef[0]) * np.exp(2.0 * (f[0] + f[ns + nh:ns + 2 * nh].sum()))
+    # 32 factors, each rounded once from tables with a relative error of up to (1 + 2 W) 2^-23, W <= 2.8
+    assert np.all(np.abs(e - ref) <= 32 * 7 * 2.0 ** -23 * abs(ref)), (e[:4], ref)
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan])
+def test_local_energy_and_forward_of_infinities(cplx, value):
+    """An infinity or a NaN in one sample's T (one bias) reaches that sample (that unit) alone."""
+    ns, nh, n = 33, 40, 300
+    net, st, bits, _ = _problem(cplx, ns, nh, n, 0.1)
+    model = qb.TransverseFieldIsing(qb.SquareLattice(1, ns), j=1.0, hx=0.7, hz=0.0)
+    _, tn, _ = dv.rbm_forward(net.flat, ns, nh, bits, logpsi=False)
+    h = dv.DeviceHamiltonian(model.lower())
+    tables = dv.move_tables(net.flat, ns, nh, h.move_i, h.move_j, h.move_kind, move_major=False)
+    ref = dv.local_energy(net.flat, ns, nh, bits, tn, h, tables)
+    bad = tn.clone()
+    bad[77, 20] = value
+    e = dv.local_energy(net.flat, ns, nh, bits, bad, h, tables)
+    others = torch.arange(n, device="cuda") != 77
+    assert torch.equal(e[others], ref[others]) and not bool(e[77].isfinite())
+    flat = net.flat.clone()
+    flat[ns + 20] = value
+    _, t2, lp = dv.rbm_forward(flat, ns, nh, bits)
+    units = torch.arange(nh, device="cuda") != 20
+    assert torch.equal(t2[:, units], tn[:, units])
+    if np.isnan(value):
+        assert bool(t2[:, 20].isnan().all()) and bool(lp.isnan().all())
+    elif not cplx:
+        assert bool((t2[:, 20] == np.sign(value)).all()) and bool((lp == np.inf).all())
