@@ -344,6 +344,36 @@ __global__ void __launch_bounds__(ELT_THREADS, ScalarTraits<T>::is_complex ? 3 :
     __syncthreads();
   }
 
+  // products that came out as zero, infinite or NaN
+  bool again = false;
+#pragma unroll
+  for (int a = 0; a < ELT_K; ++a)
+#pragma unroll
+    for (int q = 0; q < RS; ++q) {
+      const float size = CPLX ? fabsf(accr[a][q]) + fabsf(acci[a][q]) : fabsf(accr[a][q]);
+      again |= !(size > 0.f && size <= 3.402823466e38f);
+    }
+  if (again) {
+#pragma unroll
+    for (int a = 0; a < ELT_K; ++a)
+#pragma unroll
+      for (int q = 0; q < RS; ++q) {
+        const float size = CPLX ? fabsf(accr[a][q]) + fabsf(acci[a][q]) : fabsf(accr[a][q]);
+        if (((act >> (a * RS + q)) & 1u) && !(size > 0.f && size <= 3.402823466e38f)) {
+          int ex = 0;
+          const T p = eloc_product(nh, K, k0 + ELT_K * col + a, Ct, St, tanh_theta + (s0 + ELT_ROWS * q + row) * nh,
+                                   (v[a][q] >> 31) ? -1.f : 1.f, &ex);
+          if constexpr (CPLX) {
+            accr[a][q] = p.x;
+            acci[a][q] = p.y;
+          } else {
+            accr[a][q] = p;
+          }
+          v[a][q] = (v[a][q] & 0x80000000u) | (ELT_EX0 + (uint32_t)ex);
+        }
+      }
+  }
+
   // contribution = coef * exp(g*2*A + ex*ln2) * acc   (g = -sigma_i), summed over the 32 moves as a warp
   // would by xor shuffles: move distances 16, 8, 4 (thread columns), then 2 and 1 (a thread's own moves)
   float2 sum[ELT_K];
@@ -366,18 +396,14 @@ __global__ void __launch_bounds__(ELT_THREADS, ScalarTraits<T>::is_complex ? 3 :
         const float sig = -g;
         const float2 coef = make_float2(cf.x + sig * cf.z, cf.y + sig * cf.w);
         const float2 z = to_c(scal(2.f * g, Ak));
-        const float size = CPLX ? fabsf(accr[a][q]) + fabsf(acci[a][q]) : fabsf(accr[a][q]);
-        const bool again = !(size > 0.f && size <= 3.402823466e38f);
         if constexpr (CPLX) {
           float2 acc = make_float2(accr[a][q], acci[a][q]);
-          if (again) acc = eloc_product(nh, K, k, Ct, St, tanh_theta + (s0 + ELT_ROWS * q + row) * nh, g, &ex);
           renorm(acc, ex);
           const float lx = __fmul_rn(0.69314718055994531f, (float)ex);
           const float2 x = expx(make_float2(__fadd_rn(z.x, lx), z.y));
           e = coef * (x * acc);
         } else {
           float acc = accr[a][q];
-          if (again) acc = eloc_product(nh, K, k, Ct, St, tanh_theta + (s0 + ELT_ROWS * q + row) * nh, g, &ex);
           renorm(acc, ex);
           const float lx = __fmul_rn(0.69314718055994531f, (float)ex);
           const float m = expf(__fadd_rn(z.x, lx)) * acc;
