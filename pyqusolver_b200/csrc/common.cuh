@@ -128,13 +128,13 @@ QES_D float2 mulx(float2 a, float2 b) { return a * b; }
 QES_D float addx(float a, float b) { return a + b; }
 QES_D float2 addx(float2 a, float2 b) { return a + b; }
 
-// Power-of-two renormalisation of a running product: keeps |acc| in [1,2)
+// Power-of-two renormalisation of a running product: keeps |acc| in [1,2) ([2,4) from 2^127 on)
 // and moves the binary exponent into an integer so that a product over
 // thousands of hidden units can neither overflow nor underflow.
 QES_D void renorm(float& acc, int& ex) {
   const float m = fabsf(acc);
   if (m > 0.f && isfinite(m)) {
-    const int e = ((__float_as_int(m) >> 23) & 0xff) - 127;
+    const int e = min(((__float_as_int(m) >> 23) & 0xff) - 127, 126);     // 2^-127 has no normal float
     acc *= __int_as_float((127 - e) << 23);
     ex += e;
   }
@@ -142,7 +142,7 @@ QES_D void renorm(float& acc, int& ex) {
 QES_D void renorm(float2& acc, int& ex) {
   const float m = fmaxf(fabsf(acc.x), fabsf(acc.y));
   if (m > 0.f && isfinite(m)) {
-    const int e = ((__float_as_int(m) >> 23) & 0xff) - 127;
+    const int e = min(((__float_as_int(m) >> 23) & 0xff) - 127, 126);     // 2^-127 has no normal float
     const float sc = __int_as_float((127 - e) << 23);
     acc.x *= sc; acc.y *= sc;
     ex += e;

@@ -150,7 +150,7 @@ def test_logpsi_vjp_of_infinities(value):
 # four samples per thread.
 @pytest.mark.parametrize("cplx", [False, True])
 @pytest.mark.parametrize("n", [40, 3000, 30000])
-@pytest.mark.parametrize("grow", [100.0, 115.0, 121.6])
+@pytest.mark.parametrize("grow", [100.0, 115.0, 121.6, 126.6])
 def test_local_energy_of_products_near_the_float_range(cplx, n, grow):
     ns, nh = 33, 32
     model = qb.TransverseFieldIsing(qb.SquareLattice(1, ns), j=1.0, hx=0.7, hz=0.0)
