@@ -570,14 +570,19 @@ extern "C" int qes_rbm_log_derivatives(int dtype, int ns, int nh, int64_t n_samp
   QES_ARG_CHECK(ldo >= P, "qes_rbm_log_derivatives: ldo < P");
   if (n_samples == 0) return QES_OK;
   QES_ARG_CHECK(bits && tanh_theta && O_out, "qes_rbm_log_derivatives: null pointer");
-  QES_ARG_CHECK(n_samples <= 0x7fffffff, "qes_rbm_log_derivatives: too many samples");
-  if (dtype == QES_DTYPE_F32)
-    log_derivatives_kernel<float><<<(unsigned)n_samples, 32 * LD_WARPS, 0, (cudaStream_t)stream>>>(
-        ns, nh, n_samples, bits, (const float*)tanh_theta, (float*)O_out, ldo);
-  else
-    log_derivatives_kernel<float2><<<(unsigned)n_samples, 32 * LD_WARPS, 0, (cudaStream_t)stream>>>(
-        ns, nh, n_samples, bits, (const float2*)tanh_theta, (float2*)O_out, ldo);
-  QES_LAUNCH_CHECK();
+  // a block per row: parts of 2^30 rows, below the limit of a grid's x
+  constexpr int64_t part = 1ll << 30;
+  const int nw = n_words(ns);
+  for (int64_t r0 = 0; r0 < n_samples; r0 += part) {
+    const int64_t nr = std::min(part, n_samples - r0);
+    if (dtype == QES_DTYPE_F32)
+      log_derivatives_kernel<float><<<(unsigned)nr, 32 * LD_WARPS, 0, (cudaStream_t)stream>>>(
+          ns, nh, nr, bits + r0 * nw, (const float*)tanh_theta + r0 * nh, (float*)O_out + r0 * ldo, ldo);
+    else
+      log_derivatives_kernel<float2><<<(unsigned)nr, 32 * LD_WARPS, 0, (cudaStream_t)stream>>>(
+          ns, nh, nr, bits + r0 * nw, (const float2*)tanh_theta + r0 * nh, (float2*)O_out + r0 * ldo, ldo);
+    QES_LAUNCH_CHECK();
+  }
   return QES_OK;
 }
 

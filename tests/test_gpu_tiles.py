@@ -201,3 +201,24 @@ def test_local_energy_and_forward_of_infinities(cplx, value):
         assert bool(t2[:, 20].isnan().all()) and bool(lp.isnan().all())
     elif not cplx:
         assert bool((t2[:, 20] == np.sign(value)).all()) and bool((lp == np.inf).all())
+
+
+def test_log_derivative_rows_past_a_grid():
+    """More rows than one grid holds (2^31 - 1): 43 GB for the smallest network."""
+    n = 2 ** 31 + 5
+    bits = torch.zeros((n, 1), dtype=torch.int32, device="cuda")
+    tn = torch.full((n, 1), 0.25, dtype=torch.float32, device="cuda")
+    probe = [0, 2 ** 30 - 1, 2 ** 30, 2 ** 31 - 2, 2 ** 31 - 1, 2 ** 31, n - 1]
+    for k, r in enumerate(probe):
+        bits[r] = k % 2
+        tn[r] = 0.5 + k
+    flat = torch.zeros(3, dtype=torch.float32, device="cuda")
+    O = torch.full((n, 3), 7.0, dtype=torch.float32, device="cuda")
+    dv.log_derivatives(flat, 1, 1, bits, tn, out=O)
+    for k, r in enumerate(probe):
+        sg = 1.0 if k % 2 else -1.0
+        assert O[r].tolist() == [sg, 0.5 + k, sg * (0.5 + k)]
+    for r0 in range(0, n, 2 ** 29):                                            # every row is written
+        assert not bool((O[r0:r0 + 2 ** 29, 0] == 7.0).any())
+    del O, tn, bits
+    torch.cuda.empty_cache()
