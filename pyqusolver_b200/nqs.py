@@ -23,7 +23,7 @@ from typing import Any, List, Optional
 import numpy as np
 import torch
 
-from . import device as dv
+from . import _lib, device as dv
 from .hamiltonian import SpinHamiltonian
 from .rbm import RBM
 from .sampler import VMCSampler
@@ -498,13 +498,19 @@ class NQS:
         if status is not None:
             parts.append(status.to(torch.float64))
         report = torch.cat(parts)
-        before = getattr(tdvp, "_solution", None)
-        x = tdvp.solve(net, bits, tn, eloc, probs=probs)
+        kept = {k: getattr(tdvp, k) for k in ("_solution", "last_info") if hasattr(tdvp, k)}
+        failed = None
+        try:
+            x = tdvp.solve(net, bits, tn, eloc, probs=probs)
+        except _lib.QESError as e:                              # of a forward that failed, or its own
+            failed = e
         s = report.cpu().numpy()
-        if status is not None and s[7] != 0.0:                  # no update, and no start for the next solve, from this
-            if hasattr(tdvp, "_solution"):
-                tdvp._solution = before
+        if status is not None and s[7] != 0.0:                  # no update, and nothing for the next solve, from this
+            for k, v in kept.items():
+                setattr(tdvp, k, v)
             dv.check_forward_status(int(s[7]))
+        if failed is not None:
+            raise failed
         dv.param_update(net.flat, net.master, x, lr)
         net.bump()
         return {"mean": complex(s[0], s[1]), "var": float(s[2]), "std": float(s[3]), "acceptance": float(s[6]),

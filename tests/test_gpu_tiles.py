@@ -222,3 +222,27 @@ def test_log_derivative_rows_past_a_grid():
         assert not bool((O[r0:r0 + 2 ** 29, 0] == 7.0).any())
     del O, tn, bits
     torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("forward_failed", [True, False])
+def test_a_failed_forward_is_reported_before_what_the_solve_makes_of_it(monkeypatch, forward_failed):
+    model = qb.TransverseFieldIsing(qb.SquareLattice(1, 8), j=1.0, hx=1.0, hz=0.0)
+    nqs = qb.NQS("rbm", model, alpha=1.0, dtype="float32", seed=1, s_numchains=64, s_numsamples=4)
+    tdvp = TDVP(rhs_prefactor=-1.0, sr_diag_shift=1e-2)
+    nqs.train_step(lr=0.01, tdvp=tdvp)
+    weights, info = nqs.net.flat.clone(), tdvp.last_info
+    real = dv.rbm_tanh_nowait
+    status = torch.full((1,), int(forward_failed), dtype=torch.int32, device="cuda")
+    monkeypatch.setattr(dv, "rbm_tanh_nowait", lambda *a: (real(*a)[0], status))
+
+    def solve(*a, **k):
+        tdvp.last_info = {"iterations": -1}
+        raise _lib.QESError(_lib.QES_ERR_SIZE, "not positive definite")
+
+    monkeypatch.setattr(tdvp, "solve", solve)
+    with pytest.raises(_lib.QESError) as err:
+        nqs.train_step(lr=0.01, tdvp=tdvp)
+    assert err.value.code == (_lib.QES_ERR_TIMEOUT if forward_failed else _lib.QES_ERR_SIZE)
+    assert torch.equal(nqs.net.flat, weights)
+    if forward_failed:
+        assert tdvp.last_info is info
