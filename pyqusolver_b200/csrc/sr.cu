@@ -3586,7 +3586,8 @@ struct BatchSRWork {
   unsigned int* n_done; // [1] (+pad)
   float2* w;            // [n_samples_total]
   void* partial;        // [sr_part_total] of T
-  void *r, *p, *Ap, *pf; // [n_params_total] of V each (pf: p in float32)
+  void *r, *p;          // [n_params_total] of V each
+  void* pf;             // [n_params_total] of T: p in float32
 };
 
 static size_t batch_sr_layout(int dtype, int n_inst, int64_t n_params_total, int64_t n_samples_total,
@@ -3603,8 +3604,7 @@ static size_t batch_sr_layout(int dtype, int n_inst, int64_t n_params_total, int
   W.partial = take((size_t)sr_part_total * ts);
   W.r = take((size_t)n_params_total * vs);
   W.p = take((size_t)n_params_total * vs);
-  W.Ap = take((size_t)n_params_total * vs);
-  W.pf = take((size_t)n_params_total * vs);
+  W.pf = take((size_t)n_params_total * ts);
   if (L) *L = W;
   return off;
 }

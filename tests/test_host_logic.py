@@ -339,3 +339,15 @@ def test_bench_headline_fits_a_log_tail():
               "dtype", "data", "config", "gpu_launches", "clocks", "e2e"):
         assert k in got
     assert got["value"] == pytest.approx(f, rel=1e-5) and got["config"] == line["config"]
+
+
+@pytest.mark.parametrize("dtype,ts", [(_lib.DTYPE_F32, 4), (_lib.DTYPE_C64, 8)])
+def test_batched_workspace_holds_what_the_solve_uses(dtype, ts):
+    """Scalars, w, the partials, two vectors in float64 and one in float32 (p for the matvec), each rounded up to 256 bytes."""
+    lib = _lib.load()
+    nb = ctypes.c_size_t(0)
+    n_inst, P, n, part = 3, 12345, 6789, 45678
+    assert lib.qes_batch_sr_workspace_bytes(dtype, n_inst, P, n, part, ctypes.byref(nb)) == 0
+    up = lambda b: (b + 255) // 256 * 256
+    fixed = up(n * 8) + up(part * ts) + 2 * up(P * 2 * ts) + up(P * ts)
+    assert fixed < nb.value <= fixed + up(n_inst * 16 * 8) + 256
