@@ -86,7 +86,8 @@ int qes_rbm_move_tables(int dtype, int ns, int nh, const void* a, const void* W,
 
 /* ------------------------------------------------------------------------ */
 /* RBM forward on a batch of packed configurations: theta = W^T sigma + b,
- * tanh(theta) and log psi.  Any output pointer may be NULL.
+ * tanh(theta) and log psi.  Any output pointer may be NULL.  Up to 24,576
+ * sites (QES_ERR_ARG beyond).
  * Replaces the RBM apply (general_python net_rbm) as driven by
  * QES/Solver/MonteCarlo/vmc.py:1113-1164 (_batched_network_apply,
  * _init_logprobas_jax) and QES/NQS/nqs.py:1257-1280.                        */

@@ -260,6 +260,7 @@ extern "C" int qes_rbm_move_tables(int dtype, int ns, int nh, const void* a, con
 // Measured (B200), the one-thread-per-unit form / this one: 16,384 samples of 20x20 x 1,600 real, tanh 2.41 / 0.62 ms,
 // log psi 2.40 / 0.82 ms (0.28 ms at the FP32 rate; 0.81 / 0.83 ms with single-buffered slices), of 10x10 x 200
 // complex, tanh 184 / 86 us, log psi 166 / 134 us; 4,096 samples of 16 x 32 real, 8.7 / 4.1 us.
+constexpr int FWD_MAX_SITES = 24576;     // the entry's documented range, not a limit of the kernel
 constexpr int FWD_SB = 16;               // samples per block of the batched form (RS = 2)
 constexpr int FWD_TX = 32, FWD_TY = 8;
 constexpr int FWD_THREADS = FWD_TX * FWD_TY;
@@ -507,8 +508,7 @@ extern "C" int qes_rbm_forward(int dtype, int ns, int nh, int64_t n_samples, con
   QES_ARG_CHECK(dtype == QES_DTYPE_F32 || dtype == QES_DTYPE_C64, "qes_rbm_forward: bad dtype");
   QES_ARG_CHECK(bits && a && b && W, "qes_rbm_forward: null input");
   if (n_samples == 0) return QES_OK;
-  const int nw = n_words(ns);
-  QES_ARG_CHECK((size_t)FWD_SB * nw * sizeof(uint32_t) <= 48 * 1024, "qes_rbm_forward: ns too large");
+  QES_ARG_CHECK(ns <= FWD_MAX_SITES, "qes_rbm_forward: ns too large");
   if (dtype == QES_DTYPE_F32)
     return launch_forward<float>(ns, nh, n_samples, bits, (const float*)a, (const float*)b, (const float*)W,
                                  (float*)theta_out, (float*)tanh_out, (float*)logpsi_out, (cudaStream_t)stream);
