@@ -509,6 +509,31 @@ def _persistent_problem(cplx, ns, nh, n, seed=21):
     return net, bits, tn, torch.as_tensor(np.asarray(e, dtype=np.complex64)).cuda()
 
 
+# the largest operands: two stages and all 512 accumulator columns (100 x 200), an accumulator in two MMAs with one
+# k-step of samples (63 x 450), all 127 sites; both exchanges with collectors
+@pytest.mark.parametrize("cplx,ns,nh,n", [(True, 100, 200, 16384), (False, 63, 450, 1000), (True, 127, 100, 9000)])
+def test_persistent_cg_of_the_largest_operands(cplx, ns, nh, n):
+    """The one-launch solve against the kernel chain's on shapes too large for a formed matrix: the backward error in the
+    float64 form of S.  Both round the operands of S v to 16 bits of significand and stop by the same rule (which adds
+    1e-8), so that the errors differ by the order of sums and by where the mean is taken out: a factor of four."""
+    net, bits, tn, eloc = _persistent_problem(cplx, ns, nh, n)
+    kw = dict(shift=1e-2, rtol=1e-8, maxiter=400, true_residual=False)
+    before = _lib.launch_count(reset=False)
+    x, info = dv.sr_solve_cg(net.flat, ns, nh, bits, tn, eloc, **kw)
+    assert _lib.launch_count(reset=False) - before == 1
+    try:
+        _lib.call("qes_sr_set_one_launch", 0, None)
+        xc, _ = dv.sr_solve_cg(net.flat, ns, nh, bits, tn, eloc, **kw)
+        _lib.set_sr_impl(3)
+        F = dv.sr_force(net.flat, ns, nh, bits, tn, eloc)
+        err = [float((F + dv.sr_matvec(net.flat, ns, nh, bits, tn, v, shift=1e-2)).norm() / F.norm()) for v in (x, xc)]
+    finally:
+        _lib.set_sr_impl(0)
+        _lib.call("qes_sr_set_one_launch", 1, None)
+    assert abs(info["rhs_norm"] - float(F.norm())) <= 1e-4 * float(F.norm())
+    assert err[0] <= 4 * err[1] + 2e-8, err
+
+
 @pytest.mark.parametrize("cplx", [False, True])
 def test_persistent_cg_stops_as_the_rule_says(cplx):
     """No iteration for a zero force or maxiter = 0; a system that converges at once (a shift far above S:
