@@ -9,13 +9,18 @@
 //   Sigma^T Q, Q_sm = conj(t_sm) u_s                   A = Sigma^T from TMEM, B = Q built in shared
 //                                                      memory from the resident T (BF16 hi/lo)
 //   one partial P-vector per CTA, summed in float64 by the CTAs that own the entries.
-// What bounds an iteration: the three grid-wide exchanges (the partials, the dot products, the next
-// direction; 1.2-1.5 us each on 148 CTAs, 0.6-0.8 us on up to 32) and, from about 60 sites x 190 units on, the
+// What bounds an iteration: the latency of its chain of steps and, from about 60 sites x 190 units on, the
 // L2 traffic: V is read by every CTA and every CTA writes a whole partial (heis10x10: 26 + 24 + 24 MB).
-// Measured per CG iteration against the chain of four kernels (sr.cu, sr_tc.cu), which took 3-5 us per
-// kernel boundary: 16 sites x 16 units, 1,024 samples 24.4 -> 11.5 us; 63 x 126, 1,000 samples 27.4 -> 14.3;
-// 6x6 x 144 complex, 8,192 samples 30.5 -> 19.1; 63 x 189 complex, 5,000 samples 31.8 -> 23.8; 10x10 x 200
-// complex, 16,384 samples 41.4 -> 34.0 us.
+// Clocks per iteration on CTA 0 (about 1.9 GHz), of the sections in order, for 16 sites x 16 units, 1,024 samples (32 CTAs)
+// and for 63 x 189 complex, 5,000 samples (105 CTAs): direction exchange 2,600 / 4,300; first contraction with sigma . v_a
+// 2,400 / 4,900; its epilogue 600 / 2,900; u 400 / 800; Q 1,200 / 4,000; g_a and the rest of the second contraction
+// 1,200 / 1,700; partials out 600 / 6,700; their barrier 2,900 / 3,000; their sum 3,000 / 7,200; the dot products
+// 3,100 / 8,500; vectors and the next operand 800 / 1,300.  The exchanges include the wait for the last CTA.
+// Measured per CG iteration (250 against 50 iterations of a solve) against the chain of kernels (sr.cu, sr_tc.cu): 16 sites x 16
+// units, 1,024 samples 17.9 -> 9.8 us; 63 x 126, 1,000 samples 24.5 -> 12.6; 6x6 x 144 complex, 8,192 samples
+// 28.2 -> 17.7; 63 x 189 complex, 5,000 samples 30.7 -> 23.3; 10x10 x 200 complex, 16,384 samples 41.7 -> 33.6 us.
+// The last one is the largest that fits: it takes all 512 TMEM columns (NZ + Kz / 2 + R / 2) and 232,344 bytes of
+// shared memory.  Beyond it the chain runs: 208 units 42.4 us, 240 units 64, 18,944 samples 59, 11x11 x 242 units 91.
 //
 // Two exchanges of the textbook iteration are not needed:
 //  * the mean of w = O p: O-bar . p is known before w is (O-bar once per solve, then the recurrences of r and
@@ -930,9 +935,12 @@ bool pcg_plan(int dtype, int ns, int nh, int64_t n, PcgDims* out) {
   if (d.NZ > 512) return false;
   int64_t R = (n + sms - 1) / sms;
   R = (R + 15) / 16 * 16;
-  // small batches on at most kDirect CTAs, whose exchanges take half the time, while a CTA's own share (R x NZ
-  // operand entries, about 0.3 clocks each) stays below what that saves: 16 x 16 units, 1,024 samples on 64 /
-  // 32 CTAs 17.1 / 12.6 us per iteration
+  // small batches on at most kDirect CTAs, whose exchanges are shorter, while a CTA's own share (R x NZ operand entries)
+  // is small.  us per iteration on at most kDirect / on all CTAs: 16 x 16, 1,024 samples 9.7 / 11.3; 60 x 256, 1,024
+  // (R NZ = 8,192) 14.8 / 16.2; 63 x 128, 2,048 (8,192) 13.3 / 14.9; 36 x 64, 4,096 (8,192) 13.0 / 13.5; 36 x 32
+  // complex, 4,096 (8,192) 13.5 / 13.3.  Above the line the two cross between 12,000 and 25,000: 63 x 240, 2,048 (15,360)
+  // 15.5 / 17.8; 36 x 192, 4,096 (24,576) 15.1 / 15.2; complex 36 x 96, 2,048 (12,288) 13.6 / 14.5, 36 x 96, 4,096
+  // (24,576) 15.4 / 14.9
   const int64_t Rd = ((n + kDirect - 1) / kDirect + 15) / 16 * 16;
   if (Rd <= 128 && Rd * d.NZ <= 8192 && (int64_t)d.NZ * (ns + 1) / 4 + ns <= 128 * kDirect) R = std::max(R, Rd);
   if (R > 128) return false;
