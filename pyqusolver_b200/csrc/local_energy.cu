@@ -129,10 +129,10 @@ QES_D void eloc_moves_block(int kb, int64_t sb, int ns, int nh, int64_t n_sample
 // where it need not (a chunk's factors multiply up to 2^112 .. 2^127) comes out as infinite or NaN and is taken again
 // the way of the form above.
 // Bound by the FP32 and integer pipes: 2 multiply-adds and 1 xor per real factor, 8 and 2 per complex one.
-// Measured (B200, 16,384 samples unless stated), the form above / this one: 20x20 TFIM x 1,600 real 3.81 / 1.51 ms
-// (0.57 ms at the FP32 rate), TFIM-100 x 200 real 173 / 88 us, 10x10 x 200 complex 452 / 401 us, 6x6 J1-J2 x 144
-// complex, 8,192 samples, 139 / 122 us.  Packed f32x2 multiply-adds ran the same (1.53 ms, 425 us); four complex
-// samples per thread at 128 registers 413 us.
+// Measured (B200, 16,384 samples unless stated), the form above / this one: 20x20 TFIM x 1,600 real 3.81 / 1.54 ms
+// (0.57 ms at the FP32 rate), TFIM-100 x 200 real 173 / 88 us, 10x10 x 200 complex 452 / 385 us, 6x6 J1-J2 x 144
+// complex, 8,192 samples, 139 / 122 us.  Packed f32x2 multiply-adds ran the same (1.53 ms against 1.51, 425 us against
+// 401); four complex samples per thread at 128 registers 413 us against 401.
 // ----------------------------------------------------------------------------
 constexpr int ELT_K = 4;                 // moves per thread
 constexpr int ELT_COLS = 8;              // thread columns: 32 moves
@@ -160,8 +160,9 @@ __device__ __noinline__ T eloc_product(int nh, int K, int k, const T* __restrict
   *ex_out = ex;
   return acc;
 }
-// VEC: rows of C, S and T start on 16-byte boundaries every 4 (real) / 2 (complex) elements
-template <class T, int RS, bool VEC>
+// VEC: rows of C, S and T start on 16-byte boundaries every 4 (real) / 2 (complex) elements; TAIL: a last chunk of fewer units
+// is not padded to a whole one
+template <class T, int RS, bool VEC, bool TAIL>
 __global__ void __launch_bounds__(ELT_THREADS, ScalarTraits<T>::is_complex ? 3 : 2) eloc_tile_kernel(
     int ns, int nh, int64_t n_samples, const uint32_t* __restrict__ bits, const T* __restrict__ tanh_theta, int K,
     const int32_t* __restrict__ mi, const int32_t* __restrict__ mj,
@@ -275,9 +276,7 @@ __global__ void __launch_bounds__(ELT_THREADS, ScalarTraits<T>::is_complex ? 3 :
     const float* cb = s_cs + buf * NT * UM * TK + ELT_K * col;
     const float* tb = s_t + (size_t)buf * TS * TW + (size_t)row * TW;
     constexpr int UV = 4 / H;                                        // units per 16-byte load of T
-    // units past nh (only in the last chunk): C = 1, S = 0, t = 0, an exact factor of one
-#pragma unroll
-    for (int u0 = 0; u0 < UM; u0 += UV) {
+    auto units = [&](int u0) {
       float4 t4[RS];
 #pragma unroll
       for (int q = 0; q < RS; ++q) t4[q] = *reinterpret_cast<const float4*>(tb + (size_t)q * ELT_ROWS * TW + H * u0);
@@ -308,6 +307,14 @@ __global__ void __launch_bounds__(ELT_THREADS, ScalarTraits<T>::is_complex ? 3 :
           }
         }
       }
+    };
+    if (!TAIL || nh - ch * UM >= UM) {
+#pragma unroll
+      for (int u0 = 0; u0 < UM; u0 += UV) units(u0);
+    } else {
+      // the last chunk, up to a multiple of UV; units past nh: C = 1, S = 0, t = 0, an exact factor of one
+#pragma unroll 1
+      for (int u0 = 0; u0 < nh - ch * UM; u0 += UV) units(u0);
     }
     // power-of-two renormalisation (exact) of a thread whose products have left 1 .. 2^16: most never do.
     // An exponent e in [127, 142] has e + 1 = 1000xxxx in binary.
@@ -440,9 +447,14 @@ static int launch_eloc_tiles(int ns, int nh, int64_t n, const uint32_t* bits, co
   const uintptr_t al = reinterpret_cast<uintptr_t>(tt) | reinterpret_cast<uintptr_t>(Ct) | reinterpret_cast<uintptr_t>(St);
   const bool vec = nh % E == 0 && K % E == 0 && (al & 15) == 0;
   constexpr size_t smem = eloc_tile_smem<T, RS>();
-  auto kern = vec ? eloc_tile_kernel<T, RS, true> : eloc_tile_kernel<T, RS, false>;
-  static QesSmemAttr attr[2];
-  QES_CUDA_CHECK(attr[vec].set<(int)smem>(kern));
+  // complex only, where a padded unit costs 10 instructions: 82 sites x 4 units, 36,395 samples 62 -> 43 us, 4 x 37 68 -> 60,
+  // 10x10 x 200 396 -> 380.  A real factor costs 2, and the second loop slows the first: 2 x 334 107 -> 111 us
+  constexpr bool C = ScalarTraits<T>::is_complex;
+  const bool tail = C && nh % ELOC_RENORM != 0;
+  auto kern = tail ? (vec ? eloc_tile_kernel<T, RS, true, C> : eloc_tile_kernel<T, RS, false, C>)
+                   : (vec ? eloc_tile_kernel<T, RS, true, false> : eloc_tile_kernel<T, RS, false, false>);
+  static QesSmemAttr attr[4];
+  QES_CUDA_CHECK(attr[2 * tail + vec].set<(int)smem>(kern));
   kern<<<dim3(eloc_kblocks(K), (unsigned)nsb), ELT_THREADS, smem, st>>>(ns, nh, n, bits, tt, K, ham->move_i, ham->move_j,
                                                                        ham->move_kind, (const float4*)ham->move_coef, Ct,
                                                                        St, A, partial);

@@ -69,6 +69,12 @@ def test_local_energy_tiles(lx, ly, model, cplx, nh, n, scale):
     assert np.all(np.isfinite(e))
 
 
+# last chunks of 1 to 15 complex units
+@pytest.mark.parametrize("lx,ly,model,nh,n", [(35, 1, "tfim", 1, 300), (6, 2, "xxz", 14, 9000), (5, 3, "j1j2", 18, 2500), (9, 1, "tfim", 47, 70)])
+def test_local_energy_of_a_short_last_chunk(lx, ly, model, nh, n):
+    test_local_energy_tiles(lx, ly, model, True, nh, n, 0.1)
+
+
 # rows whose W blocks start on and off 16-byte boundaries (odd P, odd nh), fewer elements than one vector
 @pytest.mark.parametrize("cplx,ns,nh,n", [(False, 1, 1, 3), (False, 5, 3, 7), (True, 4, 3, 5), (True, 7, 8, 2),
                                            (False, 33, 130, 4), (True, 20, 41, 9)])
