@@ -3433,7 +3433,7 @@ __global__ void __launch_bounds__(BMM_THREADS, 2) vjp_mma_kernel(int ns, int nh,
   for (int wd = 0; wd < nw; ++wd) {
     T s = ScalarTraits<T>::zero();
 #pragma unroll 8
-    for (int sl = SW * wv; sl < SW * wv + SW; ++sl)
+    for (int sl = SW * wv; sl < min(nc, SW * wv + SW); ++sl)
       s = fma_s(((ws[sl * nw + wd] >> lane) & 1u) ? 1.f : -1.f, us[sl], s);
     if (32 * wd + lane < ns) ga[wv * ns + 32 * wd + lane] = s;
   }

@@ -133,6 +133,12 @@ def test_logpsi_vjp_at_tile_edges(cplx, ns, nh, n):
     assert np.linalg.norm(out - ref) <= 1e-6 * np.linalg.norm(ref)
 
 
+# the last split's samples end within, at and past a warp's share of 64 for g_a
+@pytest.mark.parametrize("cplx,ns,nh,n", [(True, 40, 9, 64), (False, 70, 9, 65), (True, 33, 9, 577), (False, 400, 20, 3)])
+def test_logpsi_vjp_of_few_samples(cplx, ns, nh, n):
+    test_logpsi_vjp_at_tile_edges(cplx, ns, nh, n)
+
+
 # one sample's infinity or NaN, or the largest float, leaves the same entries finite, infinite and NaN as the CUDA-core form
 @pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan, 3.4e38])
 def test_logpsi_vjp_of_infinities(value):
