@@ -522,8 +522,14 @@ extern "C" int qes_rbm_forward(int dtype, int ns, int nh, int64_t n_samples, con
 // One block per sample; its warps take the a and b parts and the W rows (one row = nh consecutive elements
 // sigma_i t_m) in turn, each written as 16-byte vectors between the elements before its first 16-byte boundary
 // and after its last.  No division per element (the flat form divided every index by nh).  Bound by the
-// stores: 4,096 rows of 20,300 complex64 elements (665 MB) 425 -> 121 us, 102 us at the measured copy rate.
+// stores: 4,096 rows of 20,300 complex64 elements (665 MB) 425 -> 121 us, 102 us at the measured copy rate.  Where the samples
+// alone do not fill the chip, several blocks share a sample (LD_BLOCKS in all): 3 rows of 423 sites x 968 units 65 -> 14 us.
 constexpr int LD_WARPS = 8;
+constexpr int LD_BLOCKS = 4 * 148;
+// Units up to which log_derivatives_flat_kernel runs, us of the form above / of the flat one: 100 sites x 12 real, 60,000
+// rows 698 / 125, x 96, 10,208 rows 124 / 118, x 127, 7,735 rows 100 / 119; complex x 12, 38,109 rows 437 / 99, x 96, 5,104 rows
+// 80 / 82, x 127, 3,867 rows 76 / 84
+constexpr int LD_FLAT = 96;
 
 // elements [0, n) of a row segment: dst[k] = f(k)
 template <class T, class F>
@@ -555,12 +561,89 @@ __global__ void __launch_bounds__(32 * LD_WARPS) log_derivatives_kernel(int ns, 
   const uint32_t* w = bits + s * n_words(ns);
   T* row = O + s * ldo;
   const T* t = tanh_theta + s * nh;
-  if (warp == 0) put_row(row, ns, lane, [&](int i) { return scal(sigma_of(w, i), ScalarTraits<T>::one()); });
-  if (warp == 1) put_row(row + ns, nh, lane, [&](int m) { return t[m]; });
-  for (int i = warp; i < ns; i += LD_WARPS) {
-    const float sg = sigma_of(w, i);
-    put_row(row + ns + nh + (int64_t)i * nh, nh, lane, [&](int m) { return scal(sg, t[m]); });
+  if (blockIdx.y == 0) {
+    if (warp == 0) put_row(row, ns, lane, [&](int i) { return scal(sigma_of(w, i), ScalarTraits<T>::one()); });
+    if (warp == 1) put_row(row + ns, nh, lane, [&](int m) { return t[m]; });
   }
+  for (int64_t i = (int64_t)blockIdx.y * LD_WARPS + warp; i < ns; i += LD_WARPS * gridDim.y) {
+    const float sg = sigma_of(w, (int)i);
+    put_row(row + ns + nh + i * nh, nh, lane, [&](int m) { return scal(sg, t[m]); });
+  }
+}
+
+// Narrow layers, whose W rows leave most of a warp without a vector: TPR threads (a warp up to P = 64 vectors, else the
+// block) walk a sample's P elements as one run of 16-byte vectors, with one division per vector.  Bound by the stores from
+// about 12 units on (2.5-4 TB/s).
+template <class T, int TPR>
+__global__ void __launch_bounds__(32 * LD_WARPS) log_derivatives_flat_kernel(int ns, int nh, int64_t n_samples,
+                                                                            const uint32_t* __restrict__ bits,
+                                                                            const T* __restrict__ tanh_theta,
+                                                                            T* __restrict__ O, int64_t ldo) {
+  constexpr int E = 16 / (int)sizeof(T);
+  const int64_t s = (int64_t)blockIdx.x * (32 * LD_WARPS / TPR) + threadIdx.x / TPR;
+  if (s >= n_samples) return;
+  const int lane = threadIdx.x % TPR, P = ns + nh + ns * nh;            // P < 2^31
+  const uint32_t* w = bits + s * n_words(ns);
+  T* row = O + s * ldo;
+  const T* t = tanh_theta + s * nh;
+  auto at = [&](int k) {
+    if (k < ns) return scal(sigma_of(w, k), ScalarTraits<T>::one());
+    if (k < ns + nh) return t[k - ns];
+    const int q = k - ns - nh, i = q / nh;
+    return scal(sigma_of(w, i), t[q - i * nh]);
+  };
+  const int mis = (int)((reinterpret_cast<uintptr_t>(row) & 15) / sizeof(T));
+  const int head = min(P, (E - mis) % E), nv = (P - head) / E, tail = P - head - nv * E;
+  if (blockIdx.y == 0) {
+    if (lane < head) row[lane] = at(lane);
+    if (lane < tail) row[P - tail + lane] = at(P - tail + lane);
+  }
+  float4* v = reinterpret_cast<float4*>(row + head);
+  for (int64_t q = (int64_t)blockIdx.y * TPR + lane; q < nv; q += TPR * gridDim.y) {
+    const int k = head + (int)q * E;
+    T x[E];
+    if (k < ns + nh) {
+#pragma unroll
+      for (int e = 0; e < E; ++e) x[e] = at(k + e);
+    } else {
+      int i = (k - ns - nh) / nh, m = (k - ns - nh) - i * nh;
+      float sg = sigma_of(w, i);
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        x[e] = scal(sg, t[m]);
+        if (++m == nh && e + 1 < E) {                                  // not past the last site
+          m = 0;
+          sg = sigma_of(w, ++i);
+        }
+      }
+    }
+    float4 o;
+    if constexpr (ScalarTraits<T>::is_complex) o = make_float4(x[0].x, x[0].y, x[1].x, x[1].y);
+    else o = make_float4(x[0], x[1], x[2], x[3]);
+    v[q] = o;
+  }
+}
+
+template <class T>
+static int launch_log_derivatives(int ns, int nh, int64_t n, const uint32_t* bits, const T* tt, T* O, int64_t ldo,
+                                  cudaStream_t st) {
+  constexpr int E = 16 / (int)sizeof(T);
+  const int64_t P = (int64_t)ns + nh + (int64_t)ns * nh;
+  const bool flat = nh <= LD_FLAT && P < (1ll << 31);
+  const int tpr = flat && P <= 64 * E ? 32 : 32 * LD_WARPS, rpb = 32 * LD_WARPS / tpr;   // threads per row, rows per block
+  // rows of several blocks where they are too few to fill the chip
+  const int64_t most = flat ? (P / E + tpr - 1) / tpr : (ns + LD_WARPS - 1) / LD_WARPS;
+  // parts of 2^30 rows, below the limit of a grid's x
+  constexpr int64_t part = 1ll << 30;
+  for (int64_t r0 = 0; r0 < n; r0 += part) {
+    const int64_t nr = std::min(part, n - r0), nb = (nr + rpb - 1) / rpb;
+    const dim3 grid((unsigned)nb, (unsigned)std::clamp<int64_t>(LD_BLOCKS / nb, 1, std::clamp<int64_t>(most, 1, 65535)));
+    auto kern = !flat ? log_derivatives_kernel<T> : tpr == 32 ? log_derivatives_flat_kernel<T, 32>
+                                                              : log_derivatives_flat_kernel<T, 32 * LD_WARPS>;
+    kern<<<grid, 32 * LD_WARPS, 0, st>>>(ns, nh, nr, bits + r0 * n_words(ns), tt + r0 * nh, O + r0 * ldo, ldo);
+    QES_LAUNCH_CHECK();
+  }
+  return QES_OK;
 }
 
 extern "C" int qes_rbm_log_derivatives(int dtype, int ns, int nh, int64_t n_samples, const uint32_t* bits,
@@ -570,20 +653,9 @@ extern "C" int qes_rbm_log_derivatives(int dtype, int ns, int nh, int64_t n_samp
   QES_ARG_CHECK(ldo >= P, "qes_rbm_log_derivatives: ldo < P");
   if (n_samples == 0) return QES_OK;
   QES_ARG_CHECK(bits && tanh_theta && O_out, "qes_rbm_log_derivatives: null pointer");
-  // a block per row: parts of 2^30 rows, below the limit of a grid's x
-  constexpr int64_t part = 1ll << 30;
-  const int nw = n_words(ns);
-  for (int64_t r0 = 0; r0 < n_samples; r0 += part) {
-    const int64_t nr = std::min(part, n_samples - r0);
-    if (dtype == QES_DTYPE_F32)
-      log_derivatives_kernel<float><<<(unsigned)nr, 32 * LD_WARPS, 0, (cudaStream_t)stream>>>(
-          ns, nh, nr, bits + r0 * nw, (const float*)tanh_theta + r0 * nh, (float*)O_out + r0 * ldo, ldo);
-    else
-      log_derivatives_kernel<float2><<<(unsigned)nr, 32 * LD_WARPS, 0, (cudaStream_t)stream>>>(
-          ns, nh, nr, bits + r0 * nw, (const float2*)tanh_theta + r0 * nh, (float2*)O_out + r0 * ldo, ldo);
-    QES_LAUNCH_CHECK();
-  }
-  return QES_OK;
+  if (dtype == QES_DTYPE_F32)
+    return launch_log_derivatives<float>(ns, nh, n_samples, bits, (const float*)tanh_theta, (float*)O_out, ldo, (cudaStream_t)stream);
+  return launch_log_derivatives<float2>(ns, nh, n_samples, bits, (const float2*)tanh_theta, (float2*)O_out, ldo, (cudaStream_t)stream);
 }
 
 // ----------------------------------------------------------------------------

@@ -90,6 +90,14 @@ def test_log_derivative_rows(cplx, ns, nh, n):
     assert torch.equal(wide[:, :-3], ref) and bool((wide[:, -3:] == 7.0).all())
 
 
+# narrow W rows as one run per sample (a warp or a block each), either form's last width, several blocks per sample
+@pytest.mark.parametrize("cplx,ns,nh,n", [
+    (False, 15, 15, 700), (False, 16, 15, 61), (True, 10, 9, 1201), (False, 300, 96, 1), (True, 300, 96, 2), (False, 2000, 97, 3),
+    (True, 129, 97, 700), (False, 60, 4, 1300), (True, 2, 1, 5000)])
+def test_log_derivative_rows_of_narrow_layers_and_few_samples(cplx, ns, nh, n):
+    test_log_derivative_rows(cplx, ns, nh, n)
+
+
 @pytest.mark.parametrize("dtype,ns,nh,n", [("float32", 5, 3, 1), ("float32", 63, 126, 700), ("complex64", 33, 40, 129)])
 def test_forward_without_wait_is_the_forward(dtype, ns, nh, n):
     net = RBM((ns,), n_hidden=nh, dtype=dtype, seed=ns, init_scale=0.1)
