@@ -256,15 +256,21 @@ extern "C" int qes_rbm_move_tables(int dtype, int ns, int nh, const void* a, con
 // product exact, so its value does not depend on the tiling.  log psi (LP) does: its terms are added as 256 threads
 // with units t, t + 256, ... would, then 32 at a time by butterflies, then the eight sums in order; a thread
 // holds the sums of its four units of both 128-unit halves.  Bound by FP32 issue.
-// W slices are copied a slice ahead (asynchronous copies into two buffers).
+// W slices are copied a slice ahead (asynchronous copies into two buffers); the last one ends at a multiple of 8 sites.
 // Measured (B200), the one-thread-per-unit form / this one: 16,384 samples of 20x20 x 1,600 real, tanh 2.41 / 0.62 ms,
 // log psi 2.40 / 0.82 ms (0.28 ms at the FP32 rate; 0.81 / 0.83 ms with single-buffered slices), of 10x10 x 200
-// complex, tanh 184 / 86 us, log psi 166 / 134 us; 4,096 samples of 16 x 32 real, 8.7 / 4.1 us.
+// complex, tanh 189 / 85 us, log psi 171 / 121 us; 20,000 samples of 100 x 64 real, 85 / 27 and 88 / 45 us.  Slower than that
+// form: log psi of a handful of sites with tens of thousands of samples (50,814 of 5 x 246 real 50 / 62 us, 39,586 of 2 x 334
+// 43 / 66 us), where a block's start and its sums over the units are most of its time.
 constexpr int FWD_MAX_SITES = 24576;     // the entry's documented range, not a limit of the kernel
 constexpr int FWD_SB = 16;               // samples per block of the batched form (RS = 2)
 constexpr int FWD_TX = 32, FWD_TY = 8;
 constexpr int FWD_THREADS = FWD_TX * FWD_TY;
+// log psi of few sites is the latency of log cosh: two real samples per thread at three blocks per SM up to FWD_FEW sites, us
+// for 20,000 samples against four samples at two blocks: 16 x 32 20 / 25, 32 x 128 24 / 29, 48 x 96 29 / 33, 64 x 128 37 / 37
+constexpr int FWD_FEW = 48, FWD_MINB = 3;
 constexpr int FWD_K = 32;                // sites per staged slice: one spin word
+constexpr int FWD_KS = 8;                // the last slice is padded to a multiple of this
 constexpr int FWD_U = 4 * FWD_TX;        // hidden units per pass
 
 template <class T>
@@ -289,8 +295,9 @@ QES_D float2 shfl_val(float2 v, int l) {
 template <class T, int RS>
 constexpr int fwd_smem() { return 2 * FWD_K * (FWD_U * (int)sizeof(T) + FWD_TY * RS * 4); }
 
-// one block of 8 RS samples starting at row s0; VEC: W rows start on 16-byte boundaries; LP: log psi asked for
-template <class T, int RS, bool VEC, bool LP>
+// one block of 8 RS samples starting at row s0; VEC: W rows start on 16-byte boundaries; LP: log psi asked for; SPREAD: a lane's
+// units 32 apart instead of in a row
+template <class T, int RS, bool VEC, bool LP, bool SPREAD>
 QES_D void rbm_forward_block(uint8_t* smem, int64_t s0, int ns, int nh, int64_t n_samples,
                              const uint32_t* __restrict__ bits, const T* __restrict__ a, const T* __restrict__ b,
                              const T* __restrict__ W, T* __restrict__ theta_out, T* __restrict__ tanh_out,
@@ -300,7 +307,6 @@ QES_D void rbm_forward_block(uint8_t* smem, int64_t s0, int ns, int nh, int64_t 
   float* sg_all = reinterpret_cast<float*>(smem + 2 * FWD_K * FWD_U * sizeof(T));       // [2][FWD_K][TS]
   const int nw = n_words(ns);
   const int tid = threadIdx.x, lane = tid & 31, row = tid >> 5;
-  constexpr bool CPLX = ScalarTraits<T>::is_complex;
   T lsum[LP ? RS : 1][2][4];                  // of the virtual threads 128 h + (unit of c)
 #pragma unroll
   for (int q = 0; q < (LP ? RS : 1); ++q)
@@ -314,6 +320,7 @@ QES_D void rbm_forward_block(uint8_t* smem, int64_t s0, int ns, int nh, int64_t 
   const int nsl = (ns + FWD_K - 1) / FWD_K, total = nsl * ((nh + FWD_U - 1) / FWD_U);
   constexpr int BPT = FWD_K * TS / FWD_THREADS;                               // spins per thread and slice
   const int sl = tid % TS, ib = (tid / TS) * BPT;
+  auto sites = [&](int i0) { return min(FWD_K, (ns - i0 + FWD_KS - 1) / FWD_KS * FWD_KS); };   // of a slice, padded
   auto spin_word = [&](int q) {
     const int i0 = (q % nsl) * FWD_K;
     return (s0 + sl < n_samples) ? bits[(s0 + sl) * nw + (i0 >> 5)] : 0u;
@@ -323,7 +330,7 @@ QES_D void rbm_forward_block(uint8_t* smem, int64_t s0, int ns, int nh, int64_t 
     T* ws = ws_all + buf * FWD_K * FWD_U;
     constexpr int PER = VEC ? 16 / (int)sizeof(T) : 1;
 #pragma unroll 4
-    for (int e = tid; e < FWD_K * FWD_U / PER; e += FWD_THREADS) {
+    for (int e = tid; e < sites(i0) * FWD_U / PER; e += FWD_THREADS) {
       const int ul = (e % (FWD_U / PER)) * PER, il = e / (FWD_U / PER);
       const bool ok = i0 + il < ns && u0 + ul < nh;                           // VEC: nh is a multiple of PER
       cp_async<PER * (int)sizeof(T)>(ws + il * FWD_U + ul, ok ? W + (int64_t)(i0 + il) * nh + u0 + ul : W, ok);
@@ -341,8 +348,8 @@ QES_D void rbm_forward_block(uint8_t* smem, int64_t s0, int ns, int nh, int64_t 
   if (total > 1) next_word = spin_word(1);
   int q_sl = 0;
   for (int u0 = 0; u0 < nh; u0 += FWD_U) {
-    const int m0 = u0 + (CPLX ? 1 : 4) * lane;                // unit c: m0 + c, complex m0 + 32 c
-    constexpr int MC = CPLX ? 32 : 1;
+    const int m0 = u0 + (SPREAD ? 1 : 4) * lane;                // unit c: m0 + c, complex m0 + 32 c
+    constexpr int MC = SPREAD ? 32 : 1;
     T acc[RS][4];
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
@@ -358,12 +365,15 @@ QES_D void rbm_forward_block(uint8_t* smem, int64_t s0, int ns, int nh, int64_t 
         stage(q_sl + 1, buf ^ 1, next_word);
         if (q_sl + 2 < total) next_word = spin_word(q_sl + 2);
       }
-      const T* ws = ws_all + buf * FWD_K * FWD_U + (CPLX ? 1 : 4) * lane;
+      const T* ws = ws_all + buf * FWD_K * FWD_U + (SPREAD ? 1 : 4) * lane;
       const float* sg = sg_all + buf * FWD_K * TS + RS * row;
-#pragma unroll 8
-      for (int il = 0; il < FWD_K; ++il) {
+      const int nk = sites(i0);
+#pragma unroll 1
+      for (int ik = 0; ik < nk; ik += FWD_KS) {
+#pragma unroll
+      for (int il = ik; il < ik + FWD_KS; ++il) {
         T w[4];
-        if constexpr (CPLX) {
+        if constexpr (SPREAD) {
 #pragma unroll
           for (int c = 0; c < 4; ++c) w[c] = ws[il * FWD_U + 32 * c];
         } else {
@@ -386,48 +396,67 @@ QES_D void rbm_forward_block(uint8_t* smem, int64_t s0, int ns, int nh, int64_t 
 #pragma unroll
           for (int c = 0; c < 4; ++c) acc[q][c] = fma_sign(x[q], w[c], acc[q][c]);
       }
+      }
     }
+    // Functions of all four units (theta = 0 past nh), whichever of them count: a lane's chains then overlap
 #pragma unroll
     for (int q = 0; q < RS; ++q) {
       const int64_t s = s0 + RS * row + q;
       if (s < n_samples) {
         const int64_t o = s * nh + m0;
-        if (CPLX || !vec) {
+        T t[4];
+        if (tanh_out) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+            if (!SPREAD || u0 + 32 * c < nh) t[c] = tanhx(acc[q][c]);
+        }
+        if (SPREAD || !vec) {
 #pragma unroll
           for (int c = 0; c < 4; ++c)
             if (m0 + MC * c < nh) {
               if (theta_out) theta_out[o + MC * c] = acc[q][c];
-              if (tanh_out) tanh_out[o + MC * c] = tanhx(acc[q][c]);
+              if (tanh_out) tanh_out[o + MC * c] = t[c];
             }
         } else if (m0 < nh) {                                  // 16-byte vectors of 4 units
           if (theta_out) *reinterpret_cast<float4*>(theta_out + o) = *reinterpret_cast<const float4*>(acc[q]);
-          if (tanh_out) {
-            T t[4];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) t[c] = tanhx(acc[q][c]);
-            *reinterpret_cast<float4*>(tanh_out + o) = *reinterpret_cast<const float4*>(t);
-          }
+          if (tanh_out) *reinterpret_cast<float4*>(tanh_out + o) = *reinterpret_cast<const float4*>(t);
         }
-        if constexpr (LP) {
-          if (logpsi_out) {
-            const bool odd = (u0 / FWD_U) & 1;
+      }
+    }
+    if constexpr (LP) {
+      if (logpsi_out) {
 #pragma unroll
-            for (int c = 0; c < 4; ++c)
-              if (m0 + MC * c < nh) {
-                const T l = log_cosh(acc[q][c]);
-                if (odd) lsum[q][1][c] = addx(lsum[q][1][c], l);
-                else lsum[q][0][c] = addx(lsum[q][0][c], l);
-              }
+        for (int c = 0; c < 4; ++c)
+          if (!SPREAD || u0 + 32 * c < nh) {
+            T l[RS];
+#pragma unroll
+            for (int q = 0; q < RS; ++q) {
+              l[q] = log_cosh(acc[q][c]);
+              if (m0 + MC * c >= nh) l[q] = ScalarTraits<T>::zero();
+            }
+            if ((u0 / FWD_U) & 1) {
+#pragma unroll
+              for (int q = 0; q < RS; ++q) lsum[q][1][c] = addx(lsum[q][1][c], l[q]);
+            } else {
+#pragma unroll
+              for (int q = 0; q < RS; ++q) lsum[q][0][c] = addx(lsum[q][0][c], l[q]);
+            }
           }
-        }
       }
     }
   }
   if constexpr (LP) {
     if (!logpsi_out) return;
+    auto unit = [&](int h, int c) { return 128 * h + (SPREAD ? lane + 32 * c : 4 * lane + c); };
+    T av[2][4];                                                // the visible terms of the first 256 sites
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) av[h][c] = unit(h, c) < ns ? a[unit(h, c)] : ScalarTraits<T>::zero();
 #pragma unroll
     for (int q = 0; q < RS; ++q) {
       const int64_t s = s0 + RS * row + q;
+      const uint32_t* wq = bits + (s < n_samples ? s : s0) * nw;
       T v = ScalarTraits<T>::zero();
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
@@ -435,13 +464,13 @@ QES_D void rbm_forward_block(uint8_t* smem, int64_t s0, int ns, int nh, int64_t 
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           x[c] = lsum[q][h][c];
-          if (s < n_samples)
-            for (int i = 128 * h + (CPLX ? lane + 32 * c : 4 * lane + c); i < ns; i += 256)
-              x[c] = fma_sign(sigma_of(bits + s * nw, i), a[i], x[c]);
+          const int i0 = unit(h, c);
+          if (i0 < ns) x[c] = fma_sign(sigma_of(wq, i0), av[h][c], x[c]);
+          for (int i = i0 + 256; i < ns; i += 256) x[c] = fma_sign(sigma_of(wq, i), a[i], x[c]);
 #pragma unroll
-          for (int o = CPLX ? 16 : 4; o > 0; o >>= 1) x[c] = addx(x[c], shfl_xor_val(x[c], o));
+          for (int o = SPREAD ? 16 : 4; o > 0; o >>= 1) x[c] = addx(x[c], shfl_xor_val(x[c], o));
         }
-        if constexpr (CPLX) {                                  // the four sums of 32, in every lane
+        if constexpr (SPREAD) {                                  // the four sums of 32, in every lane
 #pragma unroll
           for (int c = 0; c < 4; ++c) v = addx(v, x[c]);
         } else {                                               // threads 16, 8 and 4 apart above; 2 and 1 apart here
@@ -455,25 +484,33 @@ QES_D void rbm_forward_block(uint8_t* smem, int64_t s0, int ns, int nh, int64_t 
   }
 }
 
-template <class T, int RS, bool VEC, bool LP>
-__global__ void __launch_bounds__(FWD_THREADS, 2) rbm_forward_kernel(
+template <class T, int RS, bool VEC, bool LP, bool SPREAD>
+__global__ void __launch_bounds__(FWD_THREADS, LP && RS <= 2 && !ScalarTraits<T>::is_complex ? FWD_MINB : 2) rbm_forward_kernel(
     int ns, int nh, int64_t n_samples, const uint32_t* __restrict__ bits, const T* __restrict__ a,
     const T* __restrict__ b, const T* __restrict__ W, T* __restrict__ theta_out, T* __restrict__ tanh_out,
     T* __restrict__ logpsi_out) {
   extern __shared__ __align__(16) uint8_t fwd_sm[];
-  rbm_forward_block<T, RS, VEC, LP>(fwd_sm, (int64_t)blockIdx.x * FWD_TY * RS, ns, nh, n_samples, bits, a, b, W, theta_out,
+  rbm_forward_block<T, RS, VEC, LP, SPREAD>(fwd_sm, (int64_t)blockIdx.x * FWD_TY * RS, ns, nh, n_samples, bits, a, b, W, theta_out,
                                 tanh_out, logpsi_out);
 }
+
+// Real layers of few units: a lane's units 32 apart, so that a pass of few units evaluates tanh and log cosh once or twice per
+// lane and not four times, at three more loads per site: 58,532 samples of 3 x 12 tanh 29 -> 21 us, 20,000 of 100 x 30
+// 37 -> 33; 128 x 64 31 -> 35, 60 x 90 23 -> 25
+static bool fwd_spread(int ns, int nh) { return nh <= 64 && ns <= 96; }
 
 template <class T, int RS, bool LP>
 static int launch_forward_rs(int ns, int nh, int64_t n, const uint32_t* bits, const T* a, const T* b, const T* W,
                              T* theta_out, T* tanh_out, T* logpsi_out, cudaStream_t st) {
   const unsigned grid = (unsigned)((n + FWD_TY * RS - 1) / (FWD_TY * RS));
   const bool vec = nh % (16 / (int)sizeof(T)) == 0 && (reinterpret_cast<uintptr_t>(W) & 15) == 0;
-  auto kern = vec ? rbm_forward_kernel<T, RS, true, LP> : rbm_forward_kernel<T, RS, false, LP>;
+  const bool spread = ScalarTraits<T>::is_complex || fwd_spread(ns, nh);
+  constexpr bool C = ScalarTraits<T>::is_complex;
+  auto kern = spread ? (vec ? rbm_forward_kernel<T, RS, true, LP, true> : rbm_forward_kernel<T, RS, false, LP, true>)
+                     : (vec ? rbm_forward_kernel<T, RS, true, LP, C> : rbm_forward_kernel<T, RS, false, LP, C>);
   constexpr int smem = fwd_smem<T, RS>();
-  static QesSmemAttr attr[2];
-  QES_CUDA_CHECK(attr[vec].set<smem>(kern));
+  static QesSmemAttr attr[4];
+  QES_CUDA_CHECK(attr[2 * spread + vec].set<smem>(kern));
   kern<<<grid, FWD_THREADS, smem, st>>>(ns, nh, n, bits, a, b, W, theta_out, tanh_out, logpsi_out);
   QES_LAUNCH_CHECK();
   return QES_OK;
@@ -488,7 +525,7 @@ static int launch_forward(int ns, int nh, int64_t n, const uint32_t* bits, const
   auto blocks = [&](int rs) { return (n + FWD_TY * rs - 1) / (FWD_TY * rs); };
 #define QES_FWD(RS, LP) launch_forward_rs<T, RS, LP>(ns, nh, n, bits, a, b, W, theta_out, tanh_out, logpsi_out, st)
   if (logpsi_out) {
-    if (blocks(MAX / 2) >= 148) return QES_FWD(MAX / 2, true);
+    if (blocks(MAX / 2) >= 148 && (MAX / 2 == 2 || ns > FWD_FEW)) return QES_FWD(MAX / 2, true);
     if constexpr (MAX / 2 > 2)
       if (blocks(2) >= 148) return QES_FWD(2, true);
     return QES_FWD(1, true);
@@ -766,7 +803,7 @@ __global__ void __launch_bounds__(FWD_THREADS) batch_forward_kernel(const qes_ba
   const T* W = b + I.nh;
   const int64_t rows = (int64_t)I.n_chains * I.num_samples;
   extern __shared__ __align__(16) uint8_t fwd_sm[];
-  rbm_forward_block<T, 2, false, true>(fwd_sm, (int64_t)it.y * FWD_SB, I.ns, I.nh, rows, bits + I.sample_word_off, a, b, W,
+  rbm_forward_block<T, 2, false, true, ScalarTraits<T>::is_complex>(fwd_sm, (int64_t)it.y * FWD_SB, I.ns, I.nh, rows, bits + I.sample_word_off, a, b, W,
                        nullptr, tanh_out ? tanh_out + I.tanh_off : nullptr,
                        logpsi_out ? logpsi_out + I.sample_off : nullptr);
 }

@@ -43,6 +43,14 @@ def test_forward_tiles(cplx, ns, nh, n):
     assert none is None and torch.equal(t2, tn)
 
 
+# units 32 apart and in a row, slices of 8 to 32 sites, two samples per thread and four, more than 256 sites
+@pytest.mark.parametrize("cplx,ns,nh,n", [
+    (False, 96, 64, 2400), (False, 97, 64, 1200), (False, 96, 65, 4800), (False, 8, 33, 1), (False, 48, 300, 2400),
+    (False, 49, 140, 4800), (True, 41, 300, 2400), (False, 600, 40, 2400), (True, 523, 33, 1200), (False, 1, 1, 5000)])
+def test_forward_of_few_sites_and_units(cplx, ns, nh, n):
+    test_forward_tiles(cplx, ns, nh, n)
+
+
 # moves per thread (4) and per block (32), units per renormalisation (16), samples per thread and block;
 # scale 1.5: products that leave 2^+-8 and are renormalised
 @pytest.mark.parametrize("lx,ly,model,cplx,nh,n,scale", [
